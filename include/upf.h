@@ -535,7 +535,7 @@ typedef struct upf_launch_config {
   int32_t pforce_rows;
   int32_t density_mode;       /* list entries by 0: the TMA ring; 1: direct loads; 2: staged neighbourhoods */
   int32_t pforce_mode;
-  int32_t nlist_mode;         /* 0: each thread its own query box; 1: a warp walks the union of its boxes */
+  int32_t nlist_mode;         /* particles whose lists one warp builds: 0 by the particle count, 1 half as many */
   float measured_ms[4];       /* autotune: per-launch ms of the chosen shapes
                                  (neighbour lists, external forces, predicted
                                  density, pressure force); 0 otherwise */

@@ -204,7 +204,7 @@ bool shape_valid(const LaunchShape& s, bool batched, const char** why) {
   };
   if (s.nlist_threads != 64 && s.nlist_threads != 128 && s.nlist_threads != 256)
     return bad("nlist_threads must be 64, 128 or 256");
-  if (s.nlist_mode != 0 && s.nlist_mode != 1) return bad("nlist_mode must be 0 (lane boxes) or 1 (warp union)");
+  if (s.nlist_mode != 0 && s.nlist_mode != 1) return bad("nlist_mode must be 0 (particles a warp by count) or 1 (half as many)");
   if (s.external_threads != 128 && s.external_threads != 256) return bad("external_threads must be 128 or 256");
   if (!pair_ok(s.density_mode, s.density_threads, s.density_rows) ||
       !pair_ok(s.pforce_mode, s.pforce_threads, s.pforce_rows))
@@ -831,6 +831,7 @@ upf_status upf_create(const upf_params* p, int device, uint32_t capacity, upf_sy
   }
   UPF_CUDA(cudaSetDevice(device));
   UPF_CUDA(radix_init());
+  UPF_CUDA(pipeline_init());
   upf_system* s = new upf_system();
   s->prm = *p;
   s->device = device;
@@ -866,6 +867,7 @@ upf_status upf_create(const upf_params* p, int device, uint32_t capacity, upf_sy
   ALLOC(s->ncnt, c);
   ALLOC(s->cstart, s->ncells); ALLOC(s->cend, s->ncells);
   ALLOC(s->sstart, s->ncells); ALLOC(s->send, s->ncells);
+  ALLOC(s->mpos, c); ALLOC(s->mcells, (size_t)2 * s->ncells);
   ALLOC(s->spos, c); ALLOC(s->skeys, c); ALLOC(s->sid, c);
   ALLOC(s->luts, 5 * UPF_LUT_ENTRIES + kThresholds);
   ALLOC(s->st, 1);

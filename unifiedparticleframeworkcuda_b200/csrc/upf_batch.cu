@@ -205,6 +205,7 @@ upf_status upf_batch_create(const upf_params* params, const uint32_t* counts, ui
   }
   UPF_CUDA(cudaSetDevice(device));
   UPF_CUDA(radix_init());
+  UPF_CUDA(pipeline_init());
   upf_batch* b = new upf_batch();
   b->device = device;
   b->n_scenes = num_scenes;

@@ -26,6 +26,8 @@
 // which is the parity target; each kernel cites the function it restates.
 #include <cuda_runtime.h>
 
+#include <mutex>
+
 #include "upf_sys.h"
 #include "upf_tma.cuh"
 
@@ -59,9 +61,6 @@ constexpr int kUnroll = 8;
 // 8 took 128, a quarter of the SM's warps resident), which measured 0.24
 // against 0.38-0.45 ms per launch on the 1M dam.
 constexpr int kExternalUnroll = 2;
-// The list build gathers candidate positions 4 at a time: 40 registers a
-// thread against 56 with 8 (1.22 against 1.35 ms per build on the 1M dam).
-constexpr int kNlistUnroll = 4;
 
 template <int kU = kUnroll, class Load, class Use>
 __device__ __forceinline__ void for_neighbors(const uint32_t* __restrict__ col, uint32_t stride, uint32_t cnt,
@@ -142,15 +141,14 @@ struct Scope {
 // batched scenes: the key of a padding slot (above every 30-bit Morton key)
 constexpr uint32_t kPadKeyBatch = 1u << 30;
 
-// The scope of virtual block `block` (blockIdx.x, or a group taken from a
-// list of work by a resident grid).
+// The scope of a CTA whose particles start at index `slot`.
 template <bool kBatch>
-__device__ __forceinline__ Scope enter_scope_at(uint32_t block, const DevParams& Pk, const float* luts, DevState* st,
-                                                uint32_t n, const BatchView& bv, DevParams* sP, bool loop_pass) {
+__device__ __forceinline__ Scope enter_scope_slot(uint32_t slot, const DevParams& Pk, const float* luts, DevState* st,
+                                                  uint32_t n, const BatchView& bv, DevParams* sP, bool loop_pass) {
   if constexpr (!kBatch) {
     return Scope{&Pk, luts, st, n, 0u, false};
   } else {
-    const uint32_t s = bv.group_scene[(block * blockDim.x) / kSegAlign];
+    const uint32_t s = bv.group_scene[slot / kSegAlign];
     const uint32_t* src = reinterpret_cast<const uint32_t*>(bv.params + s);
     for (uint32_t k = threadIdx.x; k < sizeof(DevParams) / 4; k += blockDim.x)
       reinterpret_cast<uint32_t*>(sP)[k] = src[k];
@@ -158,6 +156,14 @@ __device__ __forceinline__ Scope enter_scope_at(uint32_t block, const DevParams&
     const bool skip = loop_pass && !*reinterpret_cast<volatile int32_t*>(&sst->loop_active);
     return Scope{sP, bv.luts + (size_t)s * kLutFloats, sst, bv.seg_end[s], s, skip};
   }
+}
+
+// The scope of virtual block `block` (blockIdx.x, or a group taken from a
+// list of work by a resident grid) with one particle a thread.
+template <bool kBatch>
+__device__ __forceinline__ Scope enter_scope_at(uint32_t block, const DevParams& Pk, const float* luts, DevState* st,
+                                                uint32_t n, const BatchView& bv, DevParams* sP, bool loop_pass) {
+  return enter_scope_slot<kBatch>(block * blockDim.x, Pk, luts, st, n, bv, sP, loop_pass);
 }
 
 template <bool kBatch>
@@ -243,221 +249,394 @@ __device__ __forceinline__ float dist2_xy(unsigned long long axy, float az, floa
   return fadd(fadd(s.x, s.y), fmul(dz, dz));
 }
 
+// The dynamic and the boundary particles as one sequence in Morton order
+// (dynamic first at equal keys), for the list build: element m holds a
+// position and, in w, the bits of its neighbour index. Each particle finds
+// its place by a binary search of the other set's sorted keys, and the cell
+// table of the sequence (start and end, as k_cell_ranges fills) follows from
+// the four keys beside it. Both sets' cells then are one contiguous range
+// each, whose order is the reference's ascending sorted-index order, and the
+// build needs no merge of its own. About 20 dependent loads a particle, all
+// of them cached: 9 us for 1,048,576 + 279,308 particles.
+__global__ void __launch_bounds__(kBlock) k_merge_sets(uint32_t n, const uint32_t* __restrict__ keys,
+                                                        const float4* __restrict__ pos, uint32_t ns,
+                                                        const uint32_t* __restrict__ skeys,
+                                                        const float4* __restrict__ spos, uint32_t static_base,
+                                                        int shift, uint32_t ncells, float4* __restrict__ mpos,
+                                                        uint32_t* __restrict__ mstart, uint32_t* __restrict__ mend) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n + ns) return;
+  const bool dyn = t < n;
+  const uint32_t j = dyn ? t : t - n;  // place in the own set
+  const uint32_t key = dyn ? keys[j] : skeys[j];
+  const uint32_t* __restrict__ other = dyn ? skeys : keys;
+  const uint32_t no = dyn ? ns : n;
+  // elements of the other set that come before: keys below, and for a
+  // boundary particle equal ones too (the dynamic set goes first)
+  uint32_t lo = 0, hi = no;
+  while (lo < hi) {
+    const uint32_t mid = lo + (hi - lo) / 2;
+    const uint32_t k = __ldg(other + mid);
+    if (dyn ? k < key : k <= key)
+      lo = mid + 1;
+    else
+      hi = mid;
+  }
+  const uint32_t m = j + lo;
+  float4 x = dyn ? pos[j] : spos[j];
+  x.w = __uint_as_float(dyn ? j : static_base + j);
+  mpos[m] = x;
+  const uint32_t c = key >> shift;
+  if (c >= ncells) return;
+  const uint32_t* __restrict__ own = dyn ? keys : skeys;
+  const uint32_t nown = dyn ? n : ns;
+  if ((j == 0 || (own[j - 1] >> shift) != c) && (lo == 0 || (other[lo - 1] >> shift) != c)) mstart[c] = m;
+  if ((j + 1 == nown || (own[j + 1] >> shift) != c) && (lo == no || (other[lo] >> shift) != c)) mend[c] = m + 1;
+}
+
 // GetNeighbors (UnifiedPhysics.cpp:2242-2280) with ZIndex::BoxQuery
-// (zIndex.cpp:43-73), one thread per particle: candidates are the search
-// cells (aligned Morton blocks of 2^cell_shift grid units, at most the
-// reference's block size) covering the query box with a one-grid-unit
-// margin. Every particle within h lies in the reference's query box, hence in
-// these cells, so the candidate set holds all of the reference's
-// neighbours. Cells are visited in ascending Morton order, each a contiguous
-// key range; within a cell the dynamic and boundary ranges are merged by
-// key. The list therefore comes out in the reference's ascending
-// sorted-index order, and membership is the reference's exact test: j != i
-// and |x_i - x_j| < h in float. Candidate positions are gathered kNlistUnroll at
-// a time. Each entry also records a list value at the current positions:
-// its kernel-table bin (WCSPH: the density and force passes read their
-// tables by it), or the pressure-gradient table's value at that bin
-// (PCISPH: the pressure-force pass, which evaluates at the current
-// positions, then reads no table).
+// (zIndex.cpp:43-73). Candidates are the search cells (aligned Morton blocks
+// of 2^cell_shift grid units, at most the reference's block size) covering
+// the query box with a one-grid-unit margin. Every particle within h lies in
+// the reference's query box, hence in these cells, so the candidate set
+// holds all of the reference's neighbours. Cells are visited in ascending
+// Morton order, each a contiguous range of the sorted set (the dynamic
+// particles, or both sets merged: kMerged, k_merge_sets). The list therefore
+// comes out in the reference's ascending sorted-index order, and membership
+// is the reference's exact test: j != i and |x_i - x_j| < h in float. Each
+// entry also records a list value at the current positions: its kernel-table
+// bin (WCSPH: the density and force passes read their tables by it), or the
+// pressure-gradient table's value at that bin (PCISPH: the pressure-force
+// pass, which evaluates at the current positions, then reads no table);
+// lval null: no values.
 //
-// kWarpUnion: the 32 lanes of a warp (32 consecutive Morton-sorted particles,
-// close together) walk the union of their query boxes, when it spans at
-// most 64 cells, instead of each lane its own box: every lane then visits
-// the same cells and candidates in the same order (no divergence; each
-// candidate position is one broadcast load) and keeps those within h of its
-// own particle. A lane's list is unchanged: all its neighbours lie in its own
-// box, a subset of the union, and the union's cells are still visited in
-// ascending Morton order.
-template <bool kBatch, int kThreads, bool kWarpUnion>
-__global__ void __launch_bounds__(kThreads) k_build_nlist(
+// One warp builds the lists of kW consecutive particles (close together in
+// Morton order). The cells that can hold a neighbour of any of them are
+// looked up and put in order once. The particles then go four at a time: the
+// cells that can hold a neighbour of one of the four are walked in chunks of
+// 32 consecutive candidates, one a lane (a coalesced load), each tested
+// against the four; a ballot gives a word of accepted bits per particle, lane
+// k keeps the words of chunk k, and those with a bit set wait in shared
+// memory. At the end lane p turns particle p's words into its list: all lanes
+// write entry after entry, so the column-major rows leave as runs of kW
+// words.
+// Bound: instruction issue (630 warp instructions a particle). On a dam one
+// particle's cells are 14 chunks, the cells of four 26, of eight 34: with 9
+// instructions a test and about 10 a chunk, four together come cheapest. Held
+// to 64 registers (eight 128-thread CTAs an SM; at 80 0.98 against 0.93 ms a
+// build of the dam from rest, at 48 it spills).
+// A thread per particle, as before, had its lanes in different cells (10.7 of
+// 32 active, 950 warp instructions a particle). Builds from rest, before and
+// now: 1,048,576 + 279,308 boundary particles 1.01 and 0.79 ms, 262,144 0.376
+// and 0.245, 32,768 (WCSPH) 0.134 and 0.062, 256 scenes 4.72 and 3.43.
+constexpr int kNlistTogether = 4;
+constexpr uint32_t kNlistWords = 16;  // words of accepted bits held per particle
+template <int kW>
+struct NlistWarp {
+  uint2 word[kNlistWords][kW];  // (accepted bits, first candidate) of particle p's chunks, word k in column
+                                // (p + k) % kW: one particle's words in different banks
+  uint2 range[64];              // the window's cells: ranges in the set
+  uint2 sel[64];                // those of the cells near the four at hand
+  uint32_t box[64];             // and their cell coordinates, 10 bits an axis
+  float4 x[kW];
+};
+template <int kThreads, int kW>
+constexpr size_t nlist_smem() { return kThreads / 32 * sizeof(NlistWarp<kW>); }
+
+// the sum of v over the lanes up to and including this one
+__device__ __forceinline__ uint32_t warp_inclusive(uint32_t v, uint32_t lane) {
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t o = __shfl_up_sync(0xffffffffu, v, d);
+    if (lane >= (uint32_t)d) v += o;
+  }
+  return v;
+}
+
+// the first lane whose v (ascending over the lanes) is above r; 31 if none
+__device__ __forceinline__ uint32_t first_above(uint32_t v, uint32_t r) {
+  uint32_t k = 0;
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1)
+    if (__shfl_sync(0xffffffffu, v, k + s - 1) <= r) k += s;
+  return k;
+}
+
+template <bool kBatch, bool kMerged, int kThreads, int kW>
+__global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_build_nlist(
     const __grid_constant__ DevParams Pk, const BatchView bv, uint32_t n, const float4* __restrict__ pos,
-    const uint32_t* __restrict__ keys, const uint32_t* __restrict__ cstart, const uint32_t* __restrict__ cend,
-    uint32_t ns, const float4* __restrict__ spos, const uint32_t* __restrict__ skeys,
-    const uint32_t* __restrict__ sstart, const uint32_t* __restrict__ send, uint32_t* __restrict__ nbr,
-    uint32_t* __restrict__ lval, uint32_t* __restrict__ ncnt, const float* __restrict__ luts,
-    DevState* __restrict__ st_plain) {
+    const float4* __restrict__ mpos, const uint32_t* __restrict__ cstart, const uint32_t* __restrict__ cend,
+    uint32_t* __restrict__ nbr, uint32_t* __restrict__ lval, uint32_t* __restrict__ ncnt,
+    const float* __restrict__ luts, DevState* __restrict__ st_plain) {
+  constexpr int kWarps = kThreads / 32;
+  static_assert(32 % kW == 0 && kSegAlign % (kWarps * kW) == 0, "a CTA's particles lie in one scene");
+  extern __shared__ __align__(16) unsigned char nlist_mem[];
   __shared__ DevParams sP;
   __shared__ float thr[kThresholds];
   __shared__ float pg[UPF_LUT_ENTRIES];
-  const Scope sc = enter_scope<kBatch>(Pk, luts, st_plain, n, bv, &sP, false);
-  for (int k = threadIdx.x; k < kThresholds; k += blockDim.x) thr[k] = sc.luts[5 * UPF_LUT_ENTRIES + k];
+  const uint32_t slot0 = blockIdx.x * (uint32_t)(kWarps * kW);
+  const Scope sc = enter_scope_slot<kBatch>(slot0, Pk, luts, st_plain, n, bv, &sP, false);
+  for (int k = threadIdx.x; k < kThresholds; k += kThreads) thr[k] = sc.luts[5 * UPF_LUT_ENTRIES + k];
   stage_lut(pg, sc.luts + LUT_PGRAD * UPF_LUT_ENTRIES);
   __syncthreads();
   const DevParams& P = *sc.P;
-  DevState* st = sc.st;
   if (kBatch) {
     // the scene's own cell table (keys are the scene's Morton keys)
     cstart += bv.cell_base[sc.scene];
     cend += bv.cell_base[sc.scene];
   }
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool active = i < sc.end;
-  if (!kWarpUnion && !active) return;
-  if (kWarpUnion && !__any_sync(0xffffffffu, active)) return;  // uniform over the warp
-  const float4 xi = active ? pos[i] : make_float4(0, 0, 0, 0);
-  const float h = P.h;
-  int lo[3], hi[3];
-  float cg[3];  // the particle's grid position, clamped to the grid as keys are
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t i0 = slot0 + warp * kW;
+  if (i0 >= sc.end) return;  // uniform over the warp; no CTA barrier follows
+  NlistWarp<kW>& M = reinterpret_cast<NlistWarp<kW>*>(nlist_mem)[warp];
+  const uint32_t lt = lanemask_lt();
+  const uint32_t maxn = P.maxn, stride = P.nstride;
+  const float h = P.h, r2_edge = thr[kThresholds - 1];
+  const int shift = (int)P.cell_shift;
+  const bool grad = P.list_grad != 0;
+  const bool mine = lane < (uint32_t)kW && i0 + lane < sc.end;
+  // lane l's particle: its grid position, clamped to the grid as keys are,
+  // and its query box in cells
+  const float4 xi = mine ? pos[i0 + lane] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  float cg[3] = {0, 0, 0};
+  int lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
   {
-    const float c[3] = {(xi.x - P.origin.x) * P.scales.x, (xi.y - P.origin.y) * P.scales.y,
-                        (xi.z - P.origin.z) * P.scales.z};
-    const float r[3] = {h * P.scales.x, h * P.scales.y, h * P.scales.z};
+    const float org[3] = {P.origin.x, P.origin.y, P.origin.z}, sca[3] = {P.scales.x, P.scales.y, P.scales.z};
+    const float x[3] = {xi.x, xi.y, xi.z};
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      float l = c[a] - r[a] - 1.0f, u = c[a] + r[a] + 1.0f;
-      int li = (l <= 0.0f) ? 0 : (l >= 1023.0f ? 1023 : (int)l);
-      int ui = (u <= 0.0f) ? 0 : (u >= 1023.0f ? 1023 : (int)u);
-      lo[a] = li >> P.cell_shift;
-      hi[a] = ui >> P.cell_shift;
-      cg[a] = fminf(fmaxf(c[a], 0.0f), 1024.0f);
+      const float c = (x[a] - org[a]) * sca[a], r = h * sca[a];
+      const float l = c - r - 1.0f, u = c + r + 1.0f;
+      const int li = (l <= 0.0f) ? 0 : (l >= 1023.0f ? 1023 : (int)l);
+      const int ui = (u <= 0.0f) ? 0 : (u >= 1023.0f ? 1023 : (int)u);
+      lo[a] = li >> shift;
+      hi[a] = ui >> shift;
+      cg[a] = fminf(fmaxf(c, 0.0f), 1024.0f);
     }
   }
-  // Cells of the query box whose nearest point lies farther than h from the
-  // particle hold no neighbour and are skipped. A particle's key cell holds
-  // its clamped grid position to within float rounding, so the cell's box is
-  // widened by one grid unit; clamping shortens no distance, and h^2 gets
-  // a 1e-5 relative margin: the test only drops cells that cannot hold a
-  // particle within h. Lanes that walk the warp's union of boxes skip none.
-  const int cs = 1 << P.cell_shift;
-  const float cull_h2 = h * h * 1.00001f;
-  bool cull = !kWarpUnion;
-  auto may_hold = [&](int bx, int by, int bz) {
-    if (!cull) return true;
-    const int b[3] = {bx, by, bz};
-    const float sc[3] = {P.scales.x, P.scales.y, P.scales.z};
-    float s = 0.0f;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const float blo = (float)(b[a] * cs) - 1.0f, bhi = (float)((b[a] + 1) * cs) + 1.0f;
-      const float d = fmaxf(0.0f, fmaxf(blo - cg[a], cg[a] - bhi)) / sc[a];
-      s += d * d;
+  if (lane < kW) M.x[lane] = xi;
+  const float cs = (float)(1 << shift), cull_h2 = h * h * 1.00001f;
+  const float inv[3] = {1.0f / P.scales.x, 1.0f / P.scales.y, 1.0f / P.scales.z};
+  uint32_t cnt_mine = 0;  // lane l: the neighbours of particle i0 + l
+  uint32_t words = 0;     // and its words in M.word
+  // the lanes of `who` turn their words into list entries
+  auto emit = [&](uint32_t who) {
+    __syncwarp();
+    if ((who >> lane) & 1u) {
+      const uint32_t i = i0 + lane;
+      uint32_t* __restrict__ out = nbr + i;
+      uint32_t* __restrict__ ov = lval + i;
+      uint32_t k = 0;
+      uint2 w = make_uint2(0, 0);
+      while (true) {
+        if (!w.x) {
+          if (k == words) break;
+          w = M.word[k][(lane + k) % kW];
+          ++k;
+        }
+        const uint32_t idx = w.y + __ffs(w.x) - 1;
+        w.x &= w.x - 1;
+        const uint32_t nb = kMerged ? __float_as_uint(__ldg(&mpos[idx].w)) : idx;
+        if (nb == i) continue;  // the particle itself
+        if (cnt_mine < maxn) {
+          out[(size_t)cnt_mine * stride] = nb;
+          if (lval) {
+            const int bin = bin_of_r2(dist2(xi, __ldg(mpos + idx)), P.lut_factor, thr);
+            ov[(size_t)cnt_mine * stride] = grad ? __float_as_uint(pg[bin]) : (uint32_t)bin;
+          }
+        }
+        ++cnt_mine;
+      }
+      words = 0;
     }
-    return s <= cull_h2;
+    __syncwarp();
   };
-  if (kWarpUnion) {
+  uint32_t pending = __ballot_sync(0xffffffffu, mine);
+  while (pending) {
+    // the particles whose boxes share one window of at most 64 cells: all
+    // that are left, or those within four cells a side of the first one's
+    // lower corner (a query box spans at most four). Warps that straddle a
+    // jump of the Morton curve take more than one round.
+    uint32_t group = pending;
     int ulo[3], uhi[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      ulo[a] = __reduce_min_sync(0xffffffffu, active ? lo[a] : 0x7fffffff);
-      uhi[a] = __reduce_max_sync(0xffffffffu, active ? hi[a] : -1);
-    }
-    if ((uhi[0] - ulo[0] + 1) * (uhi[1] - ulo[1] + 1) * (uhi[2] - ulo[2] + 1) <= 64) {
+    for (int round = 0;; ++round) {
+      const bool in = (group >> lane) & 1u;
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
-        lo[a] = ulo[a];
-        hi[a] = uhi[a];
+        ulo[a] = __reduce_min_sync(0xffffffffu, in ? lo[a] : 0x7fffffff);
+        uhi[a] = __reduce_max_sync(0xffffffffu, in ? hi[a] : -1);
       }
-    }
-  }
-  const uint32_t maxn = P.maxn, stride = P.nstride;
-  uint32_t cnt = 0;
-  uint32_t* __restrict__ out = nbr + i;
-  uint32_t* __restrict__ ov = lval + i;
-  const bool grad = P.list_grad != 0;
-  // An append stores the entry and its squared distance; the list value
-  // (bin_of_r2 and the table) follows in one pass over the finished list,
-  // where the lanes of a warp run together instead of one append at a time.
-  auto append = [&](uint32_t code, float r2) {
-    if (!active) return;
-    if (cnt < maxn) {
-      out[(size_t)cnt * stride] = code;
-      ov[(size_t)cnt * stride] = __float_as_uint(r2);
-    }
-    cnt++;
-  };
-  // one contiguous range of one set; `base` turns a set index into a
-  // neighbour index (0 for dynamic, static_base for boundary particles)
-  auto scan_range = [&](const float4* __restrict__ set, uint32_t b, uint32_t e, uint32_t base, bool skip_self) {
-    for (; b + kNlistUnroll <= e; b += kNlistUnroll) {
-      float4 xj[kNlistUnroll];
+      if (round || (uhi[0] - ulo[0] + 1) * (uhi[1] - ulo[1] + 1) * (uhi[2] - ulo[2] + 1) <= 64) break;
+      const int first = __ffs(pending) - 1;
+      bool near = (pending >> lane) & 1u;
 #pragma unroll
-      for (int u = 0; u < kNlistUnroll; ++u) xj[u] = __ldg(set + b + u);
+      for (int a = 0; a < 3; ++a) {
+        const int l0 = __shfl_sync(0xffffffffu, lo[a], first);
+        near = near && lo[a] >= l0 && hi[a] <= l0 + 3;
+      }
+      group = __ballot_sync(0xffffffffu, near) | (1u << first);
+    }
+    pending &= ~group;
+    const int nx = uhi[0] - ulo[0] + 1, ny = uhi[1] - ulo[1] + 1, nz = uhi[2] - ulo[2] + 1;
+    // the window's cells that hold particles, two a lane, in Morton order
+    uint32_t code[2], box[2], have[2], rank[2] = {0, 0};
+    uint2 range[2];
 #pragma unroll
-      for (int u = 0; u < kNlistUnroll; ++u) {
-        const uint32_t j = b + u;
-        const float r2 = dist2(xi, xj[u]);
-        if (!(skip_self && j == i) && r2 < thr[kThresholds - 1]) append(j + base, r2);
+    for (int q = 0; q < 2; ++q) {
+      const int c = (int)lane + 32 * q;
+      const int t = c / nx, bz = t / ny;
+      const int b[3] = {ulo[0] + c - t * nx, ulo[1] + t - bz * ny, ulo[2] + bz};
+      code[q] = morton3(b[0], b[1], b[2]);
+      box[q] = (uint32_t)b[0] | ((uint32_t)b[1] << 10) | ((uint32_t)b[2] << 20);
+      range[q] = make_uint2(0, 0);
+      if (bz < nz) range[q] = make_uint2(__ldg(cstart + code[q]), __ldg(cend + code[q]));
+      have[q] = __ballot_sync(0xffffffffu, range[q].x < range[q].y);
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+      for (uint32_t m = have[q]; m; m &= m - 1) {
+        const uint32_t c = __shfl_sync(0xffffffffu, code[q], __ffs(m) - 1);
+        rank[0] += c < code[0];
+        rank[1] += c < code[1];
       }
-    }
-    for (; b < e; ++b) {
-      const float r2 = dist2(xi, __ldg(set + b));
-      if (!(skip_self && b == i) && r2 < thr[kThresholds - 1]) append(b + base, r2);
-    }
-  };
-  auto visit = [&](uint32_t c) {
-    uint32_t ds = cstart[c], de = cend[c];
-    uint32_t ss = 0, se = 0;
-    if (ns) {
-      ss = sstart[c];
-      se = send[c];
-    }
-    if (ss == se) {
-      scan_range(pos, ds, de, 0u, true);
-      return;
-    }
-    if (ds == de) {
-      scan_range(spos, ss, se, P.static_base, false);
-      return;
-    }
-    while (ds < de || ss < se) {  // both sets present: merge by key
-      bool take_dyn = (ds < de) && (ss >= se || keys[ds] <= skeys[ss]);
-      if (take_dyn) {
-        uint32_t j = ds++;
-        const float r2 = dist2(xi, pos[j]);
-        if (j != i && r2 < thr[kThresholds - 1]) append(j, r2);
-      } else {
-        uint32_t j = ss++;
-        const float r2 = dist2(xi, spos[j]);
-        if (r2 < thr[kThresholds - 1]) append(j + P.static_base, r2);
+    __syncwarp();  // the last group's cells have been read
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+      if ((have[q] >> lane) & 1u) {
+        M.range[rank[q]] = range[q];
+        M.box[rank[q]] = box[q];
       }
+    const uint32_t ncell = __popc(have[0]) + __popc(have[1]);
+    __syncwarp();
+    // lane l: the lower bounds of cells l and l + 32, widened by one grid unit
+    float blo[2][3];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const uint32_t c = lane + 32 * q;
+      const uint32_t b = c < ncell ? M.box[c] : 0u;
+      blo[q][0] = (float)(b & 1023u) * cs - 1.0f;
+      blo[q][1] = (float)((b >> 10) & 1023u) * cs - 1.0f;
+      blo[q][2] = (float)(b >> 20) * cs - 1.0f;
     }
-  };
-  const int nx = hi[0] - lo[0] + 1, ny = hi[1] - lo[1] + 1, nz = hi[2] - lo[2] + 1;
-  const int nblk = nx * ny * nz;
-  if (nblk <= 64) {
-    uint32_t codes[64];
-    int m = 0;
-    for (int bz = lo[2]; bz <= hi[2]; ++bz)
-      for (int by = lo[1]; by <= hi[1]; ++by)
-        for (int bx = lo[0]; bx <= hi[0]; ++bx) {
-          if (!may_hold(bx, by, bz)) continue;
-          uint32_t c = morton3(bx, by, bz);
-          int q = m++;
-          while (q > 0 && codes[q - 1] > c) {
-            codes[q] = codes[q - 1];
-            --q;
-          }
-          codes[q] = c;
+    for (uint32_t left = group; left;) {
+      // the next four particles (at the group's end fewer: the rest lie at
+      // infinity, where nothing is accepted)
+      uint32_t who[kNlistTogether], four = 0;
+      unsigned long long pxy[kNlistTogether];
+      float pz[kNlistTogether];
+#pragma unroll
+      for (int t = 0; t < kNlistTogether; ++t) {
+        float4 x = make_float4(INFINITY, INFINITY, INFINITY, 0.0f);
+        who[t] = 32;
+        if (left) {
+          who[t] = __ffs(left) - 1;
+          four |= 1u << who[t];
+          left &= left - 1;
+          x = M.x[who[t]];
         }
-    for (int q = 0; q < m; ++q) visit(codes[q]);
-  } else {
-    for (int bz = lo[2]; bz <= hi[2]; ++bz)
-      for (int by = lo[1]; by <= hi[1]; ++by)
-        for (int bx = lo[0]; bx <= hi[0]; ++bx)
-          if (may_hold(bx, by, bz)) visit(morton3(bx, by, bz));
-  }
-  if (!active) return;
-  const uint32_t m = cnt < maxn ? cnt : maxn;
-  // the list values at the entries' squared distances, four entries' loads
-  // in flight at a time
-  uint32_t k = 0;
-  for (; k + 4 <= m; k += 4) {
-    float r2[4];
+        pxy[t] = pk2(x.x, x.y);
+        pz[t] = x.z;
+      }
+      // Cells farther than h from the box around the four hold no neighbour
+      // and are left out. A particle's key cell holds its clamped grid
+      // position to within float rounding, so the cell's box is widened by
+      // one grid unit; clamping shortens no distance, and h^2 gets a 1e-5
+      // relative margin. (Clamped grid positions are not negative: their
+      // bits order as they do.)
+      const bool in = (four >> lane) & 1u;
+      float near2[2] = {0.0f, 0.0f};
 #pragma unroll
-    for (int u = 0; u < 4; ++u) r2[u] = __uint_as_float(ov[(size_t)(k + u) * stride]);
+      for (int a = 0; a < 3; ++a) {
+        const uint32_t bits = __float_as_uint(cg[a]);
+        const float gl = __uint_as_float(__reduce_min_sync(0xffffffffu, in ? bits : 0x7f800000u));
+        const float gh = __uint_as_float(__reduce_max_sync(0xffffffffu, in ? bits : 0u));
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int bin = bin_of_r2(r2[u], P.lut_factor, thr);
-      ov[(size_t)(k + u) * stride] = grad ? __float_as_uint(pg[bin]) : (uint32_t)bin;
+        for (int q = 0; q < 2; ++q) {
+          const float d = fmaxf(0.0f, fmaxf(blo[q][a] - gh, gl - (blo[q][a] + cs + 2.0f))) * inv[a];
+          near2[q] += d * d;
+        }
+      }
+      // the ranges of the selected cells, in order, 32 at a time (a lane
+      // each), cut into chunks of 32 candidates; lane k takes chunk k
+      const bool in0 = lane < ncell && near2[0] <= cull_h2, in1 = lane + 32 < ncell && near2[1] <= cull_h2;
+      const uint32_t sel0 = __ballot_sync(0xffffffffu, in0), sel1 = __ballot_sync(0xffffffffu, in1);
+      const uint32_t nsel = __popc(sel0) + __popc(sel1);
+      __syncwarp();
+      if (in0) M.sel[__popc(sel0 & lt)] = M.range[lane];
+      if (in1) M.sel[__popc(sel0) + __popc(sel1 & lt)] = M.range[lane + 32];
+      __syncwarp();
+      uint32_t c0 = 0, k0 = 0;  // first cell of this round, chunks of its cells already done
+      while (c0 < nsel) {
+        const uint2 cell = c0 + lane < nsel ? M.sel[c0 + lane] : make_uint2(0, 0);
+        const uint32_t upto = warp_inclusive((cell.y - cell.x + 31) / 32, lane);
+        const uint32_t all = __shfl_sync(0xffffffffu, upto, 31);
+        const uint32_t mine_k = k0 + lane;  // this lane's chunk, among those of the 32 cells
+        const uint32_t chunks = min(all - k0, 32u);
+        const uint32_t of = first_above(upto, mine_k);
+        const uint32_t before_of = __shfl_sync(0xffffffffu, upto, of - 1);
+        const uint32_t s0 = __shfl_sync(0xffffffffu, cell.x, of), end = __shfl_sync(0xffffffffu, cell.y, of);
+        const uint32_t from = s0 + 32 * (mine_k - (of ? before_of : 0u));
+        k0 += 32;
+        if (k0 >= all) {
+          c0 += 32;
+          k0 = 0;
+        }
+        uint32_t hit[kNlistTogether];
+#pragma unroll
+        for (int t = 0; t < kNlistTogether; ++t) hit[t] = 0;
+        // two chunks' loads in flight (an odd last one is tested twice, and
+        // its second word, past the chunks, is dropped)
+        for (uint32_t k = 0; k < chunks; k += 2) {
+          float4 xj[2];
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const uint32_t ku = min(k + u, chunks - 1);
+            const uint32_t b = __shfl_sync(0xffffffffu, from, ku), e = __shfl_sync(0xffffffffu, end, ku);
+            xj[u] = __ldg(mpos + min(b + lane, e - 1));
+          }
+#pragma unroll
+          for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int t = 0; t < kNlistTogether; ++t) {
+              // (infinities and their differences compare false)
+              const uint32_t h = __ballot_sync(0xffffffffu, dist2_xy(pxy[t], pz[t], xj[u]) < r2_edge);
+              if (lane == k + u) hit[t] = h;
+            }
+        }
+        const uint32_t cands = lane < chunks ? end - from : 0u;
+        const uint32_t valid = cands >= 32 ? 0xffffffffu : (1u << cands) - 1u;
+        // the words with a bit set go to shared memory, in order
+#pragma unroll
+        for (int t = 0; t < kNlistTogether; ++t) {
+          const uint32_t w = hit[t] & valid, p = who[t];
+          uint32_t some = __ballot_sync(0xffffffffu, w != 0);
+          while (some) {
+            uint32_t at = __shfl_sync(0xffffffffu, words, p);
+            if (at == kNlistWords) {  // no room left: this particle's entries first
+              emit(1u << p);
+              at = 0;
+            }
+            const uint32_t to = at + __popc(some & lt);
+            const bool put = ((some >> lane) & 1u) && to < kNlistWords;
+            if (put) M.word[to][(p + to) % kW] = make_uint2(w, from);
+            const uint32_t done = __ballot_sync(0xffffffffu, put);
+            if (lane == p) words = at + __popc(done);
+            some &= ~done;
+          }
+        }
+      }
     }
   }
-  for (; k < m; ++k) {
-    const int bin = bin_of_r2(__uint_as_float(ov[(size_t)k * stride]), P.lut_factor, thr);
-    ov[(size_t)k * stride] = grad ? __float_as_uint(pg[bin]) : (uint32_t)bin;
+  emit(0xffffffffu);
+  const uint32_t held = min(cnt_mine, maxn);
+  if (mine) ncnt[i0 + lane] = held;
+  const uint32_t most = __reduce_max_sync(0xffffffffu, cnt_mine);
+  if (lane == 0) {
+    DevState* st = sc.st;
+    if (most > maxn) atomicOr(&st->error_flags, (uint32_t)ERR_OVERFLOW);
+    // most warps find a larger count there already
+    if (most > *reinterpret_cast<volatile uint32_t*>(&st->max_neighbors)) atomicMax(&st->max_neighbors, most);
   }
-  ncnt[i] = m;
-  if (cnt > maxn) atomicOr(&st->error_flags, (uint32_t)ERR_OVERFLOW);
-  atomicMax(&st->max_neighbors, cnt);
 }
 
 // ---------------------------------------------------------------- WCSPH
@@ -1880,22 +2059,37 @@ __global__ void __launch_bounds__(kBlock) k_static_wvol(DevParams P, uint32_t ns
 inline uint32_t grid_of(uint32_t n) { return (n + kBlock - 1) / kBlock; }
 
 // ---- launches of the tunable passes at a LaunchShape
-template <bool kBatch>
+// Particles a warp of the list build takes. More share the cell look-up and
+// write longer rows (at 1,048,576 particles 0.79 ms with 32, 0.87 with 16);
+// fewer leave more warps (at 32,768 0.062 ms with 8, 0.075 with 4 and 0.063
+// with 16; at 262,144 16 and 32 are level, and 16 has the shorter last wave).
+// nlist_mode 1 halves the number.
+inline int nlist_warp_particles(const LaunchShape& sh, uint32_t n) {
+  const int w = n >= 524288 ? 32 : (n >= 65536 ? 16 : (n >= 16384 ? 8 : 4));
+  return sh.nlist_mode == 1 && w > 4 ? w / 2 : w;
+}
+
+template <bool kBatch, bool kMerged>
 cudaError_t run_nlist(const LaunchShape& sh, cudaStream_t st, const DevParams& P, const BatchView& bv, uint32_t n,
-                      const float4* pos, const uint32_t* keys, const uint32_t* cstart, const uint32_t* cend,
-                      uint32_t ns, const float4* spos, const uint32_t* skeys, const uint32_t* sstart,
-                      const uint32_t* send, uint32_t* nbr, uint32_t* lval, uint32_t* ncnt, const float* luts,
-                      DevState* stp) {
-#define UPF_NL(T, W)                                                                                          \
-  k_build_nlist<kBatch, T, W><<<(n + T - 1) / T, T, 0, st>>>(P, bv, n, pos, keys, cstart, cend, ns, spos, skeys, \
-                                                             sstart, send, nbr, lval, ncnt, luts, stp)
-  switch (sh.nlist_threads * 10 + sh.nlist_mode) {
-    case 640: UPF_NL(64, false); break;
-    case 1280: UPF_NL(128, false); break;
-    case 2560: UPF_NL(256, false); break;
-    case 641: UPF_NL(64, true); break;
-    case 1281: UPF_NL(128, true); break;
-    case 2561: UPF_NL(256, true); break;
+                      const float4* pos, const float4* mpos, const uint32_t* cstart, const uint32_t* cend,
+                      uint32_t* nbr, uint32_t* lval, uint32_t* ncnt, const float* luts, DevState* stp) {
+#define UPF_NL(T, W)                                                                                           \
+  k_build_nlist<kBatch, kMerged, T, W><<<(n + T / 32 * W - 1) / (T / 32 * W), T, nlist_smem<T, W>(), st>>>(P, bv, n, pos, mpos,  \
+                                                                                        cstart, cend, nbr, lval, \
+                                                                                        ncnt, luts, stp)
+  switch (sh.nlist_threads * 100 + nlist_warp_particles(sh, n)) {
+    case 6404: UPF_NL(64, 4); break;
+    case 6408: UPF_NL(64, 8); break;
+    case 6416: UPF_NL(64, 16); break;
+    case 12804: UPF_NL(128, 4); break;
+    case 12808: UPF_NL(128, 8); break;
+    case 12816: UPF_NL(128, 16); break;
+    case 25604: UPF_NL(256, 4); break;
+    case 25608: UPF_NL(256, 8); break;
+    case 25616: UPF_NL(256, 16); break;
+    case 6432: UPF_NL(64, 32); break;
+    case 12832: UPF_NL(128, 32); break;
+    case 25632: UPF_NL(256, 32); break;
     default: return cudaErrorInvalidConfiguration;
   }
 #undef UPF_NL
@@ -1975,6 +2169,30 @@ cudaError_t run_pforce(const LaunchShape& sh, cudaStream_t st, const DevParams& 
 }  // namespace
 
 // ----------------------------------------------------------------- launchers
+// The list build's shapes whose shared memory is over 48 KB are opted in on
+// the current device, once per device (before any capture that launches them).
+template <bool kBatch, bool kMerged>
+static cudaError_t nlist_opt_in() {
+  static_assert(nlist_smem<256, 16>() + 3072 <= 48 * 1024, "the other shapes fit without");
+  return cudaFuncSetAttribute(k_build_nlist<kBatch, kMerged, 256, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)nlist_smem<256, 32>());
+}
+
+cudaError_t pipeline_init() {
+  static std::mutex mu;
+  static bool done[64] = {};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(mu);
+  if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
+  if ((e = nlist_opt_in<false, false>()) != cudaSuccess) return e;
+  if ((e = nlist_opt_in<false, true>()) != cudaSuccess) return e;
+  if ((e = nlist_opt_in<true, false>()) != cudaSuccess) return e;
+  if (dev >= 0 && dev < 64) done[dev] = true;
+  return cudaSuccess;
+}
+
 cudaError_t launch_sort_phase(System& s, cudaStream_t st) {
   const uint32_t n = s.n_dyn;
   if (n == 0) return cudaSuccess;
@@ -2014,8 +2232,20 @@ cudaError_t launch_neighbor_phase(System& s, cudaStream_t st) {
   k_step_init<<<1, 1, 0, st>>>(s.st, s.prm.method == UPF_METHOD_WCSPH ? 1 : 0);
   if (n == 0) return cudaGetLastError();
   s.lists_staged = false;
-  cudaError_t e = run_nlist<false>(s.shape, st, s.dp, BatchView{}, n, s.B.pos, s.keysA, s.cstart, s.cend, s.n_static,
-                                   s.spos, s.skeys, s.sstart, s.send, s.nbr, s.lval, s.ncnt, s.luts, s.st);
+  cudaError_t e;
+  if (s.n_static) {
+    const uint32_t all = n + s.n_static;
+    if ((e = cudaMemsetAsync(s.mcells, 0, 2 * sizeof(uint32_t) * s.ncells, st)) != cudaSuccess) return e;
+    k_merge_sets<<<grid_of(all), kBlock, 0, st>>>(n, s.keysA, s.B.pos, s.n_static, s.skeys, s.spos, s.dp.static_base,
+                                                  3 * (int)s.dp.cell_shift, s.ncells, s.mpos, s.mcells,
+                                                  s.mcells + s.ncells);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    e = run_nlist<false, true>(s.shape, st, s.dp, BatchView{}, n, s.B.pos, s.mpos, s.mcells, s.mcells + s.ncells, s.nbr,
+                               s.lval, s.ncnt, s.luts, s.st);
+  } else {
+    e = run_nlist<false, false>(s.shape, st, s.dp, BatchView{}, n, s.B.pos, s.B.pos, s.cstart, s.cend, s.nbr, s.lval,
+                                s.ncnt, s.luts, s.st);
+  }
   if (e != cudaSuccess || !stages_lists(s)) return e;
   return launch_stage_lists(s, st);
 }
@@ -2137,13 +2367,14 @@ cudaError_t launch_static_setup(System& s, cudaStream_t st) {
 }
 
 // Neighbour lists of one sorted set with no boundary set (the adjoint's
-// per-step lists); P.nstride is the list stride, P.maxn its rows.
-cudaError_t launch_nlist_plain(const DevParams& P, uint32_t n, const float4* pos, const uint32_t* keys,
-                               const uint32_t* cstart, const uint32_t* cend, uint32_t* nbr, uint32_t* lval,
-                               uint32_t* ncnt, const float* luts, DevState* st, cudaStream_t stream) {
+// per-step lists), without list values; P.nstride is the list stride, P.maxn
+// its rows.
+cudaError_t launch_nlist_plain(const DevParams& P, uint32_t n, const float4* pos, const uint32_t* cstart,
+                               const uint32_t* cend, uint32_t* nbr, uint32_t* ncnt, const float* luts, DevState* st,
+                               cudaStream_t stream) {
   if (!n) return cudaSuccess;
-  return run_nlist<false>(LaunchShape{}, stream, P, BatchView{}, n, pos, keys, cstart, cend, 0u, nullptr, nullptr,
-                          nullptr, nullptr, nbr, lval, ncnt, luts, st);
+  return run_nlist<false, false>(LaunchShape{}, stream, P, BatchView{}, n, pos, pos, cstart, cend, nbr, nullptr, ncnt,
+                                 luts, st);
 }
 
 // ----------------------------------------------------------- batched launchers
@@ -2186,8 +2417,8 @@ cudaError_t batch_launch_neighbors(BatchSystem& b, cudaStream_t st) {
   const uint32_t n = b.n_slots;
   k_step_init_batch<<<1, 256, 0, st>>>(b.st_d, b.n_scenes);
   if (!n) return cudaGetLastError();
-  return run_nlist<true>(b.shape, st, DevParams{}, b.view, n, b.B.pos, b.keysA, b.cstart, b.cend, 0u, nullptr, nullptr,
-                         nullptr, nullptr, b.nbr, b.lval, b.ncnt, nullptr, nullptr);
+  return run_nlist<true, false>(b.shape, st, DevParams{}, b.view, n, b.B.pos, b.B.pos, b.cstart, b.cend, b.nbr, b.lval,
+                                b.ncnt, nullptr, nullptr);
 }
 
 cudaError_t batch_launch_forces(BatchSystem& b, cudaStream_t st) {
@@ -2331,7 +2562,8 @@ cudaError_t batch_launch_integrate(BatchSystem& b, cudaStream_t st) {
 
 int pipeline_launches_per_step(const System& s, int iterations) {
   int sort = radix_launches(s.key_bits) + 1 /*reorder*/ + 1 /*cells*/ + (s.rb.n_rigid ? 1 : 0) /*rigid slots*/;
-  int nl = 2 + (stages_lists(s) ? 1 : 0);  // step init + neighbour lists (+ staging)
+  // step init + neighbour lists (+ merge of the two sets, + staging)
+  int nl = 2 + (s.n_static ? 1 : 0) + (stages_lists(s) ? 1 : 0);
   if (s.prm.method == UPF_METHOD_WCSPH) return sort + nl + 2;
   return sort + nl + 1 /*external*/ + 1 /*loop init*/ + 3 * iterations + 1 /*integrate*/ + rigid_launches_per_step(s);
 }

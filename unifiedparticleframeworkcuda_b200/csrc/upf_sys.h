@@ -65,7 +65,7 @@ struct LaunchShape {
   int density_mode = 0;        // list entries by 0: the TMA ring, 1: direct loads (rows = entries per batch),
                                // 2: staged neighbourhoods (256 threads; rows = entries per batch)
   int pforce_mode = 0;
-  int nlist_mode = 0;          // 0: each lane its own query box; 1: the warp's union of boxes
+  int nlist_mode = 0;          // particles a warp: 0 by the particle count, 1 half as many
 };
 bool shape_valid(const LaunchShape& s, bool batched, const char** why);
 // (mode, threads, rows) triples of the loop passes: TMA ring (mode 0),
@@ -197,6 +197,11 @@ struct System {
   uint32_t* cend = nullptr;
   uint32_t* sstart = nullptr;
   uint32_t* send = nullptr;
+  // both sets in Morton order, for the list build (k_merge_sets): position
+  // and neighbour index (the bits of w), [capacity]; cell start and end,
+  // [2][ncells]
+  float4* mpos = nullptr;
+  uint32_t* mcells = nullptr;
 
   // boundary set
   float4* spos = nullptr;
@@ -284,10 +289,12 @@ struct BatchSystem {
   std::vector<void*> checkpoint_slots;
 };
 
+// upf_pipeline.cu: per-device set-up of the pass kernels (before any launch or capture)
+cudaError_t pipeline_init();
 // upf_pipeline.cu: neighbour lists of one sorted set without boundary set
-cudaError_t launch_nlist_plain(const DevParams& P, uint32_t n, const float4* pos, const uint32_t* keys,
-                               const uint32_t* cstart, const uint32_t* cend, uint32_t* nbr, uint32_t* lval,
-                               uint32_t* ncnt, const float* luts, DevState* st, cudaStream_t stream);
+cudaError_t launch_nlist_plain(const DevParams& P, uint32_t n, const float4* pos, const uint32_t* cstart,
+                               const uint32_t* cend, uint32_t* nbr, uint32_t* ncnt, const float* luts, DevState* st,
+                               cudaStream_t stream);
 
 // upf_pipeline.cu: batched phase launchers (asynchronous on `st`)
 cudaError_t batch_launch_init(BatchSystem& b, cudaStream_t st);   // keys and lagged state after upload
