@@ -248,6 +248,12 @@ LaunchShape config_to_shape(const upf_launch_config& c) {
   return s;
 }
 
+bool same_loop_shapes(const LaunchShape& a, const LaunchShape& b) {
+  return a.density_mode == b.density_mode && a.density_threads == b.density_threads &&
+         a.density_rows == b.density_rows && a.pforce_mode == b.pforce_mode &&
+         a.pforce_threads == b.pforce_threads && a.pforce_rows == b.pforce_rows;
+}
+
 upf_status autotune_shapes(const TuneOps& ops, int repeats, upf_launch_config* out) {
   if (repeats < 1) repeats = 1;
   cudaStream_t st = ops.stream;
@@ -491,17 +497,23 @@ upf_status build_step_graph(System& s) {
     if (e == cudaSuccess && S.prm.method == UPF_METHOD_PCISPH) e = launch_loop_init(S, st);
     return e;
   };
-  if (s.prm.method == UPF_METHOD_PCISPH)
+  s.loop_in_graph = loop_fused(s);
+  if (s.prm.method == UPF_METHOD_PCISPH && !s.loop_in_graph)
     parts.loop = [](void* c, cudaStream_t st, cudaGraphConditionalHandle h) {
       return launch_loop_body(*static_cast<System*>(c), st, h, true);
     };
-  parts.post = [](void* c, cudaStream_t st) { return launch_integrate_phase(*static_cast<System*>(c), st); };
+  parts.post = [](void* c, cudaStream_t st) {
+    System& S = *static_cast<System*>(c);
+    cudaError_t e = S.loop_in_graph ? launch_fused_loop(S, st) : cudaSuccess;
+    return e == cudaSuccess ? launch_integrate_phase(S, st) : e;
+  };
   // capturing runs the launchers' host code without running the kernels:
   // the host-side record of whether the current lists are staged is kept,
   // and whether a step of this graph stages them is noted for upf_step
   const bool staged_now = s.lists_staged;
   const upf_status rc = capture_step_graph(parts, &s.step_graph, &s.step_exec);
   s.graph_stages = s.lists_staged;
+  s.loop_in_graph = false;
   s.lists_staged = staged_now;
   return rc;
 }
@@ -870,7 +882,8 @@ upf_status upf_create(const upf_params* p, int device, uint32_t capacity, upf_sy
   ALLOC(s->mpos, c); ALLOC(s->mcells, (size_t)2 * s->ncells);
   ALLOC(s->spos, c); ALLOC(s->skeys, c); ALLOC(s->sid, c);
   ALLOC(s->luts, 5 * UPF_LUT_ENTRIES + kThresholds);
-  ALLOC(s->st, 1);
+  ALLOC(s->st, 1); ALLOC(s->loop_sync, 2); ALLOC(s->loop_max, 2);
+  s->loop_sms = loop_cooperative_sms();
   if (p->method == UPF_METHOD_PCISPH) {
     // staged neighbourhoods of the loop passes (loop-pass mode 2)
     const size_t chunks = ((size_t)c + kStageChunk - 1) / kStageChunk;
@@ -1575,6 +1588,8 @@ upf_status upf_set_launch_config(upf_system* s, const upf_launch_config* cfg) {
     return UPF_ERR_INVALID_ARG;
   }
   UPF_CUDA(cudaStreamSynchronize(s->stream));
+  // (the shapes in use, given back unchanged, are no choice)
+  s->shape_set = s->shape_set || !same_loop_shapes(s->shape, sh);
   s->shape = sh;
   return s->have_particles ? build_step_graph(*s) : UPF_OK;
 }
@@ -1641,6 +1656,7 @@ upf_status upf_autotune(upf_system* s, int32_t repeats, upf_launch_config* chose
   const upf_status rc = autotune_shapes(ops, repeats, chosen);
   s->stage_always = false;
   UPF_TRY(rc);
+  s->shape_set = false;
   UPF_TRY(check_device_errors(*s));
   return build_step_graph(*s);
 }

@@ -115,10 +115,15 @@ upf_status build_batch_graph(upf_batch* b) {
     if (e == cudaSuccess) e = batch_launch_loop_init(B, st);
     return e;
   };
-  parts.loop = [](void* c, cudaStream_t st, cudaGraphConditionalHandle h) {
-    return batch_capture_loop_body(*static_cast<BatchSystem*>(c), st, h);
+  if (!batch_loop_fused(*b))
+    parts.loop = [](void* c, cudaStream_t st, cudaGraphConditionalHandle h) {
+      return batch_capture_loop_body(*static_cast<BatchSystem*>(c), st, h);
+    };
+  parts.post = [](void* c, cudaStream_t st) {
+    BatchSystem& B = *static_cast<BatchSystem*>(c);
+    cudaError_t e = batch_loop_fused(B) ? batch_launch_fused_loop(B, st) : cudaSuccess;
+    return e == cudaSuccess ? batch_launch_integrate(B, st) : e;
   };
-  parts.post = [](void* c, cudaStream_t st) { return batch_launch_integrate(*static_cast<BatchSystem*>(c), st); };
   return capture_step_graph(parts, &b->step_graph, &b->step_exec);
 }
 
@@ -263,6 +268,8 @@ upf_status upf_batch_create(const upf_params* params, const uint32_t* counts, ui
   ALLOC(b->st_d, num_scenes);
   ALLOC(b->group_scene_d, group_scene.size()); ALLOC(b->seg_begin_d, num_scenes); ALLOC(b->seg_end_d, num_scenes);
   ALLOC(b->cell_base_d, num_scenes); ALLOC(b->any_active_d, 1);
+  ALLOC(b->loop_sync, 2); ALLOC(b->loop_max, (size_t)2 * num_scenes);
+  b->loop_sms = loop_cooperative_sms();
   ALLOC(b->active_groups_d, n / kSegAlign + 1); ALLOC(b->n_active_groups_d, 1);
   ALLOC(b->x.comp_begin_d, num_scenes); ALLOC(b->x.stage_a, std::max<size_t>(total, 1));
   ALLOC(b->x.stage_b, std::max<size_t>(total, 1));
@@ -649,6 +656,7 @@ upf_status upf_batch_set_launch_config(upf_batch* b, const upf_launch_config* cf
     return UPF_ERR_INVALID_ARG;
   }
   UPF_CUDA(cudaStreamSynchronize(b->stream));
+  b->shape_set = b->shape_set || !same_loop_shapes(b->shape, sh);
   b->shape = sh;
   return b->have_particles ? build_batch_graph(b) : UPF_OK;
 }

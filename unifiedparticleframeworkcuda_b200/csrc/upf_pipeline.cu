@@ -1756,7 +1756,9 @@ __global__ void __launch_bounds__(kStageChunk, pforce_staged_min_blocks(kRows)) 
   if (bad) atomicOr(&st->error_flags, (uint32_t)ERR_NAN);
 }
 
-__global__ void k_loop_init(DevState* st) {
+__global__ void k_loop_init(DevState* st, unsigned long long* sync, uint32_t* loop_max) {
+  sync[0] = 0;  // arrivals at the fused loop's barrier
+  loop_max[0] = loop_max[1] = 0;
   st->iteration = 0;
   st->too_large = 1;
   st->max_rho_bits = 0;
@@ -1774,32 +1776,344 @@ __global__ void k_step_init(DevState* st, int count_step) {
 // Loop control of PredictionCorrectionStep (UnifiedPhysics.cpp:5376-5420):
 // continue while iteration < min_loops, or the error is still too large and
 // iteration < max_loops. The "too large" flag is sticky-false, as in the
-// reference. Runs on the device and feeds the graph's conditional node.
-__device__ __forceinline__ int loop_ctl(const DevParams& P, DevState* st) {
-  const int it = st->iteration + 1;
+// reference. Runs on the device. First half: iteration `it` (from 1) has its
+// maximum density; the record of it, and the flag.
+__device__ __forceinline__ void loop_note(const DevParams& P, DevState* st, int it, uint32_t max_rho_bits) {
   st->iteration = it;
-  const float maxd = __uint_as_float(st->max_rho_bits);
+  const float maxd = __uint_as_float(max_rho_bits);
   const float e = mx0(P.err_scale * maxd - 100.0f, 0.0f);
   if (it <= 64) st->iter_max_rho[it - 1] = maxd;
   if (e < P.max_err) st->too_large = 0;
-  int cont = (it < P.min_loops) || (st->too_large && it < P.max_loops);
-  if (st->error_flags & ERR_NAN) cont = 0;
   st->final_iterations = it;
   st->final_max_rho = maxd;
   st->final_err = e;
   st->max_rho_bits = 0;
-  if (!cont) {
-    st->total_steps += 1;
-    st->total_iterations += it;
-    if (it >= P.max_loops) st->steps_at_max += 1;
-    if (e > st->max_step_err) st->max_step_err = e;
-  }
+}
+
+// Second half: whether the loop goes on after iteration `it`.
+__device__ __forceinline__ bool loop_goes_on(const DevParams& P, int it, int too_large, uint32_t error_flags) {
+  return ((it < P.min_loops) || (too_large && it < P.max_loops)) && !(error_flags & ERR_NAN);
+}
+
+// The step's count, when the loop has ended after iteration `it`.
+__device__ __forceinline__ void loop_end(const DevParams& P, DevState* st, int it) {
+  st->total_steps += 1;
+  st->total_iterations += it;
+  if (it >= P.max_loops) st->steps_at_max += 1;
+  if (st->final_err > st->max_step_err) st->max_step_err = st->final_err;
+}
+
+// The loop test as a pass of its own; feeds the graph's conditional node.
+__device__ __forceinline__ int loop_ctl(const DevParams& P, DevState* st) {
+  const int it = st->iteration + 1;
+  loop_note(P, st, it, st->max_rho_bits);
+  const int cont = loop_goes_on(P, it, st->too_large, st->error_flags);
+  if (!cont) loop_end(P, st, it);
   return cont;
 }
 
 __global__ void k_loop_ctl(DevParams P, DevState* st, cudaGraphConditionalHandle h, int use_handle) {
   const int cont = loop_ctl(P, st);
   if (use_handle) cudaGraphSetConditional(h, cont ? 1u : 0u);
+}
+
+// ---------------------------------------------------------------- fused loop
+// The whole predict-correct loop in one cooperative launch: the density and
+// pressure-force passes of density_block and pforce_block with a grid
+// barrier between them, the loop test done by the grid itself. For as many
+// particles as the SMs hold at once (151,552 on a B200) an iteration of three
+// graph nodes is mostly the nodes: their launches, drains and cold starts,
+// and gathers with few warps to hide them. A step of 50 iterations, before
+// and now (sort, lists and forces included, about 0.12 ms): 1,728 particles
+// 1.15 and 0.36 ms, 8,000 1.31 and 0.54, 32,768 1.31 and 0.82, 53,157 1.44
+// and 1.19, 144,256 2.01 and 1.62. Above that several chunks a CTA came to
+// 2.87 ms at 196,608 against 2.73 with the passes as launches of their own
+// (3.45 and 3.23 at 262,144), so those keep the launches.
+// kLanes: lanes a particle. With few particles one thread each leaves an SM a
+// warp or two, and an iteration is their 3,000 instructions one after the
+// other; instead kLanes lanes compute the terms of every kLanes-th list entry
+// and put them in shared memory, where they are added in list order (a lane
+// per component), so that every sum keeps the reference's order.
+// kHeld: list entries a particle keeps in shared memory for the whole loop
+// (the barrier's acquire empties L1, so lists left there would come from L2
+// in every pass); longer lists go on from global memory.
+// A CTA keeps to its particles, whose own data stays in registers. A batch's
+// scenes end their loops one by one; the CTAs of a finished scene
+// only keep the barrier.
+constexpr uint64_t kGridWaitLimitNs = 4000000000ull;
+
+// Every CTA of the (cooperative) grid arrives, adding `add` to the counter
+// (1, or 1 and a mark in the upper half), and waits until the lower half
+// reaches `target`. What was written before is then seen by plain loads
+// everywhere (release, acquire and the CTA barriers). Returns the counter, 0
+// if the wait ran out.
+__device__ __forceinline__ unsigned long long grid_wait(unsigned long long* arrived, unsigned long long add,
+                                                        uint32_t target) {
+  __shared__ unsigned long long seen_all;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(arrived), "l"(add) : "memory");
+    unsigned long long seen = 0;
+    uint64_t t0 = 0;
+    for (uint32_t s = 0; s < kWaitSpins; ++s) {
+      asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(seen) : "l"(arrived) : "memory");
+      if ((uint32_t)seen >= target) break;
+      if ((s & 63u) == 63u) {
+        const uint64_t t = globaltimer_ns();
+        if (!t0) t0 = t;
+        if (t - t0 > kGridWaitLimitNs) break;
+      }
+    }
+    seen_all = (uint32_t)seen >= target ? seen : 0ull;
+  }
+  __syncthreads();
+  return seen_all;
+}
+
+// Threads an SM, at 64 registers.
+constexpr int kLoopResident = 1024;
+template <int kThreads, int kLanes, int kHeld, int kRows>
+constexpr size_t loop_smem() {
+  constexpr int particles = kThreads / kLanes;
+  return sizeof(uint32_t) * ((size_t)2 * kHeld * particles +
+                             (kLanes > 1 ? (size_t)3 * kLanes * kRows * particles : 0));
+}
+
+template <bool kBatch, int kThreads, int kResident, int kLanes, int kHeld, int kRows>
+__global__ void __launch_bounds__(kThreads, kResident / kThreads) k_pcisph_loop(
+    const __grid_constant__ DevParams Pk, const BatchView bv, const uint32_t* __restrict__ seg_begin, uint32_t n,
+    DynArrays B, const uint32_t* __restrict__ nbr, const uint32_t* __restrict__ lval,
+    const uint32_t* __restrict__ ncnt, const float* __restrict__ luts_plain, const float4* __restrict__ force,
+    float4* pforce, float4* xs, float* rho, float* press, float4* pq, DevState* st_plain,
+    unsigned long long* sync, uint32_t* loop_max) {
+  constexpr uint32_t kChunk = kThreads / kLanes;  // particles a CTA
+  static_assert(!kBatch || kSegAlign % kChunk == 0, "a CTA's particles lie in one scene");
+  constexpr uint32_t kPer = 32 / kLanes;          // particles a warp
+  constexpr uint32_t kTerms = kLanes * kRows;     // entries of a particle at a time
+  extern __shared__ uint32_t loop_mem[];
+  uint32_t* const held = loop_mem;                                   // [2 kHeld][kChunk] entries, then their values
+  __shared__ DevParams sP;
+  __shared__ float m4[UPF_LUT_ENTRIES];
+  __shared__ uint32_t wmax[kThreads / 32];
+  __shared__ int s_goes_on;
+  const Scope sc = enter_scope_slot<kBatch>(blockIdx.x * kChunk, Pk, luts_plain, st_plain, n, bv, &sP, false);
+  const float mass = kBatch ? __ldg(&bv.params[sc.scene].mass) : Pk.mass;
+  // the table times the mass, as in density_block
+  for (int k = threadIdx.x; k < UPF_LUT_ENTRIES; k += kThreads)
+    m4[k] = fmul(__ldg(sc.luts + LUT_M4 * UPF_LUT_ENTRIES + k), mass);
+  const float r2_edge = __ldg(sc.luts + 5 * UPF_LUT_ENTRIES + kLut);
+  __syncthreads();
+  const DevParams& P = *sc.P;
+  DevState* st = sc.st;
+  const bool leader = threadIdx.x == 0 && (kBatch ? blockIdx.x * kChunk == __ldg(seg_begin + sc.scene)
+                                                  : blockIdx.x == 0);
+  const uint32_t stride = P.nstride;
+  const float m = P.mass, rho0sq = P.rho0 * P.rho0;
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t sub = lane % kLanes, own = threadIdx.x / kLanes;  // lane of its particle, particle of the CTA
+  const uint32_t lead = lane - sub;                                // the particle's first lane
+  // the warp's terms: component c of entry e of its particle q at
+  // [c * kTerms * kPer + (e / 4) * 4 * kPer + 4 * q + e % 4], four entries of
+  // one particle side by side; missing entries are zeros (adding or taking
+  // off a zero changes no sum)
+  static_assert(kLanes == 1 || (kLanes > 3 && kTerms % 4 == 0), "a lane per component; terms read four at a time");
+  float* const terms = reinterpret_cast<float*>(loop_mem + 2 * kHeld * kChunk) +
+                       (threadIdx.x / 32) * (3 * kTerms * kPer) + 4 * (lane / kLanes);
+  auto term_at = [&](uint32_t e) { return terms + (e / 4) * 4 * kPer + e % 4; };
+  // the particle's own data (den and p: its first lane's); its position and
+  // forces are read again where they are used
+  const uint32_t i = blockIdx.x * kChunk + own;
+  const bool active = i < sc.end && B.type[i] == UPF_LIQUID;
+  const uint32_t cnt = active ? ncnt[i] : 0u;
+  float4 xstar = active ? xs[i] : make_float4(0, 0, 0, 0);
+  float p = active ? press[i] : 0.0f;
+  bool bad_any = false;
+  auto code_at = [&](uint32_t k) {
+    return kHeld && k < (uint32_t)kHeld ? held[k * kChunk + own] : __ldg(nbr + (size_t)k * stride + i);
+  };
+  auto value_at = [&](uint32_t k) {
+    return __uint_as_float(kHeld && k < (uint32_t)kHeld ? held[(kHeld + k) * kChunk + own]
+                                                        : __ldg(lval + (size_t)k * stride + i));
+  };
+  auto density = [&]() {
+    float den = P.kernel_self * m;
+    const unsigned long long xiy = pk2(xstar.x, xstar.y);
+    auto term = [&](float4 xj) { return m4[bin_of_r2_edge(dist2_xy(xiy, xstar.z, xj), P.lut_factor, r2_edge)]; };
+    const uint32_t walk = kLanes > 1 ? __reduce_max_sync(0xffffffffu, cnt) : cnt;
+    for (uint32_t k0 = 0; k0 < walk; k0 += kTerms) {
+      float4 xj[kRows];
+#pragma unroll
+      for (int r = 0; r < kRows; ++r)
+        if (k0 + r * kLanes + sub < cnt) xj[r] = xs[code_at(k0 + r * kLanes + sub)];
+      if (kLanes == 1) {
+#pragma unroll
+        for (int r = 0; r < kRows; ++r)
+          if (k0 + r < cnt) den += term(xj[r]);
+      } else {
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+          const uint32_t e = r * kLanes + sub;
+          *term_at(e) = k0 + e < cnt ? term(xj[r]) : 0.0f;
+        }
+        __syncwarp();
+        if (sub == 0) {
+#pragma unroll
+          for (uint32_t e = 0; e < kTerms; e += 4) {
+            const float4 t = *reinterpret_cast<const float4*>(term_at(e));
+            den += t.x;
+            den += t.y;
+            den += t.z;
+            den += t.w;
+          }
+        }
+        __syncwarp();
+      }
+    }
+    if (!active || sub) return 0u;
+    const float err = mx0(den - P.rho0, 0.0f);
+    p = p + mx0(err * P.delta, 0.0f);
+    reinterpret_cast<float*>(pq + i)[3] = p / rho0sq;
+    press[i] = p;
+    rho[i] = den;
+    return __float_as_uint(den);
+  };
+  auto pressure_force = [&]() {
+    const float4 x = active ? B.pos[i] : make_float4(0, 0, 0, 0);
+    float f[3] = {0, 0, 0};
+    float fc = 0;  // with several lanes a particle, lane c's sum is component c
+    float qi = p / rho0sq;
+    if (kLanes > 1) qi = __shfl_sync(0xffffffffu, qi, lead);
+    const uint32_t walk = kLanes > 1 ? __reduce_max_sync(0xffffffffu, cnt) : cnt;
+    auto subtract = [&](float& sum, uint32_t c) {
+#pragma unroll
+      for (uint32_t e = 0; e < kTerms; e += 4) {
+        const float4 t = *reinterpret_cast<const float4*>(term_at(e) + c * (kTerms * kPer));
+        sum = sum - t.x;
+        sum = sum - t.y;
+        sum = sum - t.z;
+        sum = sum - t.w;
+      }
+    };
+    for (uint32_t k0 = 0; k0 < walk; k0 += kTerms) {
+      float4 xj[kRows];
+      float g[kRows];
+#pragma unroll
+      for (int r = 0; r < kRows; ++r)
+        if (k0 + r * kLanes + sub < cnt) {
+          xj[r] = pq[code_at(k0 + r * kLanes + sub)];
+          g[r] = value_at(k0 + r * kLanes + sub);
+        }
+#pragma unroll
+      for (int r = 0; r < kRows; ++r) {
+        const uint32_t e = r * kLanes + sub;
+        float tx = 0.0f, ty = 0.0f, tz = 0.0f;
+        if (k0 + e < cnt) {
+          // scalar arithmetic, as in pforce_block
+          const float kx = (x.x - xj[r].x) * g[r], ky = (x.y - xj[r].y) * g[r], kz = (x.z - xj[r].z) * g[r];
+          const float grad = qi + xj[r].w;
+          tx = kx * grad * m * m;
+          ty = ky * grad * m * m;
+          tz = kz * grad * m * m;
+        }
+        if (kLanes == 1) {
+          f[0] = f[0] - tx;
+          f[1] = f[1] - ty;
+          f[2] = f[2] - tz;
+        } else {
+          float* t = term_at(e);
+          t[0] = tx;
+          t[kTerms * kPer] = ty;
+          t[2 * kTerms * kPer] = tz;
+        }
+      }
+      if (kLanes > 1) {
+        __syncwarp();
+        if (sub < 3) subtract(fc, sub);
+        __syncwarp();
+      }
+    }
+    if (kLanes > 1) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) f[c] = __shfl_sync(0xffffffffu, fc, lead + c);
+    }
+    if (!active) return;
+    if (sub == 0) pforce[i] = f4(f[0], f[1], f[2]);
+    const float4 F = force[i];
+    bool bad;
+    xstar = predict(P, x, B.vel[i], make_float3(F.x, F.y, F.z), make_float3(f[0], f[1], f[2]), bad);
+    if (sub == 0) xs[i] = xstar;
+    if (bad) {
+      bad_any = true;
+      atomicOr(&st->error_flags, (uint32_t)ERR_NAN);
+    }
+  };
+  uint32_t target = 0;
+  bool runs = true;  // the CTA's scene still iterates
+  int too_large = 1;  // thread 0
+  const bool nan_before = *reinterpret_cast<volatile uint32_t*>(&st->error_flags) & ERR_NAN;
+  if constexpr (kHeld > 0) {
+#pragma unroll 4
+    for (uint32_t k = sub; k < (uint32_t)kHeld; k += kLanes)
+      if (k < cnt) {
+        held[k * kChunk + own] = __ldg(nbr + (size_t)k * stride + i);
+        held[(kHeld + k) * kChunk + own] = __ldg(lval + (size_t)k * stride + i);
+      }
+    __syncwarp();
+  }
+  for (int it = 1;; ++it) {
+    uint32_t best = runs ? density() : 0u;
+    // the maximum over the scene, in one of two places in turn (the other is
+    // cleared while this one is read)
+    uint32_t* const maxima = loop_max + 2 * sc.scene;
+    best = __reduce_max_sync(0xffffffffu, best);
+    if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = best;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+      for (int w = 1; w < kThreads / 32; ++w) best = max(best, wmax[w]);
+      if (best) atomicMax(&maxima[it & 1], best);  // densities are positive: uint order == float order
+    }
+    if (!grid_wait(sync, 1ull, target += gridDim.x)) break;
+    uint32_t maximum = 0;
+    if (threadIdx.x == 0 && runs) {
+      maximum = *reinterpret_cast<volatile uint32_t*>(&maxima[it & 1]);
+      if (leader) maxima[(it + 1) & 1] = 0;
+    }
+    if (kBatch && !runs) {
+      // (every CTA sees the same count: it changes after the second barrier only)
+      if (threadIdx.x == 0) s_goes_on = *reinterpret_cast<volatile unsigned long long*>(sync + 1) != 0;
+      __syncthreads();
+      if (!s_goes_on) return;
+    }
+    if (runs) pressure_force();
+    const bool bad_cta = __syncthreads_or(bad_any);
+    const unsigned long long seen = grid_wait(sync, bad_cta ? (1ull << 32) + 1ull : 1ull, target += gridDim.x);
+    if (!seen) break;
+    if (!runs) continue;
+    if (threadIdx.x == 0) {
+      // the loop test; a batch's NaN is its own scene's
+      uint32_t flags = nan_before || (!kBatch && (seen >> 32)) ? (uint32_t)ERR_NAN : 0u;
+      if (kBatch && (seen >> 32)) flags |= *reinterpret_cast<volatile uint32_t*>(&st->error_flags);
+      const float e = mx0(P.err_scale * __uint_as_float(maximum) - 100.0f, 0.0f);
+      if (e < P.max_err) too_large = 0;
+      s_goes_on = loop_goes_on(P, it, too_large, flags);
+      if (leader) loop_note(P, st, it, maximum);
+    }
+    __syncthreads();
+    if (!s_goes_on) {
+      runs = false;
+      if (leader) {
+        loop_end(P, st, it);
+        if (kBatch) {
+          st->loop_active = 0;
+          atomicAdd(sync + 1, ~0ull);  // one running scene fewer
+        }
+      }
+      if (!kBatch) return;
+    }
+  }
+  // a wait ran out
+  if (threadIdx.x == 0) atomicOr(&st->error_flags, (uint32_t)ERR_TIMEOUT);
 }
 
 // ---------------------------------------------------------------- batched scenes
@@ -1874,11 +2188,17 @@ __global__ void k_step_init_batch(DevState* st, uint32_t nscenes) {
   }
 }
 
-__global__ void k_loop_init_batch(DevState* st, uint32_t nscenes, int32_t* any_active) {
+__global__ void k_loop_init_batch(DevState* st, uint32_t nscenes, int32_t* any_active,
+                                  unsigned long long* sync, uint32_t* loop_max) {
+  if (threadIdx.x == 0) {
+    sync[0] = 0;        // arrivals at the fused loop's barrier
+    sync[1] = nscenes;  // scenes whose loop still runs
+  }
   for (uint32_t s = threadIdx.x; s < nscenes; s += blockDim.x) {
     st[s].iteration = 0;
     st[s].too_large = 1;
     st[s].max_rho_bits = 0;
+    loop_max[2 * s] = loop_max[2 * s + 1] = 0;
     st[s].loop_active = 1;
   }
   if (threadIdx.x == 0) *any_active = nscenes > 0;
@@ -2178,6 +2498,23 @@ static cudaError_t nlist_opt_in() {
                               (int)nlist_smem<256, 32>());
 }
 
+// Likewise the fused loop's.
+template <bool kBatch, int kThreads, int kResident, int kLanes, int kHeld, int kRows>
+static cudaError_t loop_opt_in_shape() {
+  return cudaFuncSetAttribute(k_pcisph_loop<kBatch, kThreads, kResident, kLanes, kHeld, kRows>,
+                              cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)loop_smem<kThreads, kLanes, kHeld, kRows>());
+}
+template <bool kBatch>
+static cudaError_t loop_opt_in() {
+  cudaError_t e = loop_opt_in_shape<kBatch, 512, 1024, 32, 48, 1>();
+  if (e == cudaSuccess) e = loop_opt_in_shape<kBatch, 512, 1024, 16, 48, 2>();
+  if (e == cudaSuccess) e = loop_opt_in_shape<kBatch, 512, 1024, 8, 48, 4>();
+  if (e == cudaSuccess) e = loop_opt_in_shape<kBatch, 512, 1024, 4, 48, 4>();
+  if (e == cudaSuccess) e = loop_opt_in_shape<kBatch, 128, 512, 1, 48, 8>();
+  return e;
+}
+
 cudaError_t pipeline_init() {
   static std::mutex mu;
   static bool done[64] = {};
@@ -2189,6 +2526,8 @@ cudaError_t pipeline_init() {
   if ((e = nlist_opt_in<false, false>()) != cudaSuccess) return e;
   if ((e = nlist_opt_in<false, true>()) != cudaSuccess) return e;
   if ((e = nlist_opt_in<true, false>()) != cudaSuccess) return e;
+  if ((e = loop_opt_in<false>()) != cudaSuccess) return e;
+  if ((e = loop_opt_in<true>()) != cudaSuccess) return e;
   if (dev >= 0 && dev < 64) done[dev] = true;
   return cudaSuccess;
 }
@@ -2223,7 +2562,7 @@ cudaError_t launch_list_staging(System& s, cudaStream_t st) {
 // the lists are staged when a loop pass reads staged neighbourhoods (or
 // while the autotuner times every mode)
 static bool stages_lists(const System& s) {
-  return s.ucodes && (s.stage_always || loop_mode_staged(s.shape.density_mode) ||
+  return s.ucodes && !s.loop_in_graph && (s.stage_always || loop_mode_staged(s.shape.density_mode) ||
                       loop_mode_staged(s.shape.pforce_mode));
 }
 
@@ -2264,9 +2603,73 @@ cudaError_t launch_force_phase(System& s, cudaStream_t st) {
 }
 
 cudaError_t launch_loop_init(System& s, cudaStream_t st) {
-  k_loop_init<<<1, 1, 0, st>>>(s.st);
+  k_loop_init<<<1, 1, 0, st>>>(s.st, s.loop_sync, s.loop_max);
   return cudaGetLastError();
 }
+
+// The fused loop's shape for n particles (or slots): as many lanes a particle
+// as the SMs hold at once (1,024 threads each), in CTAs of 512, since the
+// barrier's cost is its arrivals (4,096 particles in 1,024 CTAs of 128: 11.8
+// us an iteration, in 256 of 512 5.8); one lane a particle in small CTAs at
+// first, to use every SM.
+template <bool kBatch, int kThreads, int kResident, int kLanes, int kHeld, int kRows>
+static cudaError_t run_loop_shape(cudaStream_t st, uint32_t n, void** args) {
+  constexpr uint32_t chunk = kThreads / kLanes;
+  return cudaLaunchCooperativeKernel((const void*)k_pcisph_loop<kBatch, kThreads, kResident, kLanes, kHeld, kRows>,
+                                     dim3((n + chunk - 1) / chunk), dim3(kThreads), args,
+                                     loop_smem<kThreads, kLanes, kHeld, kRows>(), st);
+}
+
+template <bool kBatch>
+static cudaError_t run_loop(cudaStream_t st, const DevParams& P, const BatchView& bv, const uint32_t* seg_begin,
+                            uint32_t n, DynArrays B, const uint32_t* nbr, const uint32_t* lval, const uint32_t* ncnt,
+                            const float* luts, const float4* force, float4* pforce, float4* xs, float* rho,
+                            float* press, float4* pq, DevState* stp, unsigned long long* sync, uint32_t* loop_max,
+                            uint32_t sms) {
+  void* args[] = {(void*)&P,    (void*)&bv,   (void*)&seg_begin, (void*)&n,     (void*)&B,      (void*)&nbr,
+                  (void*)&lval, (void*)&ncnt, (void*)&luts,      (void*)&force, (void*)&pforce, (void*)&xs,
+                  (void*)&rho,  (void*)&press, (void*)&pq,       (void*)&stp,   (void*)&sync,   (void*)&loop_max};
+  if (n <= sms * 32) return run_loop_shape<kBatch, 512, 1024, 32, 48, 1>(st, n, args);
+  if (n <= sms * 64) return run_loop_shape<kBatch, 512, 1024, 16, 48, 2>(st, n, args);
+  if (n <= sms * 128) return run_loop_shape<kBatch, 512, 1024, 8, 48, 4>(st, n, args);
+  if (n <= sms * 256) return run_loop_shape<kBatch, 512, 1024, 4, 48, 4>(st, n, args);
+  if (n <= sms * 512) return run_loop_shape<kBatch, 128, 512, 1, 48, 8>(st, n, args);
+  // (a batch's CTA takes no more than the 256 slots that are of one scene)
+  if (n <= sms * 1024) return run_loop_shape<kBatch, kBatch ? 256 : 512, 1024, 1, 0, 4>(st, n, args);
+  return cudaErrorInvalidConfiguration;
+}
+
+// The current device's SM count, where it launches cooperative grids (0
+// elsewhere).
+uint32_t loop_cooperative_sms() {
+  int dev = 0, sms = 0, coop = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return (uint32_t)sms;
+}
+
+bool loop_fused(const System& s) {
+  return s.prm.method == UPF_METHOD_PCISPH && !s.shape_set && s.n_dyn && s.n_dyn <= s.loop_sms * kLoopResident;
+}
+
+cudaError_t launch_fused_loop(System& s, cudaStream_t st) {
+  return run_loop<false>(st, s.dp, BatchView{}, nullptr, s.n_dyn, s.B, s.nbr, s.lval, s.ncnt, s.luts, s.force,
+                         s.pforce, s.xs, s.rho, s.press, s.pq, s.st, s.loop_sync, s.loop_max, s.loop_sms);
+}
+
+bool batch_loop_fused(const BatchSystem& b) {
+  return !b.shape_set && b.n_slots && b.n_slots <= b.loop_sms * kLoopResident;
+}
+
+cudaError_t batch_launch_fused_loop(BatchSystem& b, cudaStream_t st) {
+  return run_loop<true>(st, DevParams{}, b.view, b.seg_begin_d, b.n_slots, b.B, b.nbr, b.lval, b.ncnt, nullptr, b.force,
+                        b.pforce, b.xs, b.rho, b.press, b.pq, nullptr, b.loop_sync, b.loop_max, b.loop_sms);
+}
+
 
 cudaError_t launch_loop_density(System& s, cudaStream_t st) {
   const uint32_t n = s.n_dyn;
@@ -2429,7 +2832,7 @@ cudaError_t batch_launch_forces(BatchSystem& b, cudaStream_t st) {
 }
 
 cudaError_t batch_launch_loop_init(BatchSystem& b, cudaStream_t st) {
-  k_loop_init_batch<<<1, 256, 0, st>>>(b.st_d, b.n_scenes, b.any_active_d);
+  k_loop_init_batch<<<1, 256, 0, st>>>(b.st_d, b.n_scenes, b.any_active_d, b.loop_sync, b.loop_max);
   return cudaGetLastError();
 }
 

@@ -219,6 +219,12 @@ struct System {
   cudaGraphExec_t step_exec = nullptr;
   cudaGraph_t step_graph = nullptr;
   int key_bits = 30;
+  // the predict-correct loop as one cooperative launch (k_pcisph_loop)
+  unsigned long long* loop_sync = nullptr;  // [2] its barrier
+  uint32_t* loop_max = nullptr;   // [2] the maximum predicted density of odd and even iterations
+  uint32_t loop_sms = 0;          // the device's SMs (0: no cooperative launches)
+  bool shape_set = false;         // the caller chose the loop passes' shapes: they run as launches of their own
+  bool loop_in_graph = false;     // the step graph being captured has the fused loop: no staging
 
   RigidArrays rb;
   std::vector<void*> rigid_allocations;   // freed when bodies are set again
@@ -280,6 +286,10 @@ struct BatchSystem {
   uint32_t* active_groups_d = nullptr;  // [n_slots / kSegAlign] groups of the scenes still iterating
   uint32_t* n_active_groups_d = nullptr;
   uint32_t active_grid = 0;             // resident CTAs of the active-group passes
+  unsigned long long* loop_sync = nullptr;  // as System's: the fused loop's barrier, and its running scenes
+  uint32_t* loop_max = nullptr;             // [scenes][2]
+  uint32_t loop_sms = 0;
+  bool shape_set = false;
   BatchView view;
 
   cudaGraphExec_t step_exec = nullptr;
@@ -358,6 +368,7 @@ struct TuneOps {
 upf_status autotune_shapes(const TuneOps& ops, int repeats, upf_launch_config* out);
 void shape_to_config(const LaunchShape& s, upf_launch_config* c);
 LaunchShape config_to_shape(const upf_launch_config& c);
+bool same_loop_shapes(const LaunchShape& a, const LaunchShape& b);
 
 // upf_rigid.cu: list entry -> sorted index after a sort; body force/torque,
 // body integration and rigid particle sync after integration
@@ -378,6 +389,13 @@ cudaError_t launch_loop_body(System& s, cudaStream_t st, cudaGraphConditionalHan
 cudaError_t launch_loop_density(System& s, cudaStream_t st);
 cudaError_t launch_loop_pforce(System& s, cudaStream_t st);
 cudaError_t launch_loop_ctl(System& s, cudaStream_t st, cudaGraphConditionalHandle h, bool use_handle);
+// the whole loop in one cooperative launch: whether a step graph of this
+// system (batch) takes it, the launch, and the SM count it is sized by
+bool loop_fused(const System& s);
+cudaError_t launch_fused_loop(System& s, cudaStream_t st);
+bool batch_loop_fused(const BatchSystem& b);
+cudaError_t batch_launch_fused_loop(BatchSystem& b, cudaStream_t st);
+uint32_t loop_cooperative_sms();
 cudaError_t launch_list_staging(System& s, cudaStream_t st);  // k_stage_lists over the current lists
 cudaError_t launch_upload_keys(System& s, cudaStream_t st);
 cudaError_t launch_integrate_phase(System& s, cudaStream_t st);
