@@ -548,7 +548,7 @@ def batch_cpu_baseline(scs, seconds):
     nsample = sum(sc.n for sc in sample)
     pps = nsample * steps / dt
     mean_n = sum(sc.n for sc in scs) / len(scs)
-    return {"value": pps / mean_n, "unit": "scene-steps/s", "cores": threads, "kind": "port",
+    return {"value": pps / mean_n, "unit": "scene-steps/s", "cores": threads, "kind": "port", "cpu_model": cpu_model(),
             "sample": "%d of %d scenes (%d particles), %d steps, %.1f s: %.3g particle-steps/s over the batch's "
                       "mean scene size %.0f" % (len(sample), len(scs), nsample, steps, dt, pps, mean_n)}
 
