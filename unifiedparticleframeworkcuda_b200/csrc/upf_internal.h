@@ -62,7 +62,7 @@ size_t radix_temp_bytes(uint32_t n);
 cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt,
                              uint32_t* counts, uint32_t n, int key_bits, bool iota_values,
                              cudaStream_t st);
-int radix_launches(int key_bits);
+int radix_launches(uint32_t n, int key_bits);
 cudaError_t radix_init();
 cudaError_t morton_keys(const float4* pos, uint32_t n, float3 origin, float3 scales, uint32_t* keys,
                         cudaStream_t st);

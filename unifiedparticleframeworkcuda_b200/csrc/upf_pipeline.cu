@@ -2964,7 +2964,7 @@ cudaError_t batch_launch_integrate(BatchSystem& b, cudaStream_t st) {
 }
 
 int pipeline_launches_per_step(const System& s, int iterations) {
-  int sort = radix_launches(s.key_bits) + 1 /*reorder*/ + 1 /*cells*/ + (s.rb.n_rigid ? 1 : 0) /*rigid slots*/;
+  int sort = radix_launches(s.n_dyn, s.key_bits) + 1 /*reorder*/ + 1 /*cells*/ + (s.rb.n_rigid ? 1 : 0) /*rigid slots*/;
   // step init + neighbour lists (+ merge of the two sets, + staging)
   int nl = 2 + (s.n_static ? 1 : 0) + (stages_lists(s) ? 1 : 0);
   if (s.prm.method == UPF_METHOD_WCSPH) return sort + nl + 2;
