@@ -875,7 +875,7 @@ upf_status upf_create(const upf_params* p, int device, uint32_t capacity, upf_sy
   ALLOC(s->force, c); ALLOC(s->pforce, c); ALLOC(s->xs, ct);
   ALLOC(s->rho, ct); ALLOC(s->press, ct); ALLOC(s->pq, ct); ALLOC(s->wvol, ct);
   ALLOC(s->nbr, (size_t)s->nstride * p->max_neighbors);
-  ALLOC(s->lval, (size_t)s->nstride * p->max_neighbors);
+  ALLOC(s->lval, (size_t)s->nstride * ((p->max_neighbors + 3) & ~3u));
   ALLOC(s->ncnt, c);
   ALLOC(s->cstart, s->ncells); ALLOC(s->cend, s->ncells);
   ALLOC(s->sstart, s->ncells); ALLOC(s->send, s->ncells);
@@ -1657,6 +1657,7 @@ upf_status upf_autotune(upf_system* s, int32_t repeats, upf_launch_config* chose
   s->stage_always = false;
   UPF_TRY(rc);
   s->shape_set = false;
+  s->shape_tuned = true;
   UPF_TRY(check_device_errors(*s));
   return build_step_graph(*s);
 }

@@ -152,28 +152,44 @@ __device__ __forceinline__ int bin_of_r2(float r2, float factor, const float* th
 }
 
 // The same bin without reading the threshold table per pair. The bin
-// position x = r2 * rsqrtf(r2) * factor * 300 lies within 300 * (2^-21 +
+// position x = r2 * rsqrtf(r2) * (factor * 300) lies within 300 * (2^-21 +
 // 2^-22) < 2.2e-4 of the reference's sqrt_rn(r2) * factor * 300 (rsqrtf
-// within 2 ulp, two more roundings here, three there), so wherever x is at
+// within 2 ulp, three more roundings here, three there), so wherever x is at
 // least kBinEdge = 2^-10 from an integer both truncate to the same bin; only
 // within kBinEdge of a bin edge (about 0.2% of pairs, or a non-finite x)
 // does the correctly rounded root decide. r2_edge is thr[300], the first r2
 // that takes the zero entry: pairs from there on return 300 exactly as
-// bin_of_r2 does.
+// bin_of_r2 does (x is then 300 to within the same 2.2e-4, or more).
+// x is truncated by adding 1.5 * 2^23 to x - 1/2: the sum's low bits are the
+// bin, without the conversions to an integer and back (which share a quarter
+// rate unit with the root).
 constexpr float kBinEdge = 1.0f / 1024.0f;
 __device__ __forceinline__ float rsqrt_approx(float x) {
   float r;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));  // within 2 ulp
   return r;
 }
+struct BinGuess {
+  int bin;
+  bool sure;
+};
+__device__ __forceinline__ BinGuess bin_guess(float r2, float factor) {
+  // (a subnormal r2 flushes to 0 in the root: x is then NaN or infinite; the
+  // minimum keeps a NaN, and both leave the guess unsure or at 300)
+  const float y = __fmaf_rn(fmul(r2, rsqrt_approx(r2)), fmul(factor, (float)kLut), -0.5f);
+  float yc;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(yc) : "f"(y), "f"((float)kLut));
+  const float t = fadd(yc, 12582912.0f);
+  return BinGuess{__float_as_int(t) - 0x4B400000, fabsf(fsub(yc, fsub(t, 12582912.0f))) <= 0.5f - kBinEdge};
+}
+// the bin where the guess is not sure
+__device__ __forceinline__ int bin_exactly(float r2, float factor, float r2_edge) {
+  const int g = lut_index(__fsqrt_rn(r2), factor);
+  return r2 < r2_edge ? (g > kLut - 1 ? kLut - 1 : g) : kLut;
+}
 __device__ __forceinline__ int bin_of_r2_edge(float r2, float factor, float r2_edge) {
-  // (a subnormal r2 flushes to 0 in the root: x is then NaN or infinite, and
-  // the exact root decides)
-  const float x = r2 * rsqrt_approx(r2) * factor * (float)kLut;
-  int g = (int)x;
-  if (!(fabsf(x - (float)g - 0.5f) <= 0.5f - kBinEdge)) g = lut_index(__fsqrt_rn(r2), factor);
-  g = g > kLut - 1 ? kLut - 1 : g;
-  return r2 < r2_edge ? g : kLut;
+  const BinGuess b = bin_guess(r2, factor);
+  return b.sure ? b.bin : bin_exactly(r2, factor, r2_edge);
 }
 
 // PCISPH dist_lut: uint(dist * 300 / h), clamped to 300

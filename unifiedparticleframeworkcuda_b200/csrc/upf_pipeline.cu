@@ -220,6 +220,27 @@ __device__ __forceinline__ bool walk_lists(const ListArgs& L, uint32_t block, ui
   }
 }
 
+// The density table's bins of kR squared distances: the guesses, and one
+// branch for all that are not sure (a branch per pair cost three instructions
+// for each of them).
+constexpr float kFar2 = 1e30f;  // a squared distance of bin 300, whose zero changes no sum
+template <int kR>
+__device__ __forceinline__ void density_bins(const float (&r2)[kR], float factor, float r2_edge, int (&bin)[kR]) {
+  bool unsure[kR], any = false;
+#pragma unroll
+  for (int r = 0; r < kR; ++r) {
+    const BinGuess b = bin_guess(r2[r], factor);
+    bin[r] = b.bin;
+    unsure[r] = !b.sure;
+    any = any || unsure[r];
+  }
+  if (any) {
+#pragma unroll
+    for (int r = 0; r < kR; ++r)
+      if (unsure[r]) bin[r] = bin_exactly(r2[r], factor, r2_edge);
+  }
+}
+
 // ---------------------------------------------------------------- reorder
 // CopySortedParticleValuesKernel* (particles_kernel.cu:543-654): gather the
 // state into sorted order.
@@ -447,6 +468,10 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_build_nlist(
         }
         ++cnt_mine;
       }
+      // zeros up to a whole batch of four (the value rows are allocated so):
+      // the staged pressure-force pass takes whole batches
+      if (lval && cnt_mine < maxn)
+        for (uint32_t z = cnt_mine; z & 3u; ++z) ov[(size_t)z * stride] = 0u;
       words = 0;
     }
     __syncwarp();
@@ -1202,15 +1227,16 @@ __device__ __forceinline__ void density_block(
 #pragma unroll
     for (int r = 0; r < kRows; ++r)
       if (k0 + r < (int)cnt) xj[r] = __ldg(xs + code(r));
+    // the table bin of d from d^2 (exact); at or beyond h the bin is 300,
+    // whose entry 0 adds +0 exactly as the reference's skipped term does, and
+    // past the list's end too
+    float r2[kRows];
+    int bin[kRows];
 #pragma unroll
-    for (int r = 0; r < kRows; ++r) {
-      if (k0 + r < (int)cnt) {
-        // the table bin of d from d^2 (exact); at or beyond h the bin is 300,
-        // whose entry 0 adds +0 exactly as the reference's skipped term does
-        const float r2 = dist2_xy(xiy, xi.z, xj[r]);
-        den += m4[bin_of_r2_edge(r2, P.lut_factor, r2_edge)];  // table times mass
-      }
-    }
+    for (int r = 0; r < kRows; ++r) r2[r] = k0 + r < (int)cnt ? dist2_xy(xiy, xi.z, xj[r]) : kFar2;
+    density_bins(r2, P.lut_factor, r2_edge, bin);
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) den += m4[bin[r]];  // table times mass
   });
   if (!ok && lane == 0) atomicOr(&st->error_flags, (uint32_t)ERR_TIMEOUT);
   if (active) {
@@ -1523,7 +1549,7 @@ __global__ void __launch_bounds__(kStageChunk) k_stage_lists(uint32_t n, const i
   }
   __syncthreads();
   const uint32_t total = warp_tot[kStageChunk / 32 - 1];
-  if (total > cap) {
+  if (total > cap || total > kUnionEmpty) {
     if (tid == 0) ucount[chunk] = kUnionOverflow;
     return;  // uniform
   }
@@ -1543,8 +1569,10 @@ __global__ void __launch_bounds__(kStageChunk) k_stage_lists(uint32_t n, const i
   }
   if (tid == 0) ucount[chunk] = total;
   __syncthreads();
-  // (3) the chunk's entries as union positions, four to a word, in place
-  // (the next word loaded before this one is rewritten)
+  // (3) the chunk's entries as union positions (in bytes of the staged arrays'
+  // 16-byte elements), four to a word, in place (the next word loaded before
+  // this one is rewritten); a list's last word is filled up with the empty
+  // position, so that the passes take whole words
   unsigned long long vn = cnt ? out[0] : 0ull;
   for (uint32_t k0 = 0; k0 < cnt; k0 += 4) {
     const unsigned long long v = vn;
@@ -1552,11 +1580,13 @@ __global__ void __launch_bounds__(kStageChunk) k_stage_lists(uint32_t n, const i
     unsigned long long w2 = 0;
 #pragma unroll
     for (uint32_t r = 0; r < 4; ++r) {
-      if (k0 + r < cnt) {
+      if (k0 + r >= cnt) {
+        w2 |= (unsigned long long)(kUnionEmpty * 16) << (16 * r);
+      } else {
         const uint32_t e = (uint32_t)(v >> (16 * r)) & 0xffffu;
         const uint32_t slot = e >> 3, b = e & 7u;
         const uint32_t posn = bbase[slot] + __popc(bmask[slot] & ((1u << b) - 1u));
-        w2 |= (unsigned long long)posn << (16 * r);
+        w2 |= (unsigned long long)(posn * 16) << (16 * r);
       }
     }
     out[(size_t)(k0 / 4) * stride] = w2;
@@ -1565,36 +1595,49 @@ __global__ void __launch_bounds__(kStageChunk) k_stage_lists(uint32_t n, const i
 
 // The staged list walk of one lane: batches of kRows entries (kRows / 4
 // words of lloc, the next batch's words loaded before this batch's
-// arithmetic); `body(pos, k0)` gets the union positions of the batch.
+// arithmetic); `body(word, k0)` gets each batch's words with the entries'
+// positions. A batch of more than one word may end with whole words past the
+// list: they are all empty positions.
 template <int kRows, class Body>
 __device__ __forceinline__ void walk_staged(const unsigned long long* __restrict__ col, uint32_t stride, uint32_t cnt,
                                             Body&& body) {
   constexpr int kWords = kRows / 4;
+  constexpr unsigned long long kEmpty4 = 0x0001000100010001ull * (kUnionEmpty * 16);
   unsigned long long w[kWords];
 #pragma unroll
-  for (int q = 0; q < kWords; ++q) w[q] = (4 * q < (int)cnt) ? __ldg(col + (size_t)q * stride) : 0ull;
+  for (int q = 0; q < kWords; ++q) w[q] = (4 * q < (int)cnt) ? __ldg(col + (size_t)q * stride) : kEmpty4;
   for (uint32_t k0 = 0; k0 < cnt; k0 += kRows) {
     unsigned long long cur[kWords];
 #pragma unroll
     for (int q = 0; q < kWords; ++q) {
       cur[q] = w[q];
       const uint32_t kn = k0 + kRows + 4 * q;
-      if (kn < cnt) w[q] = __ldg(col + (size_t)(kn / 4) * stride);
+      w[q] = kn < cnt ? __ldg(col + (size_t)(kn / 4) * stride) : kEmpty4;
     }
-    // (positions are below kUnionMax by construction; the mask keeps every
-    // shared-memory read in bounds even on lists staged for another step)
-    body([&](int r) { return (uint32_t)(cur[r >> 2] >> (16 * (r & 3))) & (kUnionMax - 1); }, (int)k0);
+    body(cur, (int)k0);
   }
+}
+// The element of a staged array at entry r of a batch's words. (Positions
+// lie in the array by construction; the mask keeps every shared-memory read in
+// bounds even on lists staged for another step.)
+__device__ __forceinline__ float4 staged_at(const float4* s, const unsigned long long* words, int r) {
+  const uint32_t half = r & 2 ? (uint32_t)(words[r >> 2] >> 32) : (uint32_t)words[r >> 2];
+  const uint32_t at = (r & 1 ? half >> 16 : half) & ((kUnionMax - 1) * 16);
+  return *reinterpret_cast<const float4*>(reinterpret_cast<const char*>(s) + at);
 }
 
 // The predicted-density pass over staged neighbourhoods (density_block's
 // arithmetic, ComputePredictedDensityAndPressure, UnifiedPhysics.cpp:5456-5491).
+// Bound: shared-memory wavefronts (64% of the pipe: 8 for a 16-byte read whose
+// lanes' neighbours are near but not next to one another, 2.4 for the table)
+// and, in the pressure-force pass, 300 B of DRAM a particle beside them. At
+// 1,048,576 particles 80.2 and 85.1 us a launch, 28.1 and 25.3 at 262,144
+// (84.2 and 92.2, 32.8 and 26.6 with conversions to find the bin, a branch
+// for each unsure bin, and a test at every entry for the list's end).
 // Register caps (CTAs an SM the launch bounds ask for; six fit the shared
 // memory, 33-34 KB each): 4-entry batches of the density pass are held to 40
-// registers (six CTAs an SM; 8 bytes of spill, and 0.083 against 0.085 ms a
-// launch at five CTAs and 48 registers on the 1M dam), of the pressure-force
-// pass to 48; 8-entry batches to 64 (density) and 80 (pressure force), the
-// caps below which they spill.
+// registers (six CTAs an SM), of the pressure-force pass to 48 (five; at four
+// CTAs and 64 registers 92 us).
 constexpr int density_staged_min_blocks(int rows) { return rows == 4 ? 6 : 4; }
 constexpr int pforce_staged_min_blocks(int rows) { return rows == 4 ? 5 : 3; }
 
@@ -1618,6 +1661,8 @@ __global__ void __launch_bounds__(kStageChunk, density_staged_min_blocks(kRows))
     const uint32_t* __restrict__ uc = ucodes + (size_t)chunk * kUnionMax;
     const uint32_t nu = U < kUnionMax ? U : kUnionMax;
     for (uint32_t l = threadIdx.x; l < nu; l += kStageChunk) xsm[l] = __ldg(xs + __ldg(uc + l));
+    // the empty position: far from everything, and finite
+    if (threadIdx.x == 0) xsm[kUnionEmpty] = make_float4(1e15f, 1e15f, 1e15f, 0.0f);
   }
   const float r2_edge = __ldg(luts + 5 * UPF_LUT_ENTRIES + kLut);
   __syncthreads();
@@ -1627,19 +1672,22 @@ __global__ void __launch_bounds__(kStageChunk, density_staged_min_blocks(kRows))
   const float4 xi = active ? xs[i] : make_float4(0, 0, 0, 0);
   const unsigned long long xiy = pk2(xi.x, xi.y);
   float den = P.kernel_self * P.mass;
-  auto add = [&](float4 xj) {
-    const float r2 = dist2_xy(xiy, xi.z, xj);
-    den += m4[bin_of_r2_edge(r2, P.lut_factor, r2_edge)];
+  auto add = [&](const auto& xj, auto&& valid) {
+    constexpr int kR = sizeof(xj) / sizeof(xj[0]);
+    float r2[kR];
+    int bin[kR];
+#pragma unroll
+    for (int r = 0; r < kR; ++r) r2[r] = valid(r) ? dist2_xy(xiy, xi.z, xj[r]) : kFar2;
+    density_bins(r2, P.lut_factor, r2_edge, bin);
+#pragma unroll
+    for (int r = 0; r < kR; ++r) den += m4[bin[r]];
   };
   if (staged) {
-    walk_staged<kRows>(lloc + i, P.nstride, cnt, [&](auto pos, int k0) {
+    walk_staged<kRows>(lloc + i, P.nstride, cnt, [&](const unsigned long long* words, int) {
       float4 xj[kRows];
 #pragma unroll
-      for (int r = 0; r < kRows; ++r)
-        if (k0 + r < (int)cnt) xj[r] = xsm[pos(r)];
-#pragma unroll
-      for (int r = 0; r < kRows; ++r)
-        if (k0 + r < (int)cnt) add(xj[r]);
+      for (int r = 0; r < kRows; ++r) xj[r] = staged_at(xsm, words, r);
+      add(xj, [](int) { return true; });
     });
   } else {
     const uint32_t* __restrict__ col = nbr + i;
@@ -1648,9 +1696,7 @@ __global__ void __launch_bounds__(kStageChunk, density_staged_min_blocks(kRows))
 #pragma unroll
       for (int r = 0; r < 4; ++r)
         if (k0 + r < cnt) xj[r] = __ldg(xs + __ldg(col + (size_t)(k0 + r) * P.nstride));
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-        if (k0 + r < cnt) add(xj[r]);
+      add(xj, [&](int r) { return k0 + r < cnt; });
     }
   }
   uint32_t best = 0;
@@ -1691,6 +1737,7 @@ __global__ void __launch_bounds__(kStageChunk, pforce_staged_min_blocks(kRows)) 
     const uint32_t* __restrict__ uc = ucodes + (size_t)chunk * kUnionMax;
     const uint32_t nu = U < kUnionMax ? U : kUnionMax;
     for (uint32_t l = threadIdx.x; l < nu; l += kStageChunk) qsm[l] = __ldg(pq + __ldg(uc + l));
+    if (threadIdx.x == 0) qsm[kUnionEmpty] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   }
   __syncthreads();
   const uint32_t i = chunk * kStageChunk + threadIdx.x;
@@ -1711,26 +1758,34 @@ __global__ void __launch_bounds__(kStageChunk, pforce_staged_min_blocks(kRows)) 
     fz = fz - kz * grad * m * m;
   };
   if (staged) {
-    // the list values of the next batch are loaded with its positions,
-    // before this batch's arithmetic (walk_staged's prefetch, extended)
+    // whole batches of four: past the list's end the value is 0 and the
+    // neighbour the empty position, and taking off a zero changes no sum (a
+    // batch's second word may lie past the list altogether). The next batch's
+    // values are loaded with its words, before this batch's arithmetic.
+    const float* __restrict__ vc = reinterpret_cast<const float*>(vcol);
+    const size_t row = P.nstride;
     float gn[kRows];
+    auto values = [&](uint32_t k0) {
 #pragma unroll
-    for (int r = 0; r < kRows; ++r) gn[r] = r < (int)cnt ? __uint_as_float(__ldg(vcol + (size_t)r * P.nstride)) : 0.0f;
-    walk_staged<kRows>(lloc + i, P.nstride, cnt, [&](auto pos, int k0) {
+      for (int q = 0; q < kRows / 4; ++q) {
+        const bool have = k0 + 4 * q < cnt;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) gn[4 * q + r] = have ? __ldg(vc + r * row) : 0.0f;
+        vc += 4 * row;
+      }
+    };
+    values(0);
+    walk_staged<kRows>(lloc + i, P.nstride, cnt, [&](const unsigned long long* words, int k0) {
       float4 xj[kRows];
       float g[kRows];
 #pragma unroll
       for (int r = 0; r < kRows; ++r) {
         g[r] = gn[r];
-        const uint32_t kn = (uint32_t)k0 + kRows + r;
-        if (kn < cnt) gn[r] = __uint_as_float(__ldg(vcol + (size_t)kn * P.nstride));
+        xj[r] = staged_at(qsm, words, r);
       }
+      values(k0 + kRows);
 #pragma unroll
-      for (int r = 0; r < kRows; ++r)
-        if (k0 + r < (int)cnt) xj[r] = qsm[pos(r)];
-#pragma unroll
-      for (int r = 0; r < kRows; ++r)
-        if (k0 + r < (int)cnt) add(xj[r], g[r]);
+      for (int r = 0; r < kRows; ++r) add(xj[r], g[r]);
     });
   } else {
     const uint32_t* __restrict__ col = nbr + i;
@@ -1938,23 +1993,24 @@ __global__ void __launch_bounds__(kThreads, kResident / kThreads) k_pcisph_loop(
   auto density = [&]() {
     float den = P.kernel_self * m;
     const unsigned long long xiy = pk2(xstar.x, xstar.y);
-    auto term = [&](float4 xj) { return m4[bin_of_r2_edge(dist2_xy(xiy, xstar.z, xj), P.lut_factor, r2_edge)]; };
     const uint32_t walk = kLanes > 1 ? __reduce_max_sync(0xffffffffu, cnt) : cnt;
     for (uint32_t k0 = 0; k0 < walk; k0 += kTerms) {
       float4 xj[kRows];
 #pragma unroll
       for (int r = 0; r < kRows; ++r)
         if (k0 + r * kLanes + sub < cnt) xj[r] = xs[code_at(k0 + r * kLanes + sub)];
+      float r2[kRows];
+      int bin[kRows];
+#pragma unroll
+      for (int r = 0; r < kRows; ++r)
+        r2[r] = k0 + r * kLanes + sub < cnt ? dist2_xy(xiy, xstar.z, xj[r]) : kFar2;
+      density_bins(r2, P.lut_factor, r2_edge, bin);
       if (kLanes == 1) {
 #pragma unroll
-        for (int r = 0; r < kRows; ++r)
-          if (k0 + r < cnt) den += term(xj[r]);
+        for (int r = 0; r < kRows; ++r) den += m4[bin[r]];
       } else {
 #pragma unroll
-        for (int r = 0; r < kRows; ++r) {
-          const uint32_t e = r * kLanes + sub;
-          *term_at(e) = k0 + e < cnt ? term(xj[r]) : 0.0f;
-        }
+        for (int r = 0; r < kRows; ++r) *term_at(r * kLanes + sub) = m4[bin[r]];
         __syncwarp();
         if (sub == 0) {
 #pragma unroll
@@ -2559,11 +2615,27 @@ cudaError_t launch_list_staging(System& s, cudaStream_t st) {
   return s.n_dyn && s.ucodes ? launch_stage_lists(s, st) : cudaSuccess;
 }
 
+// The shapes the loop passes run at: those set or tuned; else, above the
+// fused loop's sizes, staged neighbourhoods. An iteration at 262,144
+// particles takes 53 us staged against 66 at LaunchShape's own values (165
+// against 198 at 1,048,576), and staging, 44 us (145), is paid from the fourth
+// iteration on (a step takes at least three, and 14 in a settled scene).
+static LaunchShape loop_shape(const System& s) {
+  LaunchShape sh = s.shape;
+  if (s.ucodes && !s.shape_set && !s.shape_tuned && !s.stage_always && s.n_dyn > s.loop_sms * kLoopResident) {
+    sh.density_mode = sh.pforce_mode = 2;
+    sh.density_threads = sh.pforce_threads = kStageChunk;
+    sh.density_rows = sh.pforce_rows = 4;
+  }
+  return sh;
+}
+
 // the lists are staged when a loop pass reads staged neighbourhoods (or
 // while the autotuner times every mode)
 static bool stages_lists(const System& s) {
-  return s.ucodes && !s.loop_in_graph && (s.stage_always || loop_mode_staged(s.shape.density_mode) ||
-                      loop_mode_staged(s.shape.pforce_mode));
+  const LaunchShape sh = loop_shape(s);
+  return s.ucodes && !s.loop_in_graph && (s.stage_always || loop_mode_staged(sh.density_mode) ||
+                                          loop_mode_staged(sh.pforce_mode));
 }
 
 cudaError_t launch_neighbor_phase(System& s, cudaStream_t st) {
@@ -2673,17 +2745,18 @@ cudaError_t batch_launch_fused_loop(BatchSystem& b, cudaStream_t st) {
 
 cudaError_t launch_loop_density(System& s, cudaStream_t st) {
   const uint32_t n = s.n_dyn;
-  if (n && loop_mode_staged(s.shape.density_mode)) {
+  const LaunchShape sh = loop_shape(s);
+  if (n && loop_mode_staged(sh.density_mode)) {
     // lists built under another shape (phase by phase) are staged first
     if (!s.lists_staged) {
       cudaError_t e = launch_stage_lists(s, st);
       if (e != cudaSuccess) return e;
     }
     const uint32_t g = (n + kStageChunk - 1) / kStageChunk;
-    if (s.shape.density_rows == 4)
+    if (sh.density_rows == 4)
       k_pcisph_density_staged<4><<<g, kStageChunk, 0, st>>>(s.dp, n, s.B.type, s.xs, s.nbr, s.ncnt, s.ucodes,
                                                            s.ucount, s.lloc, s.luts, s.rho, s.press, s.pq, s.st);
-    else if (s.shape.density_rows == 8)
+    else if (sh.density_rows == 8)
       k_pcisph_density_staged<8><<<g, kStageChunk, 0, st>>>(s.dp, n, s.B.type, s.xs, s.nbr, s.ncnt, s.ucodes,
                                                            s.ucount, s.lloc, s.luts, s.rho, s.press, s.pq, s.st);
     else
@@ -2691,24 +2764,25 @@ cudaError_t launch_loop_density(System& s, cudaStream_t st) {
     return cudaGetLastError();
   }
   if (n)
-    return run_density<false>(s.shape, st, s.dp, BatchView{}, n, s.B.type, s.xs, s.nbr_maps, s.nbr, s.ncnt, s.luts, s.rho,
+    return run_density<false>(sh, st, s.dp, BatchView{}, n, s.B.type, s.xs, s.nbr_maps, s.nbr, s.ncnt, s.luts, s.rho,
                               s.press, s.pq, s.st);
   return cudaGetLastError();
 }
 
 cudaError_t launch_loop_pforce(System& s, cudaStream_t st) {
   const uint32_t n = s.n_dyn;
-  if (n && loop_mode_staged(s.shape.pforce_mode)) {
+  const LaunchShape sh = loop_shape(s);
+  if (n && loop_mode_staged(sh.pforce_mode)) {
     if (!s.lists_staged) {
       cudaError_t e = launch_stage_lists(s, st);
       if (e != cudaSuccess) return e;
     }
     const uint32_t g = (n + kStageChunk - 1) / kStageChunk;
-    if (s.shape.pforce_rows == 4)
+    if (sh.pforce_rows == 4)
       k_pcisph_pressure_force_staged<4><<<g, kStageChunk, 0, st>>>(s.dp, n, s.B, s.nbr, s.lval, s.ncnt, s.ucodes,
                                                                   s.ucount, s.lloc, s.pq, s.force, s.pforce, s.xs,
                                                                   s.st);
-    else if (s.shape.pforce_rows == 8)
+    else if (sh.pforce_rows == 8)
       k_pcisph_pressure_force_staged<8><<<g, kStageChunk, 0, st>>>(s.dp, n, s.B, s.nbr, s.lval, s.ncnt, s.ucodes,
                                                                   s.ucount, s.lloc, s.pq, s.force, s.pforce, s.xs,
                                                                   s.st);
@@ -2717,7 +2791,7 @@ cudaError_t launch_loop_pforce(System& s, cudaStream_t st) {
     return cudaGetLastError();
   }
   if (n)
-    return run_pforce<false>(s.shape, st, s.dp, BatchView{}, n, s.B, s.nbr_maps, s.lval_maps, s.nbr, s.lval, s.ncnt, s.luts, s.pq,
+    return run_pforce<false>(sh, st, s.dp, BatchView{}, n, s.B, s.nbr_maps, s.lval_maps, s.nbr, s.lval, s.ncnt, s.luts, s.pq,
                              s.force, s.pforce, s.xs, s.st);
   return cudaGetLastError();
 }

@@ -88,11 +88,12 @@ static_assert(pforce_ring_fits(LaunchShape{}.pforce_mode, LaunchShape{}.pforce_t
 // rewritten once per step against the chunk's union of neighbours: ucodes
 // holds the union's neighbour indices (at most kUnionMax a chunk), ucount its
 // size (kUnionOverflow: the union did not fit, the chunk's passes read the
-// plain lists), and lloc the list entries as 16-bit positions in the union,
-// four to a 64-bit word, lloc[(k / 4) * stride + i]. A staged pass copies the
+// plain lists), and lloc the list entries as 16-bit positions in the union
+// (times 16, the staged elements' bytes), four to a 64-bit word, lloc[(k / 4) * stride + i]. A staged pass copies the
 // union's data into shared memory once and reads each neighbour from there.
 constexpr int kStageChunk = 256;
 constexpr uint32_t kUnionMax = 2048;
+constexpr uint32_t kUnionEmpty = kUnionMax - 1;  // position of no neighbour: fills a list's last word
 constexpr uint32_t kUnionOverflow = 0xffffffffu;
 constexpr bool loop_mode_staged(int mode) { return mode == 2; }
 
@@ -224,6 +225,7 @@ struct System {
   uint32_t* loop_max = nullptr;   // [2] the maximum predicted density of odd and even iterations
   uint32_t loop_sms = 0;          // the device's SMs (0: no cooperative launches)
   bool shape_set = false;         // the caller chose the loop passes' shapes: they run as launches of their own
+  bool shape_tuned = false;       // the autotuner chose them (loop_shape)
   bool loop_in_graph = false;     // the step graph being captured has the fused loop: no staging
 
   RigidArrays rb;
