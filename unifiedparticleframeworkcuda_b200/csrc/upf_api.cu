@@ -491,10 +491,11 @@ upf_status build_step_graph(System& s) {
   parts.ctx = &s;
   parts.pre = [](void* c, cudaStream_t st) {
     System& S = *static_cast<System*>(c);
+    const bool pcisph = S.prm.method == UPF_METHOD_PCISPH;
     cudaError_t e = launch_sort_phase(S, st);
-    if (e == cudaSuccess) e = launch_neighbor_phase(S, st);
-    if (e == cudaSuccess) e = launch_force_phase(S, st);
-    if (e == cudaSuccess && S.prm.method == UPF_METHOD_PCISPH) e = launch_loop_init(S, st);
+    if (e == cudaSuccess) e = launch_neighbor_phase(S, st, !pcisph);
+    if (e == cudaSuccess && pcisph) e = launch_force_phase(S, st);
+    if (e == cudaSuccess && pcisph) e = launch_loop_init(S, st);
     return e;
   };
   s.loop_in_graph = loop_fused(s);
@@ -1042,6 +1043,11 @@ upf_status upf_set_particles(upf_system* s, const float* pos4, const float* vel4
     UPF_CUDA(cudaMemcpyAsync(S.B.pos + tb, S.spos, sizeof(float4) * S.n_static, cudaMemcpyDeviceToDevice, st));
     UPF_CUDA(cudaMemcpyAsync(S.xs + tb, S.spos, sizeof(float4) * S.n_static, cudaMemcpyDeviceToDevice, st));
     UPF_CUDA(cudaMemcpyAsync(S.pq + tb, S.spos, sizeof(float4) * S.n_static, cudaMemcpyDeviceToDevice, st));
+    if (S.prm.method == UPF_METHOD_WCSPH) {  // boundary particles' (velocity, volume) for the force pass
+      std::vector<float4> wall(S.n_static, make_float4(0.0f, 0.0f, 0.0f, -1.0f));
+      UPF_CUDA(cudaMemcpyAsync(S.xs + tb, wall.data(), sizeof(float4) * S.n_static, cudaMemcpyHostToDevice, st));
+      UPF_CUDA(cudaStreamSynchronize(st));  // `wall` goes out of scope
+    }
     std::vector<int32_t> frozen(S.n_static, UPF_FROZEN);
     UPF_CUDA(cudaMemcpyAsync(S.B.type + tb, frozen.data(), sizeof(int32_t) * S.n_static, cudaMemcpyHostToDevice, st));
   }
@@ -1497,8 +1503,11 @@ upf_status state_copy(System& s, char* flat, bool to_flat, cudaMemcpyKind kind) 
   StateSeg seg[8];
   const int k = state_segments(s, seg);
   size_t off = 0;
+  CopyList list;
   for (int i = 0; i < k; ++i) {
-    if (seg[i].bytes) {
+    if (kind == cudaMemcpyDeviceToDevice) {
+      list.add(to_flat ? (void*)(flat + off) : seg[i].dev, to_flat ? seg[i].dev : (void*)(flat + off), seg[i].bytes);
+    } else if (seg[i].bytes) {
       cudaError_t e = to_flat ? cudaMemcpyAsync(flat + off, seg[i].dev, seg[i].bytes, kind, s.stream)
                               : cudaMemcpyAsync(seg[i].dev, flat + off, seg[i].bytes, kind, s.stream);
       if (e != cudaSuccess) {
@@ -1508,6 +1517,7 @@ upf_status state_copy(System& s, char* flat, bool to_flat, cudaMemcpyKind kind) 
     }
     off += (seg[i].bytes + 255) & ~size_t(255);
   }
+  UPF_CUDA(copy_arrays(list, s.stream));
   return UPF_OK;
 }
 }  // namespace

@@ -485,11 +485,12 @@ static upf_status batch_state_copy(upf_batch* b, char* flat, bool to_flat) {
              {b->A.id, n * sizeof(uint32_t)}, {b->A.type, n * sizeof(int32_t)}, {b->keysA, n * sizeof(uint32_t)},
              {b->st_d, sizeof(DevState) * b->n_scenes}};
   size_t off = 0;
+  CopyList list;
   for (const Seg& s : seg) {
-    UPF_CUDA(to_flat ? cudaMemcpyAsync(flat + off, s.p, s.bytes, cudaMemcpyDeviceToDevice, b->stream)
-                     : cudaMemcpyAsync(s.p, flat + off, s.bytes, cudaMemcpyDeviceToDevice, b->stream));
-    off += s.bytes;
+    list.add(to_flat ? (void*)(flat + off) : s.p, to_flat ? s.p : (void*)(flat + off), s.bytes);
+    off += s.bytes;  // (slots come in multiples of 256: every offset is one of 16)
   }
+  UPF_CUDA(copy_arrays(list, b->stream));
   return UPF_OK;
 }
 

@@ -26,6 +26,7 @@
 // which is the parity target; each kernel cites the function it restates.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "upf_sys.h"
@@ -92,39 +93,6 @@ __device__ __forceinline__ void for_neighbors(const uint32_t* __restrict__ col, 
       if (u < rem) use(code[u], v[u]);
   }
 }
-
-// The same, also handing each entry's stored list value (the kernel-table
-// bin, in the WCSPH passes) to `use`.
-template <class Load, class Use>
-__device__ __forceinline__ void for_neighbors_bin(const uint32_t* __restrict__ col, const uint32_t* __restrict__ bcol,
-                                                  uint32_t stride, uint32_t cnt, Load&& load, Use&& use) {
-  using T = decltype(load(0u));
-  uint32_t k = 0;
-  for (; k + kUnroll <= cnt; k += kUnroll) {
-    uint32_t code[kUnroll];
-    uint32_t bin[kUnroll];
-    T v[kUnroll];
-#pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
-      code[u] = __ldg(col + (size_t)(k + u) * stride);
-      bin[u] = __ldg(bcol + (size_t)(k + u) * stride);
-    }
-#pragma unroll
-    for (int u = 0; u < kUnroll; ++u) v[u] = load(code[u]);
-#pragma unroll
-    for (int u = 0; u < kUnroll; ++u) use(code[u], bin[u], v[u]);
-  }
-  for (; k < cnt; ++k) {
-    const uint32_t code = __ldg(col + (size_t)k * stride);
-    const uint32_t bin = __ldg(bcol + (size_t)k * stride);
-    use(code, bin, load(code));
-  }
-}
-
-struct PosP {
-  float4 x;
-  float p;
-};
 
 // What a CTA works on: one system (plain launch) or, in a batched launch,
 // the scene its slots belong to (BatchView). Batched CTAs copy the scene's
@@ -270,6 +238,104 @@ __device__ __forceinline__ float dist2_xy(unsigned long long axy, float az, floa
   return fadd(fadd(s.x, s.y), fmul(dz, dz));
 }
 
+// ---------------------------------------------------------------- WCSPH density
+// DistanceToWall (UnifiedPhysics.cpp:5926-5990) and WallWeight (6032-6060)
+__device__ float wall_weight(const DevParams& P, const float* m4, float4 x) {
+  const float L = P.wmax.x - P.wmin.x, H = P.wmax.y - P.wmin.y, W = P.wmax.z - P.wmin.z;
+  float res = mx0(L, mx0(H, W));
+  float d;
+  d = mx0(x.y - P.wmin.y, 0.0f); res = (res <= d) ? res : d;
+  d = mx0(P.wmax.y - x.y, 0.0f); res = (res <= d) ? res : d;
+  d = mx0(x.x - P.wmin.x, 0.0f); res = (res <= d) ? res : d;
+  d = mx0(P.wmax.x - x.x, 0.0f); res = (res <= d) ? res : d;
+  d = mx0(x.z - P.wmin.z, 0.0f); res = (res <= d) ? res : d;
+  d = mx0(P.wmax.z - x.z, 0.0f); res = (res <= d) ? res : d;
+  const float eff = P.h - P.radius;
+  if (res >= eff) return 0.0f;
+  const float s = P.spacing;
+  float d1 = res + P.radius;
+  float d2 = d1 + s;
+  float d3 = sqrtf(d1 * d1 + s * s);
+  float d4 = sqrtf(d1 * d1 + (s * 2) * (s * 2));
+  float d5 = sqrtf(d2 * d2 + s * s);
+  float d6 = sqrtf(d2 * d2 + (s * 2) * (s * 2));
+  float k1 = lut_at(m4, d1, P.lut_factor), k2 = lut_at(m4, d2, P.lut_factor),
+        k3 = lut_at(m4, d3, P.lut_factor), k4 = lut_at(m4, d4, P.lut_factor),
+        k5 = lut_at(m4, d5, P.lut_factor), k6 = lut_at(m4, d6, P.lut_factor);
+  return P.mass * (k1 + k2 + 2 * (k3 + k4 + k5 + k6));
+}
+
+// What the WCSPH passes exchange: density and pressure, and for the force
+// pass's two gathers a neighbour's (position, p / rho^2) and (velocity,
+// m / rho); the volume is -1 where the particle is not liquid (boundary
+// particles: set once, in the tails).
+struct WcsphOut {
+  const float4* vel = nullptr;
+  const int32_t* type = nullptr;
+  float* rho = nullptr;
+  float* press = nullptr;
+  float4* xq = nullptr;
+  float4* vn = nullptr;
+};
+
+// CalculateDensityPressurePureFluidSPH + CalculatePressureWCSPH
+// (UnifiedPhysics.cpp:2408-2501): the pressure of a liquid particle from its
+// summed density.
+__device__ __forceinline__ void wcsph_store(const DevParams& P, const float* m4, const WcsphOut& W, uint32_t i,
+                                            float4 xi, float den) {
+  float4 v = W.vel[i];
+  float q = 0.0f;
+  if (W.type[i] == UPF_LIQUID) {
+    if (P.flags & UPF_FLAG_WALL_WEIGHT) den += wall_weight(P, m4, xi);
+    const float frac = den / P.rho0;
+    // pow(float, float) of the reference's host build is glibc powf, which
+    // evaluates in double and rounds once; the double pow rounded to float
+    // gives the same float (CUDA's single-precision powf may differ by ulps,
+    // which the stiff Tait equation amplifies over many steps)
+    const float powg = (float)pow((double)frac, (double)P.gamma);
+    float pr = P.gas_b * (powg - 1.0f);
+    pr = (0.0f >= pr) ? 0.0f : pr;
+    W.rho[i] = den;
+    W.press[i] = pr;
+    q = pr / (den * den);
+    v.w = P.mass / den;
+  } else {
+    v.w = -1.0f;
+  }
+  W.xq[i] = make_float4(xi.x, xi.y, xi.z, q);
+  W.vn[i] = v;
+}
+
+// The density pass on its own (the phase entry point; a step sums the
+// densities while it builds the lists, k_build_nlist).
+__global__ void __launch_bounds__(kBlock) k_wcsph_density(DevParams P, uint32_t n, const float4* __restrict__ pos,
+                                                           const uint32_t* __restrict__ lval,
+                                                           const uint32_t* __restrict__ ncnt,
+                                                           const float* __restrict__ luts, WcsphOut W) {
+  __shared__ float m4[UPF_LUT_ENTRIES];
+  stage_lut(m4, luts + LUT_M4 * UPF_LUT_ENTRIES);
+  __syncthreads();
+  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const float m = P.mass;
+  float den = P.kernel_self * m;
+  // densities at the positions the list was built at: every entry is within
+  // h and carries its kernel-table bin, so only the bins are read (list values)
+  const uint32_t* __restrict__ b = lval + i;
+  const uint32_t c = ncnt[i];
+  uint32_t k = 0;
+  for (; k + kUnroll <= c; k += kUnroll) {
+    uint32_t bb[kUnroll];
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) bb[u] = __ldg(b + (size_t)(k + u) * P.nstride);
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) den += m4[bb[u]] * m;
+  }
+  for (; k < c; ++k) den += m4[__ldg(b + (size_t)k * P.nstride)] * m;
+  wcsph_store(P, m4, W, i, pos[i], den);
+}
+
+// ---------------------------------------------------------------- neighbour lists
 // The dynamic and the boundary particles as one sequence in Morton order
 // (dynamic first at equal keys), for the list build: element m holds a
 // position and, in w, the bits of its neighbour index. Each particle finds
@@ -383,12 +449,14 @@ __device__ __forceinline__ uint32_t first_above(uint32_t v, uint32_t r) {
   return k;
 }
 
-template <bool kBatch, bool kMerged, int kThreads, int kW>
+// kWcsph: the step's density pass as well, summed entry by entry as the list
+// is written (a pass of its own read the bins back: 9.4 us at 32,768).
+template <bool kBatch, bool kMerged, bool kWcsph, int kThreads, int kW>
 __global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_build_nlist(
     const __grid_constant__ DevParams Pk, const BatchView bv, uint32_t n, const float4* __restrict__ pos,
     const float4* __restrict__ mpos, const uint32_t* __restrict__ cstart, const uint32_t* __restrict__ cend,
     uint32_t* __restrict__ nbr, uint32_t* __restrict__ lval, uint32_t* __restrict__ ncnt,
-    const float* __restrict__ luts, DevState* __restrict__ st_plain) {
+    const float* __restrict__ luts, DevState* __restrict__ st_plain, const WcsphOut wc) {
   constexpr int kWarps = kThreads / 32;
   static_assert(32 % kW == 0 && kSegAlign % (kWarps * kW) == 0, "a CTA's particles lie in one scene");
   extern __shared__ __align__(16) unsigned char nlist_mem[];
@@ -398,7 +466,8 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_build_nlist(
   const uint32_t slot0 = blockIdx.x * (uint32_t)(kWarps * kW);
   const Scope sc = enter_scope_slot<kBatch>(slot0, Pk, luts, st_plain, n, bv, &sP, false);
   for (int k = threadIdx.x; k < kThresholds; k += kThreads) thr[k] = sc.luts[5 * UPF_LUT_ENTRIES + k];
-  stage_lut(pg, sc.luts + LUT_PGRAD * UPF_LUT_ENTRIES);
+  // (the density sums read the M4 table where the gradient's is not needed)
+  stage_lut(pg, sc.luts + (kWcsph ? LUT_M4 : LUT_PGRAD) * UPF_LUT_ENTRIES);
   __syncthreads();
   const DevParams& P = *sc.P;
   if (kBatch) {
@@ -414,7 +483,8 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_build_nlist(
   const uint32_t maxn = P.maxn, stride = P.nstride;
   const float h = P.h, r2_edge = thr[kThresholds - 1];
   const int shift = (int)P.cell_shift;
-  const bool grad = P.list_grad != 0;
+  const bool grad = !kWcsph && P.list_grad != 0;
+  float den = kWcsph ? P.kernel_self * P.mass : 0.0f;  // lane l: the density of particle i0 + l
   const bool mine = lane < (uint32_t)kW && i0 + lane < sc.end;
   // lane l's particle: its grid position, clamped to the grid as keys are,
   // and its query box in cells
@@ -464,6 +534,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_build_nlist(
           if (lval) {
             const int bin = bin_of_r2(dist2(xi, __ldg(mpos + idx)), P.lut_factor, thr);
             ov[(size_t)cnt_mine * stride] = grad ? __float_as_uint(pg[bin]) : (uint32_t)bin;
+            if (kWcsph) den += pg[bin] * P.mass;
           }
         }
         ++cnt_mine;
@@ -654,7 +725,10 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_build_nlist(
   }
   emit(0xffffffffu);
   const uint32_t held = min(cnt_mine, maxn);
-  if (mine) ncnt[i0 + lane] = held;
+  if (mine) {
+    ncnt[i0 + lane] = held;
+    if constexpr (kWcsph) wcsph_store(P, pg, wc, i0 + lane, xi, den);
+  }
   const uint32_t most = __reduce_max_sync(0xffffffffu, cnt_mine);
   if (lane == 0) {
     DevState* st = sc.st;
@@ -664,73 +738,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_build_nlist(
   }
 }
 
-// ---------------------------------------------------------------- WCSPH
-// DistanceToWall (UnifiedPhysics.cpp:5926-5990) and WallWeight (6032-6060)
-__device__ float wall_weight(const DevParams& P, const float* m4, float4 x) {
-  const float L = P.wmax.x - P.wmin.x, H = P.wmax.y - P.wmin.y, W = P.wmax.z - P.wmin.z;
-  float res = mx0(L, mx0(H, W));
-  float d;
-  d = mx0(x.y - P.wmin.y, 0.0f); res = (res <= d) ? res : d;
-  d = mx0(P.wmax.y - x.y, 0.0f); res = (res <= d) ? res : d;
-  d = mx0(x.x - P.wmin.x, 0.0f); res = (res <= d) ? res : d;
-  d = mx0(P.wmax.x - x.x, 0.0f); res = (res <= d) ? res : d;
-  d = mx0(x.z - P.wmin.z, 0.0f); res = (res <= d) ? res : d;
-  d = mx0(P.wmax.z - x.z, 0.0f); res = (res <= d) ? res : d;
-  const float eff = P.h - P.radius;
-  if (res >= eff) return 0.0f;
-  const float s = P.spacing;
-  float d1 = res + P.radius;
-  float d2 = d1 + s;
-  float d3 = sqrtf(d1 * d1 + s * s);
-  float d4 = sqrtf(d1 * d1 + (s * 2) * (s * 2));
-  float d5 = sqrtf(d2 * d2 + s * s);
-  float d6 = sqrtf(d2 * d2 + (s * 2) * (s * 2));
-  float k1 = lut_at(m4, d1, P.lut_factor), k2 = lut_at(m4, d2, P.lut_factor),
-        k3 = lut_at(m4, d3, P.lut_factor), k4 = lut_at(m4, d4, P.lut_factor),
-        k5 = lut_at(m4, d5, P.lut_factor), k6 = lut_at(m4, d6, P.lut_factor);
-  return P.mass * (k1 + k2 + 2 * (k3 + k4 + k5 + k6));
-}
-
-// CalculateDensityPressurePureFluidSPH + CalculatePressureWCSPH
-// (UnifiedPhysics.cpp:2408-2501), liquid particles.
-__global__ void __launch_bounds__(kBlock) k_wcsph_density(
-    DevParams P, uint32_t n, const float4* __restrict__ pos, const int32_t* __restrict__ type,
-    const uint32_t* __restrict__ lval, const uint32_t* __restrict__ ncnt, const float* __restrict__ luts,
-    float* __restrict__ rho, float* __restrict__ press) {
-  __shared__ float m4[UPF_LUT_ENTRIES];
-  stage_lut(m4, luts + LUT_M4 * UPF_LUT_ENTRIES);
-  __syncthreads();
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  if (type[i] != UPF_LIQUID) return;
-  const float4 xi = pos[i];
-  const float m = P.mass;
-  float den = P.kernel_self * m;
-  // densities at the positions the list was built at: every entry is within
-  // h and carries its kernel-table bin, so only the bins are read (list values)
-  const uint32_t* __restrict__ b = lval + i;
-  const uint32_t c = ncnt[i];
-  uint32_t k = 0;
-  for (; k + kUnroll <= c; k += kUnroll) {
-    uint32_t bb[kUnroll];
-#pragma unroll
-    for (int u = 0; u < kUnroll; ++u) bb[u] = __ldg(b + (size_t)(k + u) * P.nstride);
-#pragma unroll
-    for (int u = 0; u < kUnroll; ++u) den += m4[bb[u]] * m;
-  }
-  for (; k < c; ++k) den += m4[__ldg(b + (size_t)k * P.nstride)] * m;
-  if (P.flags & UPF_FLAG_WALL_WEIGHT) den += wall_weight(P, m4, xi);
-  const float frac = den / P.rho0;
-  // pow(float, float) of the reference's host build is glibc powf, which
-  // evaluates in double and rounds once; the double pow rounded to float
-  // gives the same float (CUDA's single-precision powf may differ by ulps,
-  // which the stiff Tait equation amplifies over many steps)
-  const float powg = (float)pow((double)frac, (double)P.gamma);
-  const float pr = P.gas_b * (powg - 1.0f);
-  rho[i] = den;
-  press[i] = (0.0f >= pr) ? 0.0f : pr;
-}
-
+// ---------------------------------------------------------------- WCSPH forces
 // WeightingKernel::kernelSplineSurfaceTension (WeightingKernel.cpp:210-231)
 __device__ float cohesion_spline(float dist, float sr) {
   const float c = 32.0f / ((3.14159274f * sr * sr * sr * sr * sr * sr * sr * sr * sr));
@@ -800,79 +808,129 @@ __device__ __forceinline__ void integrate_store(const DevParams& P, uint32_t i, 
 
 // CalculateLiquidParticleForces (UnifiedPhysics.cpp:3009-3083) + gravity +
 // integration (the reference's GPU path fuses these too,
-// CalculateForcesInBlocksKernelWCSPH particles_kernel.cu:2399-2653).
+// CalculateForcesInBlocksKernelWCSPH particles_kernel.cu:2399-2653). Positions
+// are those the list was built at: entries are within h and carry their
+// kernel-table bin. A neighbour is two 16-byte gathers (WcsphOut), its p /
+// rho^2 and m / rho divided once by its own thread, as the reference divides
+// them in every pair.
+// kLanes: lanes a particle, as in the fused loop (k_pcisph_loop): at tens of
+// thousands of particles a thread each leaves an SM a few warps, whose 30
+// entries of dependent gathers are the pass. The lanes' terms (pressure,
+// viscosity, with kSurface surface tension, per component) wait in shared
+// memory and are taken off in list order by a lane per component.
+constexpr int kForceRows = 4;  // list entries a lane takes at a time
+template <int kLanes, bool kSurface>
 __global__ void __launch_bounds__(kBlock) k_wcsph_force_integrate(
-    DevParams P, uint32_t n, DynArrays B, DynArrays A, uint32_t* __restrict__ keysA,
+    const __grid_constant__ DevParams P, uint32_t n, DynArrays B, DynArrays A, uint32_t* __restrict__ keysA,
     const uint32_t* __restrict__ nbr, const uint32_t* __restrict__ lval, const uint32_t* __restrict__ ncnt,
     const float* __restrict__ luts, const float* __restrict__ rho, const float* __restrict__ press,
-    float4* __restrict__ force, DevState* __restrict__ st) {
+    const float4* __restrict__ xq, const float4* __restrict__ vn, float4* __restrict__ force,
+    DevState* __restrict__ st) {
+  constexpr uint32_t kPer = 32 / kLanes;                // particles a warp
+  constexpr uint32_t kEntries = kLanes * kForceRows;    // entries of a particle at a time
+  constexpr uint32_t kParts = kSurface ? 3 : 2;         // terms an entry and component
+  constexpr uint32_t kTerms = kEntries * kParts;
   __shared__ float pg[UPF_LUT_ENTRIES], vl[UPF_LUT_ENTRIES];
+  __shared__ __align__(16) float term_mem[kLanes > 1 ? kBlock / 32 * 3 * kTerms * kPer : 4];
   stage_lut(pg, luts + LUT_PGRAD * UPF_LUT_ENTRIES);
   stage_lut(vl, luts + LUT_VISC * UPF_LUT_ENTRIES);
   __syncthreads();
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t lane = threadIdx.x & 31, sub = lane % kLanes, lead = lane - sub;
+  const uint32_t i = (blockIdx.x * kBlock + threadIdx.x) / kLanes;
+  // component c, term t of the warp's particle q at [c * kTerms * kPer +
+  // (t / 4) * 4 * kPer + 4 * q + t % 4]
+  static_assert(kTerms % 4 == 0, "terms are read four at a time");
+  float* const terms = term_mem + (kLanes > 1 ? (threadIdx.x / 32) * (3 * kTerms * kPer) + 4 * (lane / kLanes) : 0);
+  auto term_at = [&](uint32_t t) { return terms + (t / 4) * 4 * kPer + t % 4; };
   double ke = 0, mx = 0, my = 0, mz = 0;
+  const int32_t ti = i < n ? B.type[i] : -1;
+  const bool liquid = ti == UPF_LIQUID;
+  float4 xi = make_float4(0, 0, 0, 0), vi = xi;
   if (i < n) {
-    const int32_t ti = B.type[i];
-    float4 xi = B.pos[i], vi = B.vel[i];
-    if (ti == UPF_LIQUID) {
-      const float m = P.mass, h = P.h;
-      const float di = rho[i], pi = press[i];
-      const float invD = (float)(1.0 / (double)di);
-      const float pVol = m * invD;
-      float fx = 0, fy = 0, fz = 0;
-      struct WNb {
-        float4 x, v;
-        float d, p;
-        int32_t t;
-      };
-      const float4* __restrict__ bpos = B.pos;
-      const float4* __restrict__ bvel = B.vel;
-      const int32_t* __restrict__ btype = B.type;
-      // positions are those the list was built at: entries are within h and
-      // carry their kernel-table bin
-      for_neighbors_bin(
-          nbr + i, lval + i, P.nstride, ncnt[i],
-          [&](uint32_t code) {
-            WNb s;
-            // boundary particles (array tails) are FROZEN and skipped below
-            s.t = __ldg(btype + code);
-            s.x = __ldg(bpos + code);
-            s.v = __ldg(bvel + code);
-            s.d = __ldg(rho + code);
-            s.p = __ldg(press + code);
-            return s;
-          },
-          [&](uint32_t, uint32_t bin, const WNb& s) {
-        if (s.t != UPF_LIQUID) return;
-        const float4 xj = s.x;
-        const float kv = vl[bin];
-        const float dj = s.d, pj = s.p;
-        const float nVol = m / dj;
-        const float dvx = xi.x - xj.x, dvy = xi.y - xj.y, dvz = xi.z - xj.z;
-        const float g = pg[bin];
-        const float grad = pi * invD * invD + pj / (dj * dj);
-        fx = fx - dvx * g * grad * m * m;
-        fy = fy - dvy * g * grad * m * m;
-        fz = fz - dvz * g * grad * m * m;
-        const float4 vj = s.v;
-        const float vx = vi.x - vj.x, vy = vi.y - vj.y, vz = vi.z - vj.z;
-        fx = fx - vx * pVol * nVol * P.visc * kv;
-        fy = fy - vy * pVol * nVol * P.visc * kv;
-        fz = fz - vz * pVol * nVol * P.visc * kv;
-        if (P.flags & UPF_FLAG_SURFACE_TENSION) {
-          const float d = dist3(xi, xj);
-          if (!(d >= h * 0.25f)) return;
-          const float sp = cohesion_spline(d, h);
-          const float inv = 1.0f / d;
-          fx = fx - dvx * P.st_gamma * m * m * sp * inv;
-          fy = fy - dvy * P.st_gamma * m * m * sp * inv;
-          fz = fz - dvz * P.st_gamma * m * m * sp * inv;
+    xi = B.pos[i];
+    vi = B.vel[i];
+  }
+  const float m = P.mass, h = P.h;
+  const uint32_t cnt = liquid ? ncnt[i] : 0u;
+  const float invD = liquid ? (float)(1.0 / (double)rho[i]) : 0.0f;
+  const float pVol = m * invD;
+  const float qi = liquid ? press[i] * invD * invD : 0.0f;
+  float f[3] = {0, 0, 0};
+  float fc = 0;  // with several lanes, lane c's sum is component c
+  const uint32_t walk = kLanes > 1 ? __reduce_max_sync(0xffffffffu, cnt) : cnt;
+  for (uint32_t k0 = 0; k0 < walk; k0 += kEntries) {
+    float4 xj[kForceRows], vj[kForceRows];
+    uint32_t bin[kForceRows];
+#pragma unroll
+    for (int r = 0; r < kForceRows; ++r) {
+      const uint32_t k = k0 + r * kLanes + sub;
+      if (k < cnt) {
+        const uint32_t code = __ldg(nbr + (size_t)k * P.nstride + i);
+        bin[r] = __ldg(lval + (size_t)k * P.nstride + i);
+        xj[r] = __ldg(xq + code);
+        vj[r] = __ldg(vn + code);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < kForceRows; ++r) {
+      const uint32_t k = k0 + r * kLanes + sub;
+      float t[3][3] = {};  // [pressure, viscosity, surface tension][component]; zeros change no sum
+      if (k < cnt && !(vj[r].w < 0.0f)) {  // (a negative volume: not a liquid neighbour)
+        const float nVol = vj[r].w, kv = vl[bin[r]], g = pg[bin[r]];
+        const float grad = qi + xj[r].w;
+        const float dx[3] = {xi.x - xj[r].x, xi.y - xj[r].y, xi.z - xj[r].z};
+        const float dv[3] = {vi.x - vj[r].x, vi.y - vj[r].y, vi.z - vj[r].z};
+        float sp = 0.0f, inv = 0.0f;
+        bool surface = false;
+        if (kSurface) {
+          const float d = dist3(xi, xj[r]);
+          surface = d >= h * 0.25f;
+          if (surface) {
+            sp = cohesion_spline(d, h);
+            inv = 1.0f / d;
+          }
         }
-          });
-      fy -= m * P.gravity;
-      force[i] = f4(fx, fy, fz);
-      integrate_store(P, i, xi, vi, make_float3(fx, fy, fz), A, keysA, B, ke, mx, my, mz);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          t[0][c] = dx[c] * g * grad * m * m;
+          t[1][c] = dv[c] * pVol * nVol * P.visc * kv;
+          if (kSurface && surface) t[2][c] = dx[c] * P.st_gamma * m * m * sp * inv;
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (uint32_t p = 0; p < kParts; ++p) {
+          if (kLanes == 1)
+            f[c] = f[c] - t[p][c];
+          else
+            term_at((r * kLanes + sub) * kParts + p)[c * (kTerms * kPer)] = t[p][c];
+        }
+    }
+    if (kLanes > 1) {
+      __syncwarp();
+      if (sub < 3) {
+#pragma unroll
+        for (uint32_t t = 0; t < kTerms; t += 4) {
+          const float4 q = *reinterpret_cast<const float4*>(term_at(t) + sub * (kTerms * kPer));
+          fc = fc - q.x;
+          fc = fc - q.y;
+          fc = fc - q.z;
+          fc = fc - q.w;
+        }
+      }
+      __syncwarp();
+    }
+  }
+  if (kLanes > 1) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) f[c] = __shfl_sync(0xffffffffu, fc, lead + c);
+  }
+  if (i < n && sub == 0) {
+    if (liquid) {
+      f[1] -= m * P.gravity;
+      force[i] = f4(f[0], f[1], f[2]);
+      integrate_store(P, i, xi, vi, make_float3(f[0], f[1], f[2]), A, keysA, B, ke, mx, my, mz);
     } else {
       A.pos[i] = xi;
       A.vel[i] = vi;
@@ -2432,6 +2490,30 @@ __global__ void __launch_bounds__(kBlock) k_static_wvol(DevParams P, uint32_t ns
   if (inv != 0.0f) wvol[i] = (float)(1.0 / (double)inv);
 }
 
+// CopyList, four 16-byte words a thread in flight. Bound by HBM when large (63
+// MB of a 1,048,576-particle state: 23 us), by its one launch when small.
+__global__ void __launch_bounds__(kBlock) k_copy_arrays(CopyList L) {
+  const uint64_t step = (uint64_t)gridDim.x * kBlock;
+  const uint64_t t0 = (uint64_t)blockIdx.x * kBlock + threadIdx.x;
+  for (int a = 0; a < L.count; ++a) {
+    const uint64_t words = L.bytes[a] / 16;
+    const uint4* __restrict__ src = static_cast<const uint4*>(L.src[a]);
+    uint4* __restrict__ dst = static_cast<uint4*>(L.dst[a]);
+    for (uint64_t w = t0; w < words; w += 4 * step) {
+      uint4 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (w + u * step < words) v[u] = src[w + u * step];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (w + u * step < words) dst[w + u * step] = v[u];
+    }
+    const uint64_t rest = (L.bytes[a] - words * 16) / 4;
+    if (t0 < rest)
+      reinterpret_cast<uint32_t*>(dst + words)[t0] = reinterpret_cast<const uint32_t*>(src + words)[t0];
+  }
+}
+
 inline uint32_t grid_of(uint32_t n) { return (n + kBlock - 1) / kBlock; }
 
 // ---- launches of the tunable passes at a LaunchShape
@@ -2445,14 +2527,15 @@ inline int nlist_warp_particles(const LaunchShape& sh, uint32_t n) {
   return sh.nlist_mode == 1 && w > 4 ? w / 2 : w;
 }
 
-template <bool kBatch, bool kMerged>
+template <bool kBatch, bool kMerged, bool kWcsph = false>
 cudaError_t run_nlist(const LaunchShape& sh, cudaStream_t st, const DevParams& P, const BatchView& bv, uint32_t n,
                       const float4* pos, const float4* mpos, const uint32_t* cstart, const uint32_t* cend,
-                      uint32_t* nbr, uint32_t* lval, uint32_t* ncnt, const float* luts, DevState* stp) {
+                      uint32_t* nbr, uint32_t* lval, uint32_t* ncnt, const float* luts, DevState* stp,
+                      const WcsphOut& wc = WcsphOut{}) {
 #define UPF_NL(T, W)                                                                                           \
-  k_build_nlist<kBatch, kMerged, T, W><<<(n + T / 32 * W - 1) / (T / 32 * W), T, nlist_smem<T, W>(), st>>>(P, bv, n, pos, mpos,  \
+  k_build_nlist<kBatch, kMerged, kWcsph, T, W><<<(n + T / 32 * W - 1) / (T / 32 * W), T, nlist_smem<T, W>(), st>>>(P, bv, n, pos, mpos,  \
                                                                                         cstart, cend, nbr, lval, \
-                                                                                        ncnt, luts, stp)
+                                                                                        ncnt, luts, stp, wc)
   switch (sh.nlist_threads * 100 + nlist_warp_particles(sh, n)) {
     case 6404: UPF_NL(64, 4); break;
     case 6408: UPF_NL(64, 8); break;
@@ -2547,10 +2630,10 @@ cudaError_t run_pforce(const LaunchShape& sh, cudaStream_t st, const DevParams& 
 // ----------------------------------------------------------------- launchers
 // The list build's shapes whose shared memory is over 48 KB are opted in on
 // the current device, once per device (before any capture that launches them).
-template <bool kBatch, bool kMerged>
+template <bool kBatch, bool kMerged, bool kWcsph>
 static cudaError_t nlist_opt_in() {
   static_assert(nlist_smem<256, 16>() + 3072 <= 48 * 1024, "the other shapes fit without");
-  return cudaFuncSetAttribute(k_build_nlist<kBatch, kMerged, 256, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  return cudaFuncSetAttribute(k_build_nlist<kBatch, kMerged, kWcsph, 256, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)nlist_smem<256, 32>());
 }
 
@@ -2579,13 +2662,24 @@ cudaError_t pipeline_init() {
   if (e != cudaSuccess) return e;
   std::lock_guard<std::mutex> lock(mu);
   if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
-  if ((e = nlist_opt_in<false, false>()) != cudaSuccess) return e;
-  if ((e = nlist_opt_in<false, true>()) != cudaSuccess) return e;
-  if ((e = nlist_opt_in<true, false>()) != cudaSuccess) return e;
+  if ((e = nlist_opt_in<false, false, false>()) != cudaSuccess) return e;
+  if ((e = nlist_opt_in<false, true, false>()) != cudaSuccess) return e;
+  if ((e = nlist_opt_in<true, false, false>()) != cudaSuccess) return e;
+  if ((e = nlist_opt_in<false, false, true>()) != cudaSuccess) return e;
+  if ((e = nlist_opt_in<false, true, true>()) != cudaSuccess) return e;
   if ((e = loop_opt_in<false>()) != cudaSuccess) return e;
   if ((e = loop_opt_in<true>()) != cudaSuccess) return e;
   if (dev >= 0 && dev < 64) done[dev] = true;
   return cudaSuccess;
+}
+
+cudaError_t copy_arrays(const CopyList& list, cudaStream_t st) {
+  uint64_t most = 0;
+  for (int a = 0; a < list.count; ++a) most = std::max(most, list.bytes[a] / 16);
+  if (!list.count) return cudaSuccess;
+  const uint64_t blocks = std::min<uint64_t>((most + kBlock * 4 - 1) / (kBlock * 4) + 1, 148 * 16);
+  k_copy_arrays<<<(uint32_t)blocks, kBlock, 0, st>>>(list);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_sort_phase(System& s, cudaStream_t st) {
@@ -2638,7 +2732,9 @@ static bool stages_lists(const System& s) {
                                           loop_mode_staged(sh.pforce_mode));
 }
 
-cudaError_t launch_neighbor_phase(System& s, cudaStream_t st) {
+static WcsphOut wcsph_out(System& s) { return WcsphOut{s.B.vel, s.B.type, s.rho, s.press, s.pq, s.xs}; }
+
+cudaError_t launch_neighbor_phase(System& s, cudaStream_t st, bool with_density) {
   const uint32_t n = s.n_dyn;
   k_step_init<<<1, 1, 0, st>>>(s.st, s.prm.method == UPF_METHOD_WCSPH ? 1 : 0);
   if (n == 0) return cudaGetLastError();
@@ -2651,11 +2747,16 @@ cudaError_t launch_neighbor_phase(System& s, cudaStream_t st) {
                                                   3 * (int)s.dp.cell_shift, s.ncells, s.mpos, s.mcells,
                                                   s.mcells + s.ncells);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    e = run_nlist<false, true>(s.shape, st, s.dp, BatchView{}, n, s.B.pos, s.mpos, s.mcells, s.mcells + s.ncells, s.nbr,
-                               s.lval, s.ncnt, s.luts, s.st);
+    const uint32_t *ms = s.mcells, *me = s.mcells + s.ncells;
+    e = with_density ? run_nlist<false, true, true>(s.shape, st, s.dp, BatchView{}, n, s.B.pos, s.mpos, ms, me, s.nbr,
+                                                    s.lval, s.ncnt, s.luts, s.st, wcsph_out(s))
+                     : run_nlist<false, true>(s.shape, st, s.dp, BatchView{}, n, s.B.pos, s.mpos, ms, me, s.nbr, s.lval,
+                                              s.ncnt, s.luts, s.st);
   } else {
-    e = run_nlist<false, false>(s.shape, st, s.dp, BatchView{}, n, s.B.pos, s.B.pos, s.cstart, s.cend, s.nbr, s.lval,
-                                s.ncnt, s.luts, s.st);
+    e = with_density ? run_nlist<false, false, true>(s.shape, st, s.dp, BatchView{}, n, s.B.pos, s.B.pos, s.cstart,
+                                                     s.cend, s.nbr, s.lval, s.ncnt, s.luts, s.st, wcsph_out(s))
+                     : run_nlist<false, false>(s.shape, st, s.dp, BatchView{}, n, s.B.pos, s.B.pos, s.cstart, s.cend,
+                                               s.nbr, s.lval, s.ncnt, s.luts, s.st);
   }
   if (e != cudaSuccess || !stages_lists(s)) return e;
   return launch_stage_lists(s, st);
@@ -2665,8 +2766,7 @@ cudaError_t launch_force_phase(System& s, cudaStream_t st) {
   const uint32_t n = s.n_dyn;
   if (n == 0) return cudaSuccess;
   if (s.prm.method == UPF_METHOD_WCSPH) {
-    k_wcsph_density<<<grid_of(n), kBlock, 0, st>>>(s.dp, n, s.B.pos, s.B.type, s.lval, s.ncnt, s.luts, s.rho,
-                                                   s.press);
+    k_wcsph_density<<<grid_of(n), kBlock, 0, st>>>(s.dp, n, s.B.pos, s.lval, s.ncnt, s.luts, wcsph_out(s));
   } else {
     return run_external<false>(s.shape, st, s.dp, BatchView{}, n, s.B, s.wvol, s.rb.id_body, s.nbr, s.ncnt, s.luts,
                                s.force, s.pforce, s.xs, s.press, s.pq, s.st);
@@ -2816,8 +2916,19 @@ cudaError_t launch_integrate_phase(System& s, cudaStream_t st) {
   const uint32_t n = s.n_dyn;
   if (n == 0) return cudaSuccess;
   if (s.prm.method == UPF_METHOD_WCSPH) {
-    k_wcsph_force_integrate<<<grid_of(n), kBlock, 0, st>>>(s.dp, n, s.B, s.A, s.keysA, s.nbr, s.lval, s.ncnt,
-                                                           s.luts, s.rho, s.press, s.force, s.st);
+    // four lanes a particle while they all find room on the SMs at once
+#define UPF_WF(L, S)                                                                                             \
+  k_wcsph_force_integrate<L, S><<<(uint32_t)(((uint64_t)n * L + kBlock - 1) / kBlock), kBlock, 0, st>>>(           \
+      s.dp, n, s.B, s.A, s.keysA, s.nbr, s.lval, s.ncnt, s.luts, s.rho, s.press, s.pq, s.xs, s.force, s.st)
+    const bool surface = s.prm.flags & UPF_FLAG_SURFACE_TENSION;
+    if (n <= 65536) {
+      if (surface) UPF_WF(4, true);
+      else UPF_WF(4, false);
+    } else {
+      if (surface) UPF_WF(1, true);
+      else UPF_WF(1, false);
+    }
+#undef UPF_WF
   } else {
     k_pcisph_integrate<false><<<grid_of(n), kBlock, 0, st>>>(s.dp, BatchView{}, n, s.B, s.A, s.keysA, s.force, s.pforce, s.rho, s.press,
                                                       s.st);

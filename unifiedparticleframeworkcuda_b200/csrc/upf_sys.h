@@ -169,6 +169,7 @@ struct System {
   float4* xs = nullptr;
   float* rho = nullptr;
   float* press = nullptr;
+  // (WCSPH keeps what its force pass gathers in pq and xs: WcsphOut)
   float4* pq = nullptr;        // (position, press / rest_density^2): the pressure-force pass's one gather
   float* wvol = nullptr;       // Akinci volume per neighbour index (dynamic, then boundary tail)
 
@@ -301,6 +302,23 @@ struct BatchSystem {
   std::vector<void*> checkpoint_slots;
 };
 
+// upf_pipeline.cu: several device arrays copied by one launch (checkpoints: 7
+// arrays of a small system are 7 copies of 2 us otherwise). Addresses are
+// multiples of 16, sizes of 4.
+struct CopyList {
+  static constexpr int kMax = 8;
+  const void* src[kMax];
+  void* dst[kMax];
+  uint64_t bytes[kMax];
+  int count = 0;
+  void add(void* d, const void* s, uint64_t n) {
+    if (!n) return;
+    src[count] = s;
+    dst[count] = d;
+    bytes[count++] = n;
+  }
+};
+cudaError_t copy_arrays(const CopyList& list, cudaStream_t st);
 // upf_pipeline.cu: per-device set-up of the pass kernels (before any launch or capture)
 cudaError_t pipeline_init();
 // upf_pipeline.cu: neighbour lists of one sorted set without boundary set
@@ -384,7 +402,8 @@ int rigid_launches_per_step(const System& s);
 
 // upf_pipeline.cu: phase launchers (all asynchronous on s.stream)
 cudaError_t launch_sort_phase(System& s, cudaStream_t st);
-cudaError_t launch_neighbor_phase(System& s, cudaStream_t st);
+// with_density: the WCSPH density pass in the same launch
+cudaError_t launch_neighbor_phase(System& s, cudaStream_t st, bool with_density = false);
 cudaError_t launch_force_phase(System& s, cudaStream_t st);
 cudaError_t launch_loop_init(System& s, cudaStream_t st);
 cudaError_t launch_loop_body(System& s, cudaStream_t st, cudaGraphConditionalHandle h, bool use_handle);
