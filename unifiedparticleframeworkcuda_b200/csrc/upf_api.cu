@@ -492,10 +492,9 @@ upf_status build_step_graph(System& s) {
   parts.pre = [](void* c, cudaStream_t st) {
     System& S = *static_cast<System*>(c);
     const bool pcisph = S.prm.method == UPF_METHOD_PCISPH;
-    cudaError_t e = launch_sort_phase(S, st);
-    if (e == cudaSuccess) e = launch_neighbor_phase(S, st, !pcisph);
+    cudaError_t e = launch_sort_phase(S, st, true);
+    if (e == cudaSuccess) e = launch_neighbor_phase(S, st, true);
     if (e == cudaSuccess && pcisph) e = launch_force_phase(S, st);
-    if (e == cudaSuccess && pcisph) e = launch_loop_init(S, st);
     return e;
   };
   s.loop_in_graph = loop_fused(s);
@@ -878,9 +877,9 @@ upf_status upf_create(const upf_params* p, int device, uint32_t capacity, upf_sy
   ALLOC(s->nbr, (size_t)s->nstride * p->max_neighbors);
   ALLOC(s->lval, (size_t)s->nstride * ((p->max_neighbors + 3) & ~3u));
   ALLOC(s->ncnt, c);
-  ALLOC(s->cstart, s->ncells); ALLOC(s->cend, s->ncells);
+  ALLOC(s->cells, (size_t)4 * s->ncells);
   ALLOC(s->sstart, s->ncells); ALLOC(s->send, s->ncells);
-  ALLOC(s->mpos, c); ALLOC(s->mcells, (size_t)2 * s->ncells);
+  ALLOC(s->mpos, c);
   ALLOC(s->spos, c); ALLOC(s->skeys, c); ALLOC(s->sid, c);
   ALLOC(s->luts, 5 * UPF_LUT_ENTRIES + kThresholds);
   ALLOC(s->st, 1); ALLOC(s->loop_sync, 2); ALLOC(s->loop_max, 2);
@@ -2050,8 +2049,8 @@ upf_status upf_get_sorted_keys(upf_system* s, uint32_t* keys, uint32_t* ids, uin
 
 upf_status upf_get_cell_ranges(upf_system* s, uint32_t* start, uint32_t* end, uint32_t* ncells_out) {
   UPF_TRY(phase_guard(s));
-  if (start) UPF_CUDA(cudaMemcpyAsync(start, s->cstart, sizeof(uint32_t) * s->ncells, cudaMemcpyDeviceToHost, s->stream));
-  if (end) UPF_CUDA(cudaMemcpyAsync(end, s->cend, sizeof(uint32_t) * s->ncells, cudaMemcpyDeviceToHost, s->stream));
+  if (start) UPF_CUDA(cudaMemcpyAsync(start, s->cstart(), sizeof(uint32_t) * s->ncells, cudaMemcpyDeviceToHost, s->stream));
+  if (end) UPF_CUDA(cudaMemcpyAsync(end, s->cend(), sizeof(uint32_t) * s->ncells, cudaMemcpyDeviceToHost, s->stream));
   UPF_CUDA(cudaStreamSynchronize(s->stream));
   if (ncells_out) *ncells_out = s->ncells;
   return UPF_OK;

@@ -209,21 +209,6 @@ __device__ __forceinline__ void density_bins(const float (&r2)[kR], float factor
   }
 }
 
-// ---------------------------------------------------------------- reorder
-// CopySortedParticleValuesKernel* (particles_kernel.cu:543-654): gather the
-// state into sorted order.
-__global__ void __launch_bounds__(kBlock) k_reorder(uint32_t n, const uint32_t* __restrict__ perm,
-                                                     DynArrays A, DynArrays B, bool with_lag) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  uint32_t j = perm[i];
-  B.pos[i] = A.pos[j];
-  B.vel[i] = A.vel[j];
-  B.id[i] = A.id[j];
-  B.type[i] = A.type[j];
-  if (with_lag) B.lag[i] = A.lag[j];
-}
-
 // ---------------------------------------------------------------- neighbours
 // Squared distance with the rounding of dist3 (no sqrt).
 __device__ __forceinline__ float dist2(float4 a, float4 b) {
@@ -336,26 +321,81 @@ __global__ void __launch_bounds__(kBlock) k_wcsph_density(DevParams P, uint32_t 
 }
 
 // ---------------------------------------------------------------- neighbour lists
-// The dynamic and the boundary particles as one sequence in Morton order
+// ---------------------------------------------------------------- sorted sets
+// What starts a step, where the graph's first kernel does it: the statistics
+// (k_step_init) and the loop state (k_loop_init).
+struct StepStart {
+  DevState* st = nullptr;  // null: not here
+  unsigned long long* sync = nullptr;
+  uint32_t* loop_max = nullptr;
+  int count_step = 0;
+};
+
+__device__ __forceinline__ void step_init(DevState* st, int count_step) {
+  st->ke = 0;
+  st->mom[0] = st->mom[1] = st->mom[2] = 0;
+  st->max_neighbors = 0;
+  if (count_step) st->total_steps += 1;  // PCISPH counts its steps in the loop control
+}
+
+__device__ __forceinline__ void loop_init(DevState* st, unsigned long long* sync, uint32_t* loop_max) {
+  sync[0] = 0;  // arrivals at the fused loop's barrier
+  loop_max[0] = loop_max[1] = 0;
+  st->iteration = 0;
+  st->too_large = 1;
+  st->max_rho_bits = 0;
+  st->ke = 0;
+  st->mom[0] = st->mom[1] = st->mom[2] = 0;
+}
+
+// CopySortedParticleValuesKernel* (particles_kernel.cu:543-654): the state
+// gathered into sorted order, with the cell table of the sorted keys
+// (CalculateBlocksKernel, particles_kernel.cu:693-726: a boundary scan, into
+// tables that are zero before), and
+// the dynamic and the boundary particles as one sequence in Morton order
 // (dynamic first at equal keys), for the list build: element m holds a
 // position and, in w, the bits of its neighbour index. Each particle finds
 // its place by a binary search of the other set's sorted keys, and the cell
-// table of the sequence (start and end, as k_cell_ranges fills) follows from
-// the four keys beside it. Both sets' cells then are one contiguous range
-// each, whose order is the reference's ascending sorted-index order, and the
-// build needs no merge of its own. About 20 dependent loads a particle, all
-// of them cached: 9 us for 1,048,576 + 279,308 particles.
-__global__ void __launch_bounds__(kBlock) k_merge_sets(uint32_t n, const uint32_t* __restrict__ keys,
-                                                        const float4* __restrict__ pos, uint32_t ns,
-                                                        const uint32_t* __restrict__ skeys,
-                                                        const float4* __restrict__ spos, uint32_t static_base,
-                                                        int shift, uint32_t ncells, float4* __restrict__ mpos,
-                                                        uint32_t* __restrict__ mstart, uint32_t* __restrict__ mend) {
+// table of the sequence follows from the four keys beside it. Both sets'
+// cells then are one contiguous range each, whose order is the reference's
+// ascending sorted-index order, and the build needs no merge of its own.
+// One launch for what were four (and a memory clearing): a launch costs a
+// small system's step about 2 us, and a large one's keys are read once.
+__global__ void __launch_bounds__(kBlock) k_reorder(
+    uint32_t n, const uint32_t* __restrict__ perm, const uint32_t* __restrict__ keys, DynArrays A, DynArrays B,
+    bool with_lag, int shift, uint32_t ncells, uint32_t* __restrict__ cstart, uint32_t* __restrict__ cend, uint32_t ns,
+    const uint32_t* __restrict__ skeys, const float4* __restrict__ spos, uint32_t static_base,
+    float4* __restrict__ mpos, uint32_t* __restrict__ mstart, uint32_t* __restrict__ mend, const StepStart start) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t == 0 && start.st) {
+    step_init(start.st, start.count_step);
+    if (start.sync) loop_init(start.st, start.sync, start.loop_max);
+  }
   if (t >= n + ns) return;
   const bool dyn = t < n;
   const uint32_t j = dyn ? t : t - n;  // place in the own set
-  const uint32_t key = dyn ? keys[j] : skeys[j];
+  const uint32_t* __restrict__ own = dyn ? keys : skeys;
+  const uint32_t nown = dyn ? n : ns;
+  const uint32_t key = own[j], c = key >> shift;
+  const bool first = j == 0 || (own[j - 1] >> shift) != c;
+  const bool last = j + 1 == nown || (own[j + 1] >> shift) != c;
+  float4 x;
+  if (dyn) {
+    const uint32_t from = perm[j];
+    x = A.pos[from];
+    B.pos[j] = x;
+    B.vel[j] = A.vel[from];
+    B.id[j] = A.id[from];
+    B.type[j] = A.type[from];
+    if (with_lag) B.lag[j] = A.lag[from];
+    if (c < ncells) {
+      if (first) cstart[c] = j;
+      if (last) cend[c] = j + 1;
+    }
+  } else {
+    x = spos[j];
+  }
+  if (!ns) return;  // the sequence is the dynamic set itself
   const uint32_t* __restrict__ other = dyn ? skeys : keys;
   const uint32_t no = dyn ? ns : n;
   // elements of the other set that come before: keys below, and for a
@@ -370,15 +410,11 @@ __global__ void __launch_bounds__(kBlock) k_merge_sets(uint32_t n, const uint32_
       hi = mid;
   }
   const uint32_t m = j + lo;
-  float4 x = dyn ? pos[j] : spos[j];
   x.w = __uint_as_float(dyn ? j : static_base + j);
   mpos[m] = x;
-  const uint32_t c = key >> shift;
   if (c >= ncells) return;
-  const uint32_t* __restrict__ own = dyn ? keys : skeys;
-  const uint32_t nown = dyn ? n : ns;
-  if ((j == 0 || (own[j - 1] >> shift) != c) && (lo == 0 || (other[lo - 1] >> shift) != c)) mstart[c] = m;
-  if ((j + 1 == nown || (own[j + 1] >> shift) != c) && (lo == no || (other[lo] >> shift) != c)) mend[c] = m + 1;
+  if (first && (lo == 0 || (other[lo - 1] >> shift) != c)) mstart[c] = m;
+  if (last && (lo == no || (other[lo] >> shift) != c)) mend[c] = m + 1;
 }
 
 // GetNeighbors (UnifiedPhysics.cpp:2242-2280) with ZIndex::BoxQuery
@@ -388,7 +424,7 @@ __global__ void __launch_bounds__(kBlock) k_merge_sets(uint32_t n, const uint32_
 // the reference's query box, hence in these cells, so the candidate set
 // holds all of the reference's neighbours. Cells are visited in ascending
 // Morton order, each a contiguous range of the sorted set (the dynamic
-// particles, or both sets merged: kMerged, k_merge_sets). The list therefore
+// particles, or both sets merged: kMerged, k_reorder). The list therefore
 // comes out in the reference's ascending sorted-index order, and membership
 // is the reference's exact test: j != i and |x_i - x_j| < h in float. Each
 // entry also records a list value at the current positions: its kernel-table
@@ -1870,21 +1906,10 @@ __global__ void __launch_bounds__(kStageChunk, pforce_staged_min_blocks(kRows)) 
 }
 
 __global__ void k_loop_init(DevState* st, unsigned long long* sync, uint32_t* loop_max) {
-  sync[0] = 0;  // arrivals at the fused loop's barrier
-  loop_max[0] = loop_max[1] = 0;
-  st->iteration = 0;
-  st->too_large = 1;
-  st->max_rho_bits = 0;
-  st->ke = 0;
-  st->mom[0] = st->mom[1] = st->mom[2] = 0;
+  loop_init(st, sync, loop_max);
 }
 
-__global__ void k_step_init(DevState* st, int count_step) {
-  st->ke = 0;
-  st->mom[0] = st->mom[1] = st->mom[2] = 0;
-  st->max_neighbors = 0;
-  if (count_step) st->total_steps += 1;  // PCISPH counts its steps in the loop control
-}
+__global__ void k_step_init(DevState* st, int count_step) { step_init(st, count_step); }
 
 // Loop control of PredictionCorrectionStep (UnifiedPhysics.cpp:5376-5420):
 // continue while iteration < min_loops, or the error is still too large and
@@ -2682,18 +2707,29 @@ cudaError_t copy_arrays(const CopyList& list, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_sort_phase(System& s, cudaStream_t st) {
+cudaError_t launch_sort_phase(System& s, cudaStream_t st, bool starts_step) {
   const uint32_t n = s.n_dyn;
-  if (n == 0) return cudaSuccess;
+  if (n == 0) {
+    if (starts_step) {
+      k_step_init<<<1, 1, 0, st>>>(s.st, s.prm.method == UPF_METHOD_WCSPH ? 1 : 0);
+      if (s.prm.method == UPF_METHOD_PCISPH) k_loop_init<<<1, 1, 0, st>>>(s.st, s.loop_sync, s.loop_max);
+    }
+    return cudaGetLastError();
+  }
   uint32_t* kalt = s.sort_tmp;
   uint32_t* valt = kalt + ((n + 63) & ~63u);
   uint32_t* counts = valt + ((n + 63) & ~63u);
   cudaError_t e = radix_sort_pairs(s.keysA, s.perm, kalt, valt, counts, n, s.key_bits, true, st);
   if (e != cudaSuccess) return e;
-  k_reorder<<<grid_of(n), kBlock, 0, st>>>(n, s.perm, s.A, s.B, s.prm.method == UPF_METHOD_PCISPH);
+  if ((e = cudaMemsetAsync(s.cells, 0, sizeof(uint32_t) * s.ncells * (s.n_static ? 4 : 2), st)) != cudaSuccess) return e;
+  StepStart start;
+  const bool pcisph = s.prm.method == UPF_METHOD_PCISPH;
+  if (starts_step) start = StepStart{s.st, pcisph ? s.loop_sync : nullptr, s.loop_max, pcisph ? 0 : 1};
+  k_reorder<<<grid_of(n + s.n_static), kBlock, 0, st>>>(
+      n, s.perm, s.keysA, s.A, s.B, pcisph, 3 * (int)s.dp.cell_shift, s.ncells, s.cstart(), s.cend(), s.n_static,
+      s.skeys, s.spos, s.dp.static_base, s.mpos, s.mstart(), s.mend(), start);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  if ((e = launch_rigid_slots(s, st)) != cudaSuccess) return e;
-  return cell_ranges(s.keysA, n, 3 * (int)s.dp.cell_shift, s.ncells, s.cstart, s.cend, st);
+  return launch_rigid_slots(s, st);
 }
 
 // The union and union positions of each chunk's lists (k_stage_lists).
@@ -2734,28 +2770,23 @@ static bool stages_lists(const System& s) {
 
 static WcsphOut wcsph_out(System& s) { return WcsphOut{s.B.vel, s.B.type, s.rho, s.press, s.pq, s.xs}; }
 
-cudaError_t launch_neighbor_phase(System& s, cudaStream_t st, bool with_density) {
+cudaError_t launch_neighbor_phase(System& s, cudaStream_t st, bool in_step) {
   const uint32_t n = s.n_dyn;
-  k_step_init<<<1, 1, 0, st>>>(s.st, s.prm.method == UPF_METHOD_WCSPH ? 1 : 0);
+  if (!in_step) k_step_init<<<1, 1, 0, st>>>(s.st, s.prm.method == UPF_METHOD_WCSPH ? 1 : 0);
   if (n == 0) return cudaGetLastError();
   s.lists_staged = false;
+  const bool with_density = in_step && s.prm.method == UPF_METHOD_WCSPH;
   cudaError_t e;
   if (s.n_static) {
-    const uint32_t all = n + s.n_static;
-    if ((e = cudaMemsetAsync(s.mcells, 0, 2 * sizeof(uint32_t) * s.ncells, st)) != cudaSuccess) return e;
-    k_merge_sets<<<grid_of(all), kBlock, 0, st>>>(n, s.keysA, s.B.pos, s.n_static, s.skeys, s.spos, s.dp.static_base,
-                                                  3 * (int)s.dp.cell_shift, s.ncells, s.mpos, s.mcells,
-                                                  s.mcells + s.ncells);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    const uint32_t *ms = s.mcells, *me = s.mcells + s.ncells;
+    const uint32_t *ms = s.mstart(), *me = s.mend();
     e = with_density ? run_nlist<false, true, true>(s.shape, st, s.dp, BatchView{}, n, s.B.pos, s.mpos, ms, me, s.nbr,
                                                     s.lval, s.ncnt, s.luts, s.st, wcsph_out(s))
                      : run_nlist<false, true>(s.shape, st, s.dp, BatchView{}, n, s.B.pos, s.mpos, ms, me, s.nbr, s.lval,
                                               s.ncnt, s.luts, s.st);
   } else {
-    e = with_density ? run_nlist<false, false, true>(s.shape, st, s.dp, BatchView{}, n, s.B.pos, s.B.pos, s.cstart,
-                                                     s.cend, s.nbr, s.lval, s.ncnt, s.luts, s.st, wcsph_out(s))
-                     : run_nlist<false, false>(s.shape, st, s.dp, BatchView{}, n, s.B.pos, s.B.pos, s.cstart, s.cend,
+    e = with_density ? run_nlist<false, false, true>(s.shape, st, s.dp, BatchView{}, n, s.B.pos, s.B.pos, s.cstart(),
+                                                     s.cend(), s.nbr, s.lval, s.ncnt, s.luts, s.st, wcsph_out(s))
+                     : run_nlist<false, false>(s.shape, st, s.dp, BatchView{}, n, s.B.pos, s.B.pos, s.cstart(), s.cend(),
                                                s.nbr, s.lval, s.ncnt, s.luts, s.st);
   }
   if (e != cudaSuccess || !stages_lists(s)) return e;
@@ -3149,9 +3180,8 @@ cudaError_t batch_launch_integrate(BatchSystem& b, cudaStream_t st) {
 }
 
 int pipeline_launches_per_step(const System& s, int iterations) {
-  int sort = radix_launches(s.n_dyn, s.key_bits) + 1 /*reorder*/ + 1 /*cells*/ + (s.rb.n_rigid ? 1 : 0) /*rigid slots*/;
-  // step init + neighbour lists (+ merge of the two sets, + staging)
-  int nl = 2 + (s.n_static ? 1 : 0) + (stages_lists(s) ? 1 : 0);
+  int sort = radix_launches(s.n_dyn, s.key_bits) + 1 /*reorder, cells, merged sets*/ + (s.rb.n_rigid ? 1 : 0) /*rigid slots*/;
+  int nl = 2 + (stages_lists(s) ? 1 : 0);  // step init + neighbour lists (+ staging)
   if (s.prm.method == UPF_METHOD_WCSPH) return sort + nl + 2;
   return sort + nl + 1 /*external*/ + 1 /*loop init*/ + 3 * iterations + 1 /*integrate*/ + rigid_launches_per_step(s);
 }

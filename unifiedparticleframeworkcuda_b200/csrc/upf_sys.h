@@ -195,15 +195,18 @@ struct System {
 
   // cells
   uint32_t ncells = 0;
-  uint32_t* cstart = nullptr;
-  uint32_t* cend = nullptr;
+  // [4][ncells]: start and end of the dynamic set's cells, then of both sets'
+  // in one sequence; cleared together
+  uint32_t* cells = nullptr;
+  uint32_t* cstart() const { return cells; }
+  uint32_t* cend() const { return cells + ncells; }
+  uint32_t* mstart() const { return cells + 2 * (size_t)ncells; }
+  uint32_t* mend() const { return cells + 3 * (size_t)ncells; }
   uint32_t* sstart = nullptr;
   uint32_t* send = nullptr;
-  // both sets in Morton order, for the list build (k_merge_sets): position
-  // and neighbour index (the bits of w), [capacity]; cell start and end,
-  // [2][ncells]
+  // both sets in Morton order, for the list build (k_reorder): position and
+  // neighbour index (the bits of w), [capacity]
   float4* mpos = nullptr;
-  uint32_t* mcells = nullptr;
 
   // boundary set
   float4* spos = nullptr;
@@ -401,9 +404,10 @@ cudaError_t launch_rigid_phase(System& s, cudaStream_t st);
 int rigid_launches_per_step(const System& s);
 
 // upf_pipeline.cu: phase launchers (all asynchronous on s.stream)
-cudaError_t launch_sort_phase(System& s, cudaStream_t st);
-// with_density: the WCSPH density pass in the same launch
-cudaError_t launch_neighbor_phase(System& s, cudaStream_t st, bool with_density = false);
+// starts_step: with the step's (and loop's) initial state
+cudaError_t launch_sort_phase(System& s, cudaStream_t st, bool starts_step = false);
+// in_step: the sort phase has started the step; WCSPH densities in the same launch
+cudaError_t launch_neighbor_phase(System& s, cudaStream_t st, bool in_step = false);
 cudaError_t launch_force_phase(System& s, cudaStream_t st);
 cudaError_t launch_loop_init(System& s, cudaStream_t st);
 cudaError_t launch_loop_body(System& s, cudaStream_t st, cudaGraphConditionalHandle h, bool use_handle);
