@@ -32,11 +32,11 @@ def run_system(upf, sc, p, as_passes, steps):
                        list(st.iteration_max_density), st.max_step_density_error_percent)
 
 
-# liquid particles (32, 16, 8, 4 and 1 lanes a particle on a B200) and the
-# support radius in spacings (2.7: 80 neighbours, more than a lane holds)
+# liquid particles (32, 16, 8, 4, 4, 2, 1 and 1 lanes a particle on a B200) and
+# the support radius in spacings (2.7: 80 neighbours, more than a lane holds)
 @pytest.mark.parametrize("block,h", [((5, 4, 3), 2.0), ((12, 12, 12), 2.0), ((12, 12, 12), 2.7), ((20, 17, 16), 2.0),
-                                     ((25, 24, 23), 2.7), ((37, 31, 25), 2.0), ((47, 39, 29), 2.7),
-                                     ((64, 43, 37), 2.0)])
+                                     ((25, 24, 23), 2.7), ((30, 28, 25), 2.0), ((37, 31, 25), 2.7),
+                                     ((47, 39, 29), 2.7), ((50, 42, 31), 2.7), ((64, 43, 37), 2.0)])
 def test_one_launch_equals_the_passes(upf_lib, block, h):
     nx, ny, nz = block
     s = 0.01

@@ -1962,9 +1962,9 @@ __global__ void k_loop_ctl(DevParams P, DevState* st, cudaGraphConditionalHandle
 // particles as the SMs hold at once (151,552 on a B200) an iteration of three
 // graph nodes is mostly the nodes: their launches, drains and cold starts,
 // and gathers with few warps to hide them. A step of 50 iterations, before
-// and now (sort, lists and forces included, about 0.12 ms): 1,728 particles
-// 1.15 and 0.36 ms, 8,000 1.31 and 0.54, 32,768 1.31 and 0.82, 53,157 1.44
-// and 1.19, 144,256 2.01 and 1.62. Above that several chunks a CTA came to
+// and now (sort, lists and forces included, about 0.1 ms): 1,728 particles
+// 1.15 and 0.33 ms, 8,000 1.31 and 0.49, 33,792 1.31 and 0.78, 53,157 1.44
+// and 0.96, 144,256 2.01 and 1.5. Above that several chunks a CTA came to
 // 2.87 ms at 196,608 against 2.73 with the passes as launches of their own
 // (3.45 and 3.23 at 262,144), so those keep the launches.
 // kLanes: lanes a particle. With few particles one thread each leaves an SM a
@@ -2008,7 +2008,7 @@ __device__ __forceinline__ unsigned long long grid_wait(unsigned long long* arri
   return seen_all;
 }
 
-// Threads an SM, at 64 registers.
+// The most threads an SM, at 64 registers.
 constexpr int kLoopResident = 1024;
 template <int kThreads, int kLanes, int kHeld, int kRows>
 constexpr size_t loop_smem() {
@@ -2054,7 +2054,7 @@ __global__ void __launch_bounds__(kThreads, kResident / kThreads) k_pcisph_loop(
   // [c * kTerms * kPer + (e / 4) * 4 * kPer + 4 * q + e % 4], four entries of
   // one particle side by side; missing entries are zeros (adding or taking
   // off a zero changes no sum)
-  static_assert(kLanes == 1 || (kLanes > 3 && kTerms % 4 == 0), "a lane per component; terms read four at a time");
+  static_assert(kLanes == 1 || kTerms % 4 == 0, "a lane per component; terms read four at a time");
   float* const terms = reinterpret_cast<float*>(loop_mem + 2 * kHeld * kChunk) +
                        (threadIdx.x / 32) * (3 * kTerms * kPer) + 4 * (lane / kLanes);
   auto term_at = [&](uint32_t e) { return terms + (e / 4) * 4 * kPer + e % 4; };
@@ -2167,13 +2167,18 @@ __global__ void __launch_bounds__(kThreads, kResident / kThreads) k_pcisph_loop(
       }
       if (kLanes > 1) {
         __syncwarp();
-        if (sub < 3) subtract(fc, sub);
+        if (kLanes == 2) {  // the first of two lanes takes x and z
+          subtract(fc, sub);
+          if (sub == 0) subtract(f[2], 2);
+        } else if (sub < 3) {
+          subtract(fc, sub);
+        }
         __syncwarp();
       }
     }
     if (kLanes > 1) {
 #pragma unroll
-      for (int c = 0; c < 3; ++c) f[c] = __shfl_sync(0xffffffffu, fc, lead + c);
+      for (int c = 0; c < 3; ++c) f[c] = __shfl_sync(0xffffffffu, kLanes == 2 && c == 2 ? f[2] : fc, lead + c % kLanes);
     }
     if (!active) return;
     if (sub == 0) pforce[i] = f4(f[0], f[1], f[2]);
@@ -2671,10 +2676,12 @@ static cudaError_t loop_opt_in_shape() {
 }
 template <bool kBatch>
 static cudaError_t loop_opt_in() {
-  cudaError_t e = loop_opt_in_shape<kBatch, 512, 1024, 32, 48, 1>();
-  if (e == cudaSuccess) e = loop_opt_in_shape<kBatch, 512, 1024, 16, 48, 2>();
-  if (e == cudaSuccess) e = loop_opt_in_shape<kBatch, 512, 1024, 8, 48, 4>();
+  cudaError_t e = loop_opt_in_shape<kBatch, 256, 768, 32, 48, 1>();
+  if (e == cudaSuccess) e = loop_opt_in_shape<kBatch, 256, 768, 16, 48, 2>();
+  if (e == cudaSuccess) e = loop_opt_in_shape<kBatch, 256, 768, 8, 48, 4>();
+  if (e == cudaSuccess) e = loop_opt_in_shape<kBatch, 256, 768, 4, 48, 4>();
   if (e == cudaSuccess) e = loop_opt_in_shape<kBatch, 512, 1024, 4, 48, 4>();
+  if (e == cudaSuccess) e = loop_opt_in_shape<kBatch, 256, 768, 2, 48, 4>();
   if (e == cudaSuccess) e = loop_opt_in_shape<kBatch, 128, 512, 1, 48, 8>();
   return e;
 }
@@ -2811,10 +2818,13 @@ cudaError_t launch_loop_init(System& s, cudaStream_t st) {
 }
 
 // The fused loop's shape for n particles (or slots): as many lanes a particle
-// as the SMs hold at once (1,024 threads each), in CTAs of 512, since the
-// barrier's cost is its arrivals (4,096 particles in 1,024 CTAs of 128: 11.8
-// us an iteration, in 256 of 512 5.8); one lane a particle in small CTAs at
-// first, to use every SM.
+// as the SMs hold at once, at 768 threads of 80 registers each in CTAs of 256
+// (steps of 50 iterations of 4,096, 8,000, 21,952 particles 0.400, 0.494 and
+// 0.642 ms, at 1,024 threads of 64 in CTAs of 512 0.417, 0.512 and 0.732, in
+// CTAs of 128 longer by half: the barrier's cost is its arrivals); where 1,024
+// hold twice the lanes, those (33,792: 0.782 with four lanes, 0.881 with two);
+// one lane a particle in small CTAs at first, to use every SM (53,157: 0.961
+// with two lanes, 1.072 with one).
 template <bool kBatch, int kThreads, int kResident, int kLanes, int kHeld, int kRows>
 static cudaError_t run_loop_shape(cudaStream_t st, uint32_t n, void** args) {
   constexpr uint32_t chunk = kThreads / kLanes;
@@ -2832,10 +2842,12 @@ static cudaError_t run_loop(cudaStream_t st, const DevParams& P, const BatchView
   void* args[] = {(void*)&P,    (void*)&bv,   (void*)&seg_begin, (void*)&n,     (void*)&B,      (void*)&nbr,
                   (void*)&lval, (void*)&ncnt, (void*)&luts,      (void*)&force, (void*)&pforce, (void*)&xs,
                   (void*)&rho,  (void*)&press, (void*)&pq,       (void*)&stp,   (void*)&sync,   (void*)&loop_max};
-  if (n <= sms * 32) return run_loop_shape<kBatch, 512, 1024, 32, 48, 1>(st, n, args);
-  if (n <= sms * 64) return run_loop_shape<kBatch, 512, 1024, 16, 48, 2>(st, n, args);
-  if (n <= sms * 128) return run_loop_shape<kBatch, 512, 1024, 8, 48, 4>(st, n, args);
+  if (n <= sms * 24) return run_loop_shape<kBatch, 256, 768, 32, 48, 1>(st, n, args);
+  if (n <= sms * 48) return run_loop_shape<kBatch, 256, 768, 16, 48, 2>(st, n, args);
+  if (n <= sms * 96) return run_loop_shape<kBatch, 256, 768, 8, 48, 4>(st, n, args);
+  if (n <= sms * 192) return run_loop_shape<kBatch, 256, 768, 4, 48, 4>(st, n, args);
   if (n <= sms * 256) return run_loop_shape<kBatch, 512, 1024, 4, 48, 4>(st, n, args);
+  if (n <= sms * 384) return run_loop_shape<kBatch, 256, 768, 2, 48, 4>(st, n, args);
   if (n <= sms * 512) return run_loop_shape<kBatch, 128, 512, 1, 48, 8>(st, n, args);
   // (a batch's CTA takes no more than the 256 slots that are of one scene)
   if (n <= sms * 1024) return run_loop_shape<kBatch, kBatch ? 256 : 512, 1024, 1, 0, 4>(st, n, args);
