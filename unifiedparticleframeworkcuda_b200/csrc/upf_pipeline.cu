@@ -1963,8 +1963,8 @@ __global__ void k_loop_ctl(DevParams P, DevState* st, cudaGraphConditionalHandle
 // graph nodes is mostly the nodes: their launches, drains and cold starts,
 // and gathers with few warps to hide them. A step of 50 iterations, before
 // and now (sort, lists and forces included, about 0.1 ms): 1,728 particles
-// 1.15 and 0.33 ms, 8,000 1.31 and 0.49, 33,792 1.31 and 0.78, 53,157 1.44
-// and 0.96, 144,256 2.01 and 1.5. Above that several chunks a CTA came to
+// 1.15 and 0.34 ms, 8,000 1.31 and 0.48, 33,792 1.31 and 0.77, 53,157 1.44
+// and 0.89, 109,200 1.74 and 1.15, 136,192 2.0 and 1.40. Above that several chunks a CTA came to
 // 2.87 ms at 196,608 against 2.73 with the passes as launches of their own
 // (3.45 and 3.23 at 262,144), so those keep the launches.
 // kLanes: lanes a particle. With few particles one thread each leaves an SM a
@@ -1973,8 +1973,8 @@ __global__ void k_loop_ctl(DevParams P, DevState* st, cudaGraphConditionalHandle
 // and put them in shared memory, where they are added in list order (a lane
 // per component), so that every sum keeps the reference's order.
 // kHeld: list entries a particle keeps in shared memory for the whole loop
-// (the barrier's acquire empties L1, so lists left there would come from L2
-// in every pass); longer lists go on from global memory.
+// (0: none, they come through L1 in every pass); longer lists go on from
+// global memory.
 // A CTA keeps to its particles, whose own data stays in registers. A batch's
 // scenes end their loops one by one; the CTAs of a finished scene
 // only keep the barrier.
@@ -2678,11 +2678,6 @@ template <bool kBatch>
 static cudaError_t loop_opt_in() {
   cudaError_t e = loop_opt_in_shape<kBatch, 256, 768, 32, 48, 1>();
   if (e == cudaSuccess) e = loop_opt_in_shape<kBatch, 256, 768, 16, 48, 2>();
-  if (e == cudaSuccess) e = loop_opt_in_shape<kBatch, 256, 768, 8, 48, 4>();
-  if (e == cudaSuccess) e = loop_opt_in_shape<kBatch, 256, 768, 4, 48, 4>();
-  if (e == cudaSuccess) e = loop_opt_in_shape<kBatch, 512, 1024, 4, 48, 4>();
-  if (e == cudaSuccess) e = loop_opt_in_shape<kBatch, 256, 768, 2, 48, 4>();
-  if (e == cudaSuccess) e = loop_opt_in_shape<kBatch, 128, 512, 1, 48, 8>();
   return e;
 }
 
@@ -2822,9 +2817,12 @@ cudaError_t launch_loop_init(System& s, cudaStream_t st) {
 // (steps of 50 iterations of 4,096, 8,000, 21,952 particles 0.400, 0.494 and
 // 0.642 ms, at 1,024 threads of 64 in CTAs of 512 0.417, 0.512 and 0.732, in
 // CTAs of 128 longer by half: the barrier's cost is its arrivals); where 1,024
-// hold twice the lanes, those (33,792: 0.782 with four lanes, 0.881 with two);
-// one lane a particle in small CTAs at first, to use every SM (53,157: 0.961
-// with two lanes, 1.072 with one).
+// hold twice the lanes, those (33,792: 0.773 with four lanes, 0.881 with two).
+// One lane at 768 threads an SM instead of CTAs of 128 with eight rows: 62,400
+// 0.942 and 1.140, 109,200 1.160 and 1.354. Lists are held in shared memory by
+// the smallest scenes alone, where it hides latency (1,728: 0.340, 0.363
+// without); with more lists an SM the shared memory is worth more as L1 for
+// the gathers (8,000: 0.495 held and 0.476, 53,157: 0.951 and 0.891).
 template <bool kBatch, int kThreads, int kResident, int kLanes, int kHeld, int kRows>
 static cudaError_t run_loop_shape(cudaStream_t st, uint32_t n, void** args) {
   constexpr uint32_t chunk = kThreads / kLanes;
@@ -2844,11 +2842,11 @@ static cudaError_t run_loop(cudaStream_t st, const DevParams& P, const BatchView
                   (void*)&rho,  (void*)&press, (void*)&pq,       (void*)&stp,   (void*)&sync,   (void*)&loop_max};
   if (n <= sms * 24) return run_loop_shape<kBatch, 256, 768, 32, 48, 1>(st, n, args);
   if (n <= sms * 48) return run_loop_shape<kBatch, 256, 768, 16, 48, 2>(st, n, args);
-  if (n <= sms * 96) return run_loop_shape<kBatch, 256, 768, 8, 48, 4>(st, n, args);
-  if (n <= sms * 192) return run_loop_shape<kBatch, 256, 768, 4, 48, 4>(st, n, args);
-  if (n <= sms * 256) return run_loop_shape<kBatch, 512, 1024, 4, 48, 4>(st, n, args);
-  if (n <= sms * 384) return run_loop_shape<kBatch, 256, 768, 2, 48, 4>(st, n, args);
-  if (n <= sms * 512) return run_loop_shape<kBatch, 128, 512, 1, 48, 8>(st, n, args);
+  if (n <= sms * 96) return run_loop_shape<kBatch, 256, 768, 8, 0, 4>(st, n, args);
+  if (n <= sms * 192) return run_loop_shape<kBatch, 256, 768, 4, 0, 4>(st, n, args);
+  if (n <= sms * 256) return run_loop_shape<kBatch, 512, 1024, 4, 0, 4>(st, n, args);
+  if (n <= sms * 384) return run_loop_shape<kBatch, 256, 768, 2, 0, 4>(st, n, args);
+  if (n <= sms * 768) return run_loop_shape<kBatch, 256, 768, 1, 0, 4>(st, n, args);
   // (a batch's CTA takes no more than the 256 slots that are of one scene)
   if (n <= sms * 1024) return run_loop_shape<kBatch, kBatch ? 256 : 512, 1024, 1, 0, 4>(st, n, args);
   return cudaErrorInvalidConfiguration;
