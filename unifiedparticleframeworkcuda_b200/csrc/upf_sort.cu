@@ -10,15 +10,19 @@
 //   upsweep   per-tile digit histograms (shared-memory atomics)
 //   scan      per digit, exclusive scan of its row of tile counts (one CTA
 //             per digit) and the digit's total
-//   downsweep per-tile stable ranking with warp match/ballot (each warp owns
+//   downsweep per-tile stable ranking with warp votes (each warp owns
 //             a contiguous segment of 32, 128 or 512 keys, rounds run in key
 //             order), a local sort through shared memory, and coalesced runs
 //             to global memory.
 // Stability: warps own consecutive segments and rank in order, so equal
 // digits keep their input order; an LSD sort of stable passes is stable.
-// Up to 2,048 keys one CTA runs all passes in one launch (k_radix_small): 12
-// against 21 us for the 12 launches of four passes; at 4,096 keys, which one
-// SM ranks alone, it takes 24 against 25 us and no longer pays.
+// Ranks come from a vote per bit of the digit, not from match.any, whose cost
+// grows with the distinct values in a warp (four passes of 262,144 pairs 38.8
+// against 43.0 us, 1,048,576 62.5 / 83.4, 5,204,419 264 / 360).
+// Up to 32,768 keys one CTA or one cluster runs all passes in one launch
+// (k_radix_cluster), without the gaps between 12 launches; above, the ranking
+// of more pairs an SM costs more than the gaps.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <mutex>
@@ -35,6 +39,18 @@ constexpr int kRadix = 1 << kRadixBits;
 constexpr int kThreads = 512;               // 16 warps
 constexpr int kWarps = kThreads / 32;
 static_assert(kRadix == (int)kRadixDigits, "scratch layout constants");
+
+// The lanes of the warp (all of it active) whose digit is d: a vote per bit.
+__device__ __forceinline__ uint32_t digit_peers(uint32_t d) {
+  uint32_t peers = 0xffffffffu;
+#pragma unroll
+  for (int b = 0; b < kRadixBits; ++b) {
+    const bool set = (d >> b) & 1u;
+    const uint32_t with = __ballot_sync(0xffffffffu, set);
+    peers &= set ? with : ~with;
+  }
+  return peers;
+}
 
 // kItems keys per lane: a warp ranks 32 * kItems consecutive keys, a tile is
 // kWarps warps' segments
@@ -150,16 +166,11 @@ __global__ void __launch_bounds__(kThreads) k_downsweep(const uint32_t* __restri
     k[r] = valid ? keys_in[i] : 0xffffffffu;
     v[r] = valid ? (kIotaValues ? i : vals_in[i]) : 0u;
     uint32_t d = (k[r] >> shift) & (kRadix - 1);
-    uint32_t vmask = __ballot_sync(0xffffffffu, valid);
-    local[r] = 0;
-    if (valid) {
-      uint32_t peers = __match_any_sync(vmask, d);
-      uint32_t rank = __popc(peers & lt);
-      uint32_t prior = wh[d];
-      local[r] = prior + rank;
-      __syncwarp(vmask);
-      if (rank == 0) wh[d] = prior + __popc(peers);
-    }
+    const uint32_t peers = digit_peers(d) & __ballot_sync(0xffffffffu, valid);
+    const uint32_t rank = __popc(peers & lt), prior = wh[d];
+    local[r] = prior + rank;
+    __syncwarp();
+    if (valid && rank == 0) wh[d] = prior + __popc(peers);
     __syncwarp();
   }
   __syncthreads();
@@ -241,41 +252,66 @@ __global__ void __launch_bounds__(kThreads) k_downsweep(const uint32_t* __restri
   }
 }
 
-constexpr int kSmallThreads = 1024, kSmallItems = 2;
-constexpr uint32_t kSmallMax = kSmallThreads * kSmallItems;
+constexpr int kSmallThreads = 512;
+constexpr int kSmallWarps = kSmallThreads / 32;
+constexpr int kSmallGroups = kSmallThreads / kRadix;  // of eight warps
+
+template <int kItems>
 constexpr size_t small_smem() {
-  return sizeof(uint32_t) * (kSmallThreads / 32 * kRadix + 2 * kSmallMax + kRadix);
+  return sizeof(uint2) * kSmallThreads * kItems +
+         sizeof(uint32_t) * (kSmallWarps * kRadix + kRadix + 2 * kSmallGroups * kRadix);
 }
 
-// One CTA, all passes: the keys stay in registers and shared memory, ranked
-// and exchanged as in k_downsweep.
-template <bool kIotaValues>
-__global__ void __launch_bounds__(kSmallThreads) k_radix_small(uint32_t* __restrict__ keys,
-                                                               uint32_t* __restrict__ vals, uint32_t n, int passes) {
-  constexpr int kSmallWarps = kSmallThreads / 32;
-  extern __shared__ uint32_t smem[];
-  uint32_t* whist = smem;                             // [kSmallWarps][kRadix]
-  uint32_t* skeys = whist + kSmallWarps * kRadix;     // [kSmallMax]
-  uint32_t* svals = skeys + kSmallMax;                // [kSmallMax]
-  uint32_t* digit_off = svals + kSmallMax;            // [kRadix]
+// All passes in one launch of one cluster of kCtas CTAs (one CTA: no cluster),
+// each of which holds kItems * 512 consecutive pairs of the current order in
+// registers. A pass ranks them as k_downsweep does, adds the digit counts of
+// all CTAs (read from their shared memory) to the places of its own, and sends
+// every pair to the shared memory of the CTA that holds its place.
+// Bound by the ranking (0.6 us a round of 16 warps, some 70 instructions a
+// warp) and the barriers (0.3 us each across a cluster). Four passes, us, in
+// one launch and in twelve: 900 pairs 5.5 and 25, 1,728 8.3, 4,096 11.3, 8,192
+// 11.8, 16,384 16.6 and 25.2, 32,768 on 16 CTAs 21.4 and 25.9; on 8 CTAs 26.0,
+// and 50,000 on 16 31.6 and 26.3. CTAs of 1,024 threads are 1 to 2 us longer
+// (more rows of counts to add up), pairs put in order in the CTA before they
+// are sent not shorter.
+template <bool kIotaValues, int kCtas, int kItems>
+__global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kSmallThreads)
+    k_radix_cluster(uint32_t* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t n, int passes) {
+  constexpr uint32_t kTile = kSmallThreads * kItems;
+  extern __shared__ uint2 pair_mem[];
+  uint2* const pairs = pair_mem;                                       // [kTile]
+  uint32_t* const whist = reinterpret_cast<uint32_t*>(pairs + kTile);  // [kSmallWarps][kRadix]
+  uint32_t* const count = whist + kSmallWarps * kRadix;                // [kRadix] this CTA's digit counts
+  uint32_t* const part = count + kRadix;                               // [kSmallGroups][kRadix] the groups' counts
+  uint32_t* const base = part + kSmallGroups * kRadix;                 // [kSmallGroups][kRadix] a group's first place
+  namespace cg = cooperative_groups;
+  const cg::cluster_group cluster = cg::this_cluster();
+  const auto barrier = [&] {
+    if constexpr (kCtas > 1)
+      cluster.sync();
+    else
+      __syncthreads();
+  };
+  const uint32_t cta = kCtas > 1 ? cluster.block_rank() : 0u;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t lt = lanemask_lt();
-  const uint32_t seg = warp * 32 * kSmallItems + lane;
-  uint32_t k[kSmallItems], v[kSmallItems], local[kSmallItems];
+  const uint32_t seg = warp * 32 * kItems + lane;
+  uint32_t k[kItems], v[kItems], local[kItems];
 #pragma unroll
-  for (int r = 0; r < kSmallItems; ++r) {
-    const uint32_t i = seg + r * 32;
+  for (int r = 0; r < kItems; ++r) {
+    const uint32_t i = cta * kTile + seg + r * 32;
     k[r] = i < n ? keys[i] : 0xffffffffu;  // beyond the last key: behind all others in every pass
     v[r] = i < n ? (kIotaValues ? i : vals[i]) : 0u;
   }
+  uint32_t* const wh = whist + warp * kRadix;
   for (int shift = 0; shift < passes * kRadixBits; shift += kRadixBits) {
-    for (int d = threadIdx.x; d < kSmallWarps * kRadix; d += kSmallThreads) whist[d] = 0;
-    __syncthreads();
-    uint32_t* wh = whist + warp * kRadix;
 #pragma unroll
-    for (int r = 0; r < kSmallItems; ++r) {
+    for (int d = lane; d < kRadix; d += 32) wh[d] = 0;
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < kItems; ++r) {
       const uint32_t d = (k[r] >> shift) & (kRadix - 1);
-      const uint32_t peers = __match_any_sync(0xffffffffu, d);
+      const uint32_t peers = digit_peers(d);
       const uint32_t rank = __popc(peers & lt), prior = wh[d];
       local[r] = prior + rank;
       __syncwarp();
@@ -283,60 +319,136 @@ __global__ void __launch_bounds__(kSmallThreads) k_radix_small(uint32_t* __restr
       __syncwarp();
     }
     __syncthreads();
-    if (threadIdx.x < kRadix) {
-      uint32_t acc = 0;
-#pragma unroll 8
-      for (int w = 0; w < kSmallWarps; ++w) {
-        const uint32_t t = whist[w * kRadix + threadIdx.x];
-        whist[w * kRadix + threadIdx.x] = acc;
-        acc += t;
+    // per digit: exclusive prefix over the warps of each group of eight, the
+    // groups' counts and their sum
+    {
+      const int d = threadIdx.x & (kRadix - 1), g = threadIdx.x / kRadix;
+      uint32_t run = 0;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) {
+        const uint32_t t = whist[(g * 8 + w) * kRadix + d];
+        whist[(g * 8 + w) * kRadix + d] = run;
+        run += t;
       }
-      digit_off[threadIdx.x] = acc;
+      part[g * kRadix + d] = run;
     }
     __syncthreads();
-    if (warp == 0) {  // exclusive scan of the digits' counts, 8 a lane
-      uint32_t t[8], s = 0;
+    if (threadIdx.x < kRadix) {
+      uint32_t run = 0;
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        t[q] = digit_off[lane * 8 + q];
-        s += t[q];
+      for (int g = 0; g < kSmallGroups; ++g) run += part[g * kRadix + threadIdx.x];
+      count[threadIdx.x] = run;
+    }
+    barrier();
+    // the CTAs' counts: all of a digit's keys, and those of the CTAs before
+    if (threadIdx.x < kRadix) {
+      uint32_t all = 0, before = 0;
+#pragma unroll
+      for (int c = 0; c < kCtas; ++c) {
+        const uint32_t t = kCtas > 1 ? cluster.map_shared_rank(count, c)[threadIdx.x] : count[threadIdx.x];
+        all += t;
+        if (c < (int)cta) before += t;
       }
-      uint32_t incl = s;
+      // exclusive scan of the 256 totals: in the warp, then over eight warps
+      uint32_t incl = all;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += y;
       }
-      uint32_t run = incl - s;
+      __shared__ uint32_t warp_total[kRadix / 32];
+      if (lane == 31) warp_total[warp] = incl;
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      uint32_t run = incl - all + before;
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        digit_off[lane * 8 + q] = run;
-        run += t[q];
+      for (int w = 0; w < kRadix / 32; ++w)
+        if (w < warp) run += warp_total[w];
+#pragma unroll
+      for (int g = 0; g < kSmallGroups; ++g) {
+        base[g * kRadix + threadIdx.x] = run;
+        run += part[g * kRadix + threadIdx.x];
       }
     }
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < kSmallItems; ++r) {
+    for (int r = 0; r < kItems; ++r) {
       const uint32_t d = (k[r] >> shift) & (kRadix - 1);
-      const uint32_t at = digit_off[d] + wh[d] + local[r];
-      skeys[at] = k[r];
-      svals[at] = v[r];
+      const uint32_t at = base[(warp / 8) * kRadix + d] + wh[d] + local[r];
+      uint2* const to = kCtas > 1 ? cluster.map_shared_rank(pairs, at / kTile) : pairs;
+      to[at % kTile] = make_uint2(k[r], v[r]);
     }
-    __syncthreads();
+    barrier();
 #pragma unroll
-    for (int r = 0; r < kSmallItems; ++r) {
-      k[r] = skeys[seg + r * 32];
-      v[r] = svals[seg + r * 32];
+    for (int r = 0; r < kItems; ++r) {
+      const uint2 p = pairs[seg + r * 32];
+      k[r] = p.x;
+      v[r] = p.y;
     }
   }
 #pragma unroll
-  for (int r = 0; r < kSmallItems; ++r) {
-    const uint32_t i = seg + r * 32;
+  for (int r = 0; r < kItems; ++r) {
+    const uint32_t i = cta * kTile + seg + r * 32;
     if (i < n) {
       keys[i] = k[r];
       vals[i] = v[r];
     }
   }
+}
+
+// The one-launch forms: the largest count of each, in order.
+struct SmallForm {
+  uint32_t max;
+  const void* iota;
+  const void* given;
+  uint32_t ctas;
+  size_t smem;
+};
+template <int kCtas, int kItems>
+constexpr SmallForm small_form() {
+  return {(uint32_t)kCtas * kSmallThreads * kItems, (const void*)k_radix_cluster<true, kCtas, kItems>,
+          (const void*)k_radix_cluster<false, kCtas, kItems>, (uint32_t)kCtas, small_smem<kItems>()};
+}
+const SmallForm kSmallForms[] = {
+    small_form<1, 2>(), small_form<1, 4>(), small_form<8, 2>(), small_form<8, 4>(), small_form<16, 4>(),};
+
+// The largest count the one-launch forms take on the current device: a
+// cluster of 16 needs as many free SMs in one group of the chip, which a
+// partition of it need not have. Set by radix_init.
+constexpr int kMaxDevices = 64;
+uint32_t g_small_max[kMaxDevices] = {};
+uint32_t small_max() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
+  return __atomic_load_n(&g_small_max[dev], __ATOMIC_ACQUIRE);
+}
+
+cudaError_t small_init(int dev) {
+  uint32_t fits = 0;
+  for (const SmallForm& f : kSmallForms) {
+    int clusters = 0;
+    for (const void* k : {f.iota, f.given}) {
+      cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem);
+      if (e == cudaSuccess && f.ctas > 8) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      if (e != cudaSuccess) return e;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(f.ctas);
+    cfg.blockDim = dim3(kSmallThreads);
+    cfg.dynamicSmemBytes = f.smem;
+    cudaLaunchAttribute size = {};
+    size.id = cudaLaunchAttributeClusterDimension;
+    size.val.clusterDim.x = f.ctas;
+    size.val.clusterDim.y = size.val.clusterDim.z = 1;
+    cfg.attrs = &size;
+    cfg.numAttrs = 1;
+    if (f.ctas > 1 && (cudaOccupancyMaxActiveClusters(&clusters, f.given, &cfg) != cudaSuccess || clusters < 1)) {
+      cudaGetLastError();
+      break;
+    }
+    fits = f.max;
+  }
+  if (dev >= 0 && dev < kMaxDevices) __atomic_store_n(&g_small_max[dev], fits, __ATOMIC_RELEASE);
+  return cudaSuccess;
 }
 
 }  // namespace
@@ -354,21 +466,18 @@ size_t radix_temp_bytes(uint32_t n) { return radix_temp_words(n) * sizeof(uint32
 // any stream capture that launches it).
 cudaError_t radix_init() {
   static std::mutex mu;
-  static bool done[64] = {};
+  static bool done[kMaxDevices] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   std::lock_guard<std::mutex> lock(mu);
-  if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
+  if (dev >= 0 && dev < kMaxDevices && done[dev]) return cudaSuccess;
   e = cudaFuncSetAttribute(k_downsweep<true, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)down_smem<16>());
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_downsweep<false, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)down_smem<16>());
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_radix_small<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem());
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_radix_small<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem());
-  if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = true;
+  if (e == cudaSuccess) e = small_init(dev);
+  if (e == cudaSuccess && dev >= 0 && dev < kMaxDevices) done[dev] = true;
   return e;
 }
 
@@ -382,12 +491,11 @@ cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt,
   uint32_t* totals = counts + (size_t)kRadix * ntiles;
   int passes = (key_bits + kRadixBits - 1) / kRadixBits;
   if (passes < 1) passes = 1;
-  if (n <= kSmallMax) {
-    if (iota_values)
-      k_radix_small<true><<<1, kSmallThreads, small_smem(), st>>>(keys, vals, n, passes);
-    else
-      k_radix_small<false><<<1, kSmallThreads, small_smem(), st>>>(keys, vals, n, passes);
-    return cudaGetLastError();
+  if (n <= small_max()) {
+    const SmallForm* f = kSmallForms;
+    while (n > f->max) ++f;
+    void* args[] = {&keys, &vals, &n, &passes};
+    return cudaLaunchKernel(iota_values ? f->iota : f->given, dim3(f->ctas), dim3(kSmallThreads), args, f->smem, st);
   }
   uint32_t *ki = keys, *vi = vals, *ko = keys_alt, *vo = vals_alt;
   for (int p = 0; p < passes; ++p) {
@@ -425,7 +533,7 @@ cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt,
 }
 
 int radix_launches(uint32_t n, int key_bits) {
-  if (n <= kSmallMax) return 1;
+  if (n <= small_max()) return 1;
   int passes = (key_bits + kRadixBits - 1) / kRadixBits;
   if (passes < 1) passes = 1;
   return 3 * passes;
