@@ -1222,13 +1222,15 @@ def run_ours(args, rank, world, local_rank):
     if rank != 0:
         s.close()
         return
-    launches_base = 1 + 1 + 1 + 3 * RADIX_PASSES + 1 + 1  # step init, nlist, forces, sort, reorder, cells
+    # sort (one launch up to 32,768 keys), reorder with cell tables and the step's initial state, lists (with the
+    # density in WCSPH), forces
+    launches_base = (1 if nd <= 32768 else 3 * RADIX_PASSES) + 1 + 1 + 1
     if method == "pcisph":
         rigid = (1 + 2 + 1) if sc.num_bodies else 0  # slots, reduce + integrate, sync
         staged = 1 if 2 in (tuned.get("density_mode"), tuned.get("pforce_mode")) else 0  # k_stage_lists
-        gpu_launches = args.steps * (launches_base + 2 + rigid + staged) + 3 * total_iters
+        gpu_launches = args.steps * (launches_base + 1 + rigid + staged) + 3 * total_iters  # integrate; loop passes
     else:
-        gpu_launches = args.steps * (launches_base + 1)
+        gpu_launches = args.steps * launches_base
     out = {
         "metric": metric_for(args), "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": max_ms / args.steps, "higher_is_better": True,

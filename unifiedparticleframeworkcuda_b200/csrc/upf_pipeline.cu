@@ -1,15 +1,17 @@
 // upf_pipeline.cu — the per-step kernels.
 //
-// Step = sort (Morton keys -> radix sort -> reorder -> cell ranges)
-//      -> neighbour lists
-//      -> WCSPH: density/pressure, then force + integration
+// Step = sort (Morton keys -> radix sort -> reorder with cell ranges)
+//      -> neighbour lists (WCSPH: with density and pressure)
+//      -> WCSPH: force + integration
 //         PCISPH: external forces, then the predict-correct loop
 //                 (predicted density + pressure update, pressure force +
-//                 next prediction, loop control), then integration.
-// Every kernel is one thread per particle over the sorted working set; the
-// neighbour loops read the column-major lists, so a warp's list reads are
-// coalesced and its position gathers hit the Morton-ordered neighbourhood in
-// L1/L2.
+//                 next prediction, loop control; one launch for all
+//                 iterations where the SMs hold every particle), then
+//                 integration.
+// A kernel is one thread, or a few lanes, per particle over the sorted working
+// set (the list build: one warp per 4 to 32 particles); the neighbour loops
+// read the column-major lists, so a warp's list reads are coalesced and its
+// position gathers hit the Morton-ordered neighbourhood in L1/L2.
 //
 // Reference kernels replaced (src/gpu/particles_kernel.cu):
 //   FillZindicesKernel 3360, CopySortedParticleValuesKernel* 543-654,
