@@ -672,8 +672,7 @@ def run_batch(args, rank, world, local_rank):
     seq_value = ns * args.steps * world / (seq_ms / 1e3)
     if rank != 0:
         return
-    radix = lambda bits: 3 * ((bits + 7) // 8)  # noqa: E731
-    per_step = radix(31) + 1 + radix(8) + 1 + 1 + 1 + 1 + 1 + 1 + 1  # sort, digits, reorder, cells, inits, nlist, ext, integrate
+    per_step = 1 + 1 + 1 + 1 + 1 + 1 + 1 + 1  # sort, reorder, cells, init, nlist, ext, loop init, integrate
     max_it = max(st.total_iterations for st in stats)
     out = {
         "metric": "batched scene-steps/s (256 PCISPH scenes, 2k-65k particles) vs sequential single-scene steps",

@@ -228,11 +228,13 @@ upf_status upf_batch_create(const upf_params* params, const uint32_t* counts, ui
   b->seg_begin.resize(num_scenes);
   b->seg_end.resize(num_scenes);
   b->cell_base.resize(num_scenes);
+  std::vector<uint2> segments(num_scenes);
   uint32_t off = 0, cb = 0, comp = 0, rows = 0;
   for (uint32_t s = 0; s < num_scenes; ++s) {
     const uint32_t padded = round_up(counts[s] ? counts[s] : 1, kSegAlign);
     b->seg_begin[s] = off;
     b->seg_end[s] = off + counts[s];
+    segments[s] = make_uint2(off, padded);
     for (uint32_t g = off / kSegAlign; g < (off + padded) / kSegAlign; ++g) group_scene[g] = s;
     off += padded;
     b->cell_base[s] = cb;
@@ -243,6 +245,8 @@ upf_status upf_batch_create(const upf_params* params, const uint32_t* counts, ui
     rows = std::max(rows, params[s].max_neighbors);
   }
   b->list_rows = rows;
+  std::stable_sort(segments.begin(), segments.end(), [](uint2 x, uint2 y) { return x.y > y.y; });
+  const bool by_segment = num_scenes && radix_segments_fit(segments[0].y);
   int bits = 1;
   while ((1u << bits) < num_scenes) ++bits;
   b->scene_bits = bits;
@@ -258,8 +262,12 @@ upf_status upf_batch_create(const upf_params* params, const uint32_t* counts, ui
   if ((st = balloc(*b, &(ptr), (cnt))) != UPF_OK) return bail(st);
   ALLOC(b->A.pos, n); ALLOC(b->A.vel, n); ALLOC(b->A.lag, n); ALLOC(b->A.id, n); ALLOC(b->A.type, n);
   ALLOC(b->B.pos, n); ALLOC(b->B.vel, n); ALLOC(b->B.lag, n); ALLOC(b->B.id, n); ALLOC(b->B.type, n);
-  ALLOC(b->keysA, n); ALLOC(b->perm, n); ALLOC(b->digits, n);
-  ALLOC(b->sort_tmp, radix_temp_words((uint32_t)n));
+  ALLOC(b->keysA, n); ALLOC(b->perm, n);
+  if (by_segment) {
+    ALLOC(b->segments_d, num_scenes);
+  } else {
+    ALLOC(b->digits, n); ALLOC(b->sort_tmp, radix_temp_words((uint32_t)n));
+  }
   ALLOC(b->force, n); ALLOC(b->pforce, n); ALLOC(b->xs, n);
   ALLOC(b->rho, n); ALLOC(b->press, n); ALLOC(b->pq, n);
   ALLOC(b->nbr, n * rows); ALLOC(b->lval, n * ((rows + 3) & ~3u)); ALLOC(b->ncnt, n);
@@ -294,6 +302,8 @@ upf_status upf_batch_create(const upf_params* params, const uint32_t* counts, ui
   if (e == cudaSuccess)
     e = cudaMemcpy(b->group_scene_d, group_scene.data(), sizeof(uint32_t) * group_scene.size(),
                    cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && by_segment)
+    e = cudaMemcpy(b->segments_d, segments.data(), sizeof(uint2) * num_scenes, cudaMemcpyHostToDevice);
   if (e == cudaSuccess)
     e = cudaMemcpy(b->seg_begin_d, b->seg_begin.data(), sizeof(uint32_t) * num_scenes, cudaMemcpyHostToDevice);
   if (e == cudaSuccess)
@@ -744,7 +754,10 @@ upf_status upf_batch_profile_step(upf_batch* b, upf_phase_times* out, uint64_t* 
   out->sort_ms = elapsed(ev[0], ev[1]);
   out->neighbors_ms = elapsed(ev[1], ev[2]);
   out->forces_ms = elapsed(ev[2], ev[3]);
-  int launches = 4 + 1 + 4 + 1 + 1 + 2 + 1 + 1 + 1;  // sort stages, digits, reorder, cells, init, nlist, ext, loop init
+  const int sort = b->segments_d ? 1
+                                 : radix_launches(b->n_slots, 31) + 1 /*scene digits*/ +
+                                       radix_launches(b->n_slots, b->scene_bits);
+  int launches = sort + 1 + 1 + 1 + 1 + 1 + 1;  // reorder, cells, init, nlist, ext, loop init
   float loop = 0;
   const uint32_t total_groups = b->n_slots / kSegAlign;
   for (int it = 0; it < 4096; ++it) {

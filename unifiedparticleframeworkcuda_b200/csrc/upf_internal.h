@@ -63,6 +63,12 @@ cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt,
                              uint32_t* counts, uint32_t n, int key_bits, bool iota_values,
                              cudaStream_t st);
 int radix_launches(uint32_t n, int key_bits);
+// Stable sort of each segment (first, count; none empty) of one array by its
+// 32-bit keys, one launch; whether segments of up to `longest` keys can be.
+constexpr uint32_t kRadixSegmentMax = 65536;
+cudaError_t radix_sort_segments(const uint2* segments, uint32_t count, const uint32_t* keys, uint32_t* perm,
+                                cudaStream_t st);
+bool radix_segments_fit(uint32_t longest);
 cudaError_t radix_init();
 cudaError_t morton_keys(const float4* pos, uint32_t n, float3 origin, float3 scales, uint32_t* keys,
                         cudaStream_t st);

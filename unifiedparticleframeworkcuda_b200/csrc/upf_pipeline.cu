@@ -3027,15 +3027,20 @@ cudaError_t batch_launch_keys(BatchSystem& b, cudaStream_t st) {
 cudaError_t batch_launch_sort(BatchSystem& b, cudaStream_t st) {
   const uint32_t n = b.n_slots;
   if (!n) return cudaSuccess;
-  uint32_t* kalt = b.sort_tmp;
-  uint32_t* valt = kalt + ((n + 63) & ~63u);
-  uint32_t* counts = valt + ((n + 63) & ~63u);
-  cudaError_t e = radix_sort_pairs(b.keysA, b.perm, kalt, valt, counts, n, 31, true, st);
-  if (e != cudaSuccess) return e;
-  k_scene_digits<<<grid_of(n), kBlock, 0, st>>>(n, b.perm, b.group_scene_d, b.digits);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  e = radix_sort_pairs(b.digits, b.perm, kalt, valt, counts, n, b.scene_bits, false, st);
-  if (e != cudaSuccess) return e;
+  cudaError_t e;
+  if (b.segments_d) {
+    if ((e = radix_sort_segments(b.segments_d, b.n_scenes, b.keysA, b.perm, st)) != cudaSuccess) return e;
+  } else {
+    uint32_t* kalt = b.sort_tmp;
+    uint32_t* valt = kalt + ((n + 63) & ~63u);
+    uint32_t* counts = valt + ((n + 63) & ~63u);
+    e = radix_sort_pairs(b.keysA, b.perm, kalt, valt, counts, n, 31, true, st);
+    if (e != cudaSuccess) return e;
+    k_scene_digits<<<grid_of(n), kBlock, 0, st>>>(n, b.perm, b.group_scene_d, b.digits);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    e = radix_sort_pairs(b.digits, b.perm, kalt, valt, counts, n, b.scene_bits, false, st);
+    if (e != cudaSuccess) return e;
+  }
   k_reorder_batch<<<grid_of(n), kBlock, 0, st>>>(b.view, n, b.perm, b.A, b.B, b.keysA);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if ((e = cudaMemsetAsync(b.cstart, 0, sizeof(uint32_t) * b.n_cells, st)) != cudaSuccess) return e;

@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(kThreads) k_downsweep(const uint32_t* __restri
   constexpr int kTile = kWarps * kWarpItems;
   extern __shared__ uint32_t smem[];
   uint32_t* whist = smem;                                  // [kWarps][kRadix]
-  uint32_t* skeys = whist + kWarps * kRadix;               // [kTile]
+  uint32_t* skeys = whist + kWarps * kRadix;               // [kItems * 512]
   uint32_t* svals = skeys + kTile;                         // [kTile]
   uint32_t* digit_off = svals + kTile;                     // [kRadix] tile-local digit offsets
   uint32_t* gbase = digit_off + kRadix;                    // [kRadix] global bases
@@ -255,32 +255,31 @@ __global__ void __launch_bounds__(kThreads) k_downsweep(const uint32_t* __restri
 constexpr int kSmallThreads = 512;
 constexpr int kSmallWarps = kSmallThreads / 32;
 constexpr int kSmallGroups = kSmallThreads / kRadix;  // of eight warps
+constexpr int kSegmentCtas = 8, kSegmentItems = 16;
+static_assert(kSegmentCtas * kSegmentItems * kSmallThreads == kRadixSegmentMax, "segments");
 
 template <int kItems>
-constexpr size_t small_smem() {
+constexpr size_t cluster_smem() {
   return sizeof(uint2) * kSmallThreads * kItems +
          sizeof(uint32_t) * (kSmallWarps * kRadix + kRadix + 2 * kSmallGroups * kRadix);
 }
 
-// All passes in one launch of one cluster of kCtas CTAs (one CTA: no cluster),
-// each of which holds kItems * 512 consecutive pairs of the current order in
-// registers. A pass ranks them as k_downsweep does, adds the digit counts of
-// all CTAs (read from their shared memory) to the places of its own, and sends
-// every pair to the shared memory of the CTA that holds its place.
-// Bound by the ranking (0.6 us a round of 16 warps, some 70 instructions a
-// warp) and the barriers (0.3 us each across a cluster). Four passes, us, in
-// one launch and in twelve: 900 pairs 5.5 and 25, 1,728 8.3, 4,096 11.3, 8,192
-// 11.8, 16,384 16.6 and 25.2, 32,768 on 16 CTAs 21.4 and 25.9; on 8 CTAs 26.0,
-// and 50,000 on 16 31.6 and 26.3. CTAs of 1,024 threads are 1 to 2 us longer
-// (more rows of counts to add up), pairs put in order in the CTA before they
-// are sent not shorter.
-template <bool kIotaValues, int kCtas, int kItems>
-__global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kSmallThreads)
-    k_radix_cluster(uint32_t* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t n, int passes) {
-  constexpr uint32_t kTile = kSmallThreads * kItems;
+// All passes of a sort by one cluster of kCtas CTAs (one CTA: no cluster), each
+// of which holds rounds * 512 (at most kItems * 512) consecutive pairs of the
+// current order in registers: round r of a thread is the pair at lane + 32 (r +
+// rounds * warp). A pass ranks them as k_downsweep does, adds the digit counts
+// of all CTAs (read from their shared memory) to the places of its own, and
+// sends every pair to the shared memory of the CTA that holds its place.
+// `load(i, k, v)` fetches pair i, `store(i, k, v)` takes the i-th of the order.
+template <int kCtas, int kItems, class Load, class Store>
+__device__ __forceinline__ void sort_in_cluster(uint32_t rounds, int passes, Load&& load, Store&& store) {
+  const uint32_t tile = kSmallThreads * rounds;
+  // x / rounds of x < 256, as the product with the rounded-up 16-bit inverse
+  const uint32_t inverse = (65536u + rounds - 1) / rounds;
+  static_assert(kCtas * kItems <= 256 && kItems <= 16, "inverse");
   extern __shared__ uint2 pair_mem[];
   uint2* const pairs = pair_mem;                                       // [kTile]
-  uint32_t* const whist = reinterpret_cast<uint32_t*>(pairs + kTile);  // [kSmallWarps][kRadix]
+  uint32_t* const whist = reinterpret_cast<uint32_t*>(pairs + kSmallThreads * kItems);  // [kSmallWarps][kRadix]
   uint32_t* const count = whist + kSmallWarps * kRadix;                // [kRadix] this CTA's digit counts
   uint32_t* const part = count + kRadix;                               // [kSmallGroups][kRadix] the groups' counts
   uint32_t* const base = part + kSmallGroups * kRadix;                 // [kSmallGroups][kRadix] a group's first place
@@ -295,14 +294,12 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kSmallThreads)
   const uint32_t cta = kCtas > 1 ? cluster.block_rank() : 0u;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t lt = lanemask_lt();
-  const uint32_t seg = warp * 32 * kItems + lane;
-  uint32_t k[kItems], v[kItems], local[kItems];
+  const uint32_t seg = warp * 32 * rounds + lane;
+  uint32_t k[kItems], v[kItems];
+  uint32_t local[(kItems + 1) / 2];  // 16 bits each
 #pragma unroll
-  for (int r = 0; r < kItems; ++r) {
-    const uint32_t i = cta * kTile + seg + r * 32;
-    k[r] = i < n ? keys[i] : 0xffffffffu;  // beyond the last key: behind all others in every pass
-    v[r] = i < n ? (kIotaValues ? i : vals[i]) : 0u;
-  }
+  for (int r = 0; r < kItems; ++r)
+    if ((uint32_t)r < rounds) load(cta * tile + seg + r * 32, k[r], v[r]);
   uint32_t* const wh = whist + warp * kRadix;
   for (int shift = 0; shift < passes * kRadixBits; shift += kRadixBits) {
 #pragma unroll
@@ -310,10 +307,11 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kSmallThreads)
     __syncwarp();
 #pragma unroll
     for (int r = 0; r < kItems; ++r) {
+      if ((uint32_t)r >= rounds) break;
       const uint32_t d = (k[r] >> shift) & (kRadix - 1);
       const uint32_t peers = digit_peers(d);
       const uint32_t rank = __popc(peers & lt), prior = wh[d];
-      local[r] = prior + rank;
+      local[r / 2] = r & 1 ? local[r / 2] | (prior + rank) << 16 : prior + rank;
       __syncwarp();
       if (rank == 0) wh[d] = prior + __popc(peers);
       __syncwarp();
@@ -372,27 +370,74 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kSmallThreads)
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < kItems; ++r) {
+      if ((uint32_t)r >= rounds) break;
       const uint32_t d = (k[r] >> shift) & (kRadix - 1);
-      const uint32_t at = base[(warp / 8) * kRadix + d] + wh[d] + local[r];
-      uint2* const to = kCtas > 1 ? cluster.map_shared_rank(pairs, at / kTile) : pairs;
-      to[at % kTile] = make_uint2(k[r], v[r]);
+      const uint32_t at = base[(warp / 8) * kRadix + d] + wh[d] + (local[r / 2] >> 16 * (r & 1) & 0xffffu);
+      const uint32_t owner = kCtas > 1 ? (at / kSmallThreads * inverse) >> 16 : 0u;
+      uint2* const to = kCtas > 1 ? cluster.map_shared_rank(pairs, owner) : pairs;
+      to[at - owner * tile] = make_uint2(k[r], v[r]);
     }
     barrier();
 #pragma unroll
     for (int r = 0; r < kItems; ++r) {
+      if ((uint32_t)r >= rounds) break;
       const uint2 p = pairs[seg + r * 32];
       k[r] = p.x;
       v[r] = p.y;
     }
   }
 #pragma unroll
-  for (int r = 0; r < kItems; ++r) {
-    const uint32_t i = cta * kTile + seg + r * 32;
-    if (i < n) {
-      keys[i] = k[r];
-      vals[i] = v[r];
-    }
-  }
+  for (int r = 0; r < kItems; ++r)
+    if ((uint32_t)r < rounds) store(cta * tile + seg + r * 32, k[r], v[r]);
+}
+
+// Up to kCtas * kItems * 512 pairs.
+// Bound by the ranking (0.6 us a round of 16 warps, some 70 instructions a
+// warp) and the barriers (0.3 us each across a cluster). Four passes, us, in
+// one launch and in twelve: 900 pairs 5.5 and 25, 1,728 8.3, 4,096 11.3, 8,192
+// 11.8, 16,384 16.6 and 25.2, 32,768 on 16 CTAs 21.4 and 25.9; on 8 CTAs 26.0,
+// and 50,000 on 16 31.6 and 26.3. CTAs of 1,024 threads are 1 to 2 us longer
+// (more rows of counts to add up), pairs put in order in the CTA before they
+// are sent not shorter.
+template <bool kIotaValues, int kCtas, int kItems>
+__global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kSmallThreads)
+    k_radix_cluster(uint32_t* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t n, int passes) {
+  sort_in_cluster<kCtas, kItems>(
+      kItems, passes,
+      [&](uint32_t i, uint32_t& k, uint32_t& v) {
+        k = i < n ? keys[i] : 0xffffffffu;  // beyond the last key: behind all others in every pass
+        v = i < n ? (kIotaValues ? i : vals[i]) : 0u;
+      },
+      [&](uint32_t i, uint32_t k, uint32_t v) {
+        if (i < n) {
+          keys[i] = k;
+          vals[i] = v;
+        }
+      });
+}
+
+// Segments of one array, each sorted by a cluster of its own: perm gets the
+// index (in the whole array) of each place's key; the keys stay as they are.
+// Against one sort of the whole array and a further pass by segment (24 MB of
+// keys and indices in and out five times): a batch of 256 scenes, 5.2 million
+// slots, sorted and reordered in 0.41 ms, 0.57 before; 12 scenes of 2,048 to
+// 16,384 0.039 and 0.098 (fifteen launches). One scene of 65,536 alone takes
+// 45 us either way; a longer one does not fit the cluster's registers.
+template <int kItems>
+__global__ void __cluster_dims__(kSegmentCtas, 1, 1) __launch_bounds__(kSmallThreads, 2)
+    k_radix_segments(const uint2* __restrict__ segments, const uint32_t* __restrict__ keys,
+                     uint32_t* __restrict__ perm) {
+  const uint2 seg = segments[blockIdx.x / kSegmentCtas];  // first, count
+  constexpr uint32_t round = kSegmentCtas * kSmallThreads;
+  sort_in_cluster<kSegmentCtas, kItems>(
+      (seg.y + round - 1) / round, 32 / kRadixBits,
+      [&](uint32_t i, uint32_t& k, uint32_t& v) {
+        k = i < seg.y ? keys[seg.x + i] : 0xffffffffu;
+        v = seg.x + i;
+      },
+      [&](uint32_t i, uint32_t, uint32_t v) {
+        if (i < seg.y) perm[seg.x + i] = v;
+      });
 }
 
 // The one-launch forms: the largest count of each, in order.
@@ -406,7 +451,7 @@ struct SmallForm {
 template <int kCtas, int kItems>
 constexpr SmallForm small_form() {
   return {(uint32_t)kCtas * kSmallThreads * kItems, (const void*)k_radix_cluster<true, kCtas, kItems>,
-          (const void*)k_radix_cluster<false, kCtas, kItems>, (uint32_t)kCtas, small_smem<kItems>()};
+          (const void*)k_radix_cluster<false, kCtas, kItems>, (uint32_t)kCtas, cluster_smem<kItems>()};
 }
 const SmallForm kSmallForms[] = {
     small_form<1, 2>(), small_form<1, 4>(), small_form<8, 2>(), small_form<8, 4>(), small_form<16, 4>(),};
@@ -423,6 +468,9 @@ uint32_t small_max() {
 }
 
 cudaError_t small_init(int dev) {
+  const cudaError_t e = cudaFuncSetAttribute(k_radix_segments<kSegmentItems>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)cluster_smem<kSegmentItems>());
+  if (e != cudaSuccess) return e;
   uint32_t fits = 0;
   for (const SmallForm& f : kSmallForms) {
     int clusters = 0;
@@ -531,6 +579,16 @@ cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt,
   }
   return cudaGetLastError();
 }
+
+cudaError_t radix_sort_segments(const uint2* segments, uint32_t count, const uint32_t* keys, uint32_t* perm,
+                                cudaStream_t st) {
+  if (!count) return cudaSuccess;
+  k_radix_segments<kSegmentItems><<<count * kSegmentCtas, kSmallThreads, cluster_smem<kSegmentItems>(), st>>>(
+      segments, keys, perm);
+  return cudaGetLastError();
+}
+
+bool radix_segments_fit(uint32_t longest) { return longest <= kRadixSegmentMax && small_max() >= 16384u; }
 
 int radix_launches(uint32_t n, int key_bits) {
   if (n <= small_max()) return 1;

@@ -265,6 +265,7 @@ struct BatchSystem {
   uint32_t* perm = nullptr;
   uint32_t* digits = nullptr;  // second sort stage keys (scene of each element)
   uint32_t* sort_tmp = nullptr;
+  uint2* segments_d = nullptr;  // [n_scenes] first slot and padded count, longest first; null: one is too long
   float4* force = nullptr;
   float4* pforce = nullptr;
   float4* xs = nullptr;
