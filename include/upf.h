@@ -751,9 +751,13 @@ upf_status upf_adjoint_times(upf_adjoint* a, float* forward_ms, float* backward_
  * upf_test_stage_union_cap(s, cap): lowers the number of distinct neighbours
  * a chunk of the staged loop passes (mode 2) may stage (at most 2048, the
  * default); chunks whose union is larger read the plain lists. For reaching
- * that fallback on small scenes. */
+ * that fallback on small scenes.
+ * upf_test_fill_list_values(s, byte): every byte of a PCISPH system's list
+ * values, the rows past max_neighbors included, set to `byte` (0xff: NaN);
+ * what a step leaves of them must not reach its results. */
 upf_status upf_test_fail_allocation(int32_t nth);
 upf_status upf_test_stage_union_cap(upf_system* s, uint32_t cap);
+upf_status upf_test_fill_list_values(upf_system* s, uint32_t byte);
 upf_status upf_selftest_bounded_wait(int device, uint32_t limit_us);
 upf_status upf_selftest_support_bins(int device, const upf_params* p, const float* r2, uint32_t n, int32_t* bins);
 

@@ -693,6 +693,17 @@ upf_status upf_test_stage_union_cap(upf_system* s, uint32_t cap) {
   return s->have_particles ? build_step_graph(*s) : UPF_OK;
 }
 
+upf_status upf_test_fill_list_values(upf_system* s, uint32_t byte) {
+  if (!s || byte > 255 || s->prm.method != UPF_METHOD_PCISPH) {
+    set_error("upf_test_fill_list_values: a PCISPH system and a byte");
+    return UPF_ERR_INVALID_ARG;
+  }
+  UPF_CUDA(cudaMemsetAsync(s->lval, (int)byte, sizeof(uint32_t) * s->nstride * list_value_rows(s->prm.max_neighbors),
+                           s->stream));
+  UPF_CUDA(cudaStreamSynchronize(s->stream));
+  return UPF_OK;
+}
+
 upf_status upf_test_fail_allocation(int32_t nth) {
   g_fail_alloc_at.store(nth < 0 ? -1 : (int64_t)nth);
   return UPF_OK;
@@ -875,7 +886,7 @@ upf_status upf_create(const upf_params* p, int device, uint32_t capacity, upf_sy
   ALLOC(s->force, c); ALLOC(s->pforce, c); ALLOC(s->xs, ct);
   ALLOC(s->rho, ct); ALLOC(s->press, ct); ALLOC(s->pq, ct); ALLOC(s->wvol, ct);
   ALLOC(s->nbr, (size_t)s->nstride * p->max_neighbors);
-  ALLOC(s->lval, (size_t)s->nstride * ((p->max_neighbors + 3) & ~3u));
+  ALLOC(s->lval, s->nstride * list_value_rows(p->max_neighbors));
   ALLOC(s->ncnt, c);
   ALLOC(s->cells, (size_t)4 * s->ncells);
   ALLOC(s->sstart, s->ncells); ALLOC(s->send, s->ncells);

@@ -270,7 +270,7 @@ upf_status upf_batch_create(const upf_params* params, const uint32_t* counts, ui
   }
   ALLOC(b->force, n); ALLOC(b->pforce, n); ALLOC(b->xs, n);
   ALLOC(b->rho, n); ALLOC(b->press, n); ALLOC(b->pq, n);
-  ALLOC(b->nbr, n * rows); ALLOC(b->lval, n * ((rows + 3) & ~3u)); ALLOC(b->ncnt, n);
+  ALLOC(b->nbr, n * rows); ALLOC(b->lval, n * list_value_rows(rows)); ALLOC(b->ncnt, n);
   ALLOC(b->cstart, b->n_cells); ALLOC(b->cend, b->n_cells);
   ALLOC(b->params_d, num_scenes); ALLOC(b->luts_d, (size_t)num_scenes * kLutFloats);
   ALLOC(b->st_d, num_scenes);

@@ -577,10 +577,10 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_build_nlist(
         }
         ++cnt_mine;
       }
-      // zeros up to a whole batch of four (the value rows are allocated so):
-      // the staged pressure-force pass takes whole batches
-      if (lval && cnt_mine < maxn)
-        for (uint32_t z = cnt_mine; z & 3u; ++z) ov[(size_t)z * stride] = 0u;
+      // zeros up to a whole batch of four (list_value_rows), behind a full
+      // list too: the staged pressure-force pass takes whole batches
+      if (lval)
+        for (uint32_t z = min(cnt_mine, maxn); z & 3u; ++z) ov[(size_t)z * stride] = 0u;
       words = 0;
     }
     __syncwarp();

@@ -96,6 +96,9 @@ constexpr uint32_t kUnionMax = 2048;
 constexpr uint32_t kUnionEmpty = kUnionMax - 1;  // position of no neighbour: fills a list's last word
 constexpr uint32_t kUnionOverflow = 0xffffffffu;
 constexpr bool loop_mode_staged(int mode) { return mode == 2; }
+// Rows of the list values: whole batches of four, as the staged
+// pressure-force pass takes them (k_build_nlist zeroes what lies past a list).
+constexpr size_t list_value_rows(uint32_t max_neighbors) { return ((size_t)max_neighbors + 3) & ~(size_t)3; }
 
 constexpr int kListRowVariants = 4;  // tensor maps for 2, 4, 8 and 16 rows per box
 inline int rows_index(int rows) { return rows == 2 ? 0 : (rows == 4 ? 1 : (rows == 8 ? 2 : 3)); }
