@@ -1,11 +1,11 @@
 """The staged loop passes take a list's entries in whole batches: what lies
 past a list's end must not reach the sums, also where a list is full and its
-capacity no multiple of a batch. Each case bit for bit against passes that
+capacity no multiple of a batch, or where a pressure is not finite. Each case bit for bit against passes that
 stop at the list's end."""
 import numpy as np
 import pytest
 
-from unifiedparticleframeworkcuda_b200 import scenes
+from unifiedparticleframeworkcuda_b200 import LIQUID, scenes
 
 pytestmark = pytest.mark.gpu
 
@@ -55,3 +55,26 @@ def test_lists_filled_to_a_capacity_that_is_no_multiple_of_four(upf_lib, block, 
         assert got[1] == want[1], shape
         for k in FIELDS:
             assert np.array_equal(got[0][k], want[0][k]), (shape, k)
+
+
+@pytest.mark.parametrize("rows", [4, 8])
+def test_a_pressure_that_is_not_finite(upf_lib, rows):
+    """Two particles whose correction pressure overflows: each is thrown
+    against the walls by the infinite force of its one neighbour, and the
+    batch's three other entries add nothing to it."""
+    sc = scenes.small_pcisph()
+    sc.params.flags = 0
+    p = upf_lib.derive_params(sc.params)
+    p.mass *= 4.0
+    p.density_error_factor = 1e38
+    mid = 0.5 * (np.array(p.collision_min[:]) + np.array(p.collision_max[:]))
+    pos = np.zeros((2, 4), np.float32)
+    pos[0, :3] = mid - 0.002
+    pos[1, :3] = mid + 0.002
+    vel, typ = np.zeros_like(pos), np.full(2, LIQUID, np.int32)
+    want = one_step(upf_lib, p, pos, vel, typ, (0, 128, 4))
+    assert np.isinf(want[0]["pressure"]).all() and np.isfinite(want[0]["pos"]).all()
+    got = one_step(upf_lib, p, pos, vel, typ, (2, 256, rows))
+    assert got[1] == want[1]
+    for k in FIELDS:
+        assert np.array_equal(got[0][k], want[0][k]), k

@@ -1853,11 +1853,13 @@ __global__ void __launch_bounds__(kStageChunk, pforce_staged_min_blocks(kRows)) 
     fy = fy - ky * grad * m * m;
     fz = fz - kz * grad * m * m;
   };
-  if (staged) {
-    // whole batches of four: past the list's end the value is 0 and the
-    // neighbour the empty position, and taking off a zero changes no sum (a
-    // batch's second word may lie past the list altogether). The next batch's
-    // values are loaded with its words, before this batch's arithmetic.
+  // whole batches of four: past the list's end the value is 0 and the
+  // neighbour the empty position, and taking off a zero changes no sum (a
+  // batch's second word may lie past the list altogether). That holds for a
+  // finite p / rho0^2 only (0 * inf is NaN): a particle whose pressure has
+  // overflowed walks its plain list, entry by entry. The next batch's values
+  // are loaded with its words, before this batch's arithmetic.
+  if (staged && isfinite(qi)) {
     const float* __restrict__ vc = reinterpret_cast<const float*>(vcol);
     const size_t row = P.nstride;
     float gn[kRows];
