@@ -169,14 +169,21 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));  // within 2 ulp
   return r;
 }
+__device__ __forceinline__ float fmul_ftz(float a, float b) {  // subnormals taken as zero
+  float r;
+  asm("mul.rn.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
 struct BinGuess {
   int bin;
   bool sure;
 };
 __device__ __forceinline__ BinGuess bin_guess(float r2, float factor) {
-  // (a subnormal r2 flushes to 0 in the root: x is then NaN or infinite; the
-  // minimum keeps a NaN, and both leave the guess unsure or at 300)
-  const float y = __fmaf_rn(fmul(r2, rsqrt_approx(r2)), fmul(factor, (float)kLut), -0.5f);
+  // (zero, and a subnormal r2, which both operations flush to zero: 0 times
+  // an infinite root is NaN, the minimum keeps it, and the guess is unsure.
+  // Not flushed in the product, a subnormal r2 would give infinity, taken for
+  // bin 300.)
+  const float y = __fmaf_rn(fmul_ftz(r2, rsqrt_approx(r2)), fmul(factor, (float)kLut), -0.5f);
   float yc;
   asm("min.NaN.f32 %0, %1, %2;" : "=f"(yc) : "f"(y), "f"((float)kLut));
   const float t = fadd(yc, 12582912.0f);
