@@ -723,10 +723,13 @@ upf_status upf_adjoint_destroy(upf_adjoint* a);
 upf_status upf_adjoint_set_stream(upf_adjoint* a, void* stream);
 /* Runs the T steps from the initial positions with initial velocities vel4
  * (n x 4 host floats; NULL keeps the last ones) and the given viscosity;
- * *loss (may be NULL) receives L. */
+ * *loss (may be NULL) receives L. A call that fails leaves no trajectory:
+ * until one succeeds, upf_adjoint_backward and upf_adjoint_get_state return
+ * UPF_ERR_STATE. */
 upf_status upf_adjoint_forward(upf_adjoint* a, const float* vel4, float viscosity, double* loss);
 /* Gradients of the last forward's loss: grad_vel4 (n x 4 host floats, w = 0)
- * and *grad_viscosity (either may be NULL). */
+ * and *grad_viscosity (either may be NULL). May be called again after the
+ * same forward. */
 upf_status upf_adjoint_backward(upf_adjoint* a, float* grad_vel4, double* grad_viscosity);
 /* Final positions and velocities of the last forward (n x 4 host floats). */
 upf_status upf_adjoint_get_state(upf_adjoint* a, float* pos4, float* vel4);

@@ -565,7 +565,8 @@ struct upf_adjoint {
   // graphs, captured on first use: one forward step in slot 0, and a whole
   // checkpoint interval (its forward steps, then its adjoint steps)
   cudaGraphExec_t step_exec = nullptr, interval_exec = nullptr;
-  bool have_forward = false;
+  bool have_forward = false;   // the last forward succeeded
+  bool final_in_slot0 = false;  // slot 0 holds the final state's lists and densities (else a replayed step's)
   float fwd_ms = 0.0f, bwd_ms = 0.0f;
 
   // id-order state
@@ -588,7 +589,7 @@ struct upf_adjoint {
   // backward scratch (sorted order)
   float4 *xb = nullptr, *vb = nullptr, *Fb = nullptr, *Fpb = nullptr;
   float* pcarry = nullptr;
-  double* sums = nullptr;  // [4] loss sums, [4] mu_bar
+  double* sums = nullptr;  // [4] loss sums, mu_bar, -, -, -, [4] the sums of a repeated loss pass
   double loss = 0.0;
   std::vector<void*> allocations;
 
@@ -685,6 +686,15 @@ struct upf_adjoint {
     }
     const float vol2 = dp.rest_volume * dp.rest_volume;
     k_ab_external<<<g, t, 0, q>>>(n, k, vol2, visc_d, X, V, Fb, L, xb, vb, pm, xbar, vbar, sums + 4);
+    UPF_CUDA(cudaGetLastError());
+    return UPF_OK;
+  }
+
+  // lists and densities of the state (x, v) in slot 0, and the loss's sums
+  upf_status loss_pass(double* into) {
+    UPF_TRY(prepare_step(0));
+    UPF_CUDA(cudaMemsetAsync(into, 0, sizeof(double) * 4, stream));
+    k_af_loss<<<grid(n), kT, 0, stream>>>(n, k, dp.mass, dp.rho0, xs, lists(0), rho, into);
     UPF_CUDA(cudaGetLastError());
     return UPF_OK;
   }
@@ -830,7 +840,7 @@ upf_status upf_adjoint_create(const upf_params* p, const upf_adjoint_options* op
   ALLOC(a->xstar, (size_t)C * K * N); ALLOC(a->rho, (size_t)C * K * N); ALLOC(a->p, (size_t)C * K * N);
   ALLOC(a->pair_g, (size_t)a->rows * a->stride); ALLOC(a->pair_t, (size_t)a->rows * a->stride); ALLOC(a->xq, N);
   ALLOC(a->xb, N); ALLOC(a->vb, N); ALLOC(a->Fb, N); ALLOC(a->Fpb, N);
-  ALLOC(a->pcarry, N); ALLOC(a->sums, 8); ALLOC(a->visc_d, 1);
+  ALLOC(a->pcarry, N); ALLOC(a->sums, 12); ALLOC(a->visc_d, 1);
 #undef ALLOC
   std::vector<float> lut(kLutFloats);
   build_luts(*p, lut.data());
@@ -888,6 +898,7 @@ upf_status upf_adjoint_forward(upf_adjoint* a, const float* vel4, float viscosit
     return UPF_ERR_INVALID_ARG;
   }
   UPF_CUDA(cudaSetDevice(a->device));
+  a->have_forward = a->final_in_slot0 = false;
   cudaStream_t q = a->stream;
   const uint32_t n = a->n;
   if (vel4) {
@@ -921,10 +932,7 @@ upf_status upf_adjoint_forward(upf_adjoint* a, const float* vel4, float viscosit
   UPF_CUDA(cudaMemcpyAsync(a->xf, a->x, sizeof(float4) * n, cudaMemcpyDeviceToDevice, q));
   UPF_CUDA(cudaMemcpyAsync(a->vf, a->v, sizeof(float4) * n, cudaMemcpyDeviceToDevice, q));
   // loss at the final positions (lists in slot 0)
-  UPF_TRY(a->prepare_step(0));
-  UPF_CUDA(cudaMemsetAsync(a->sums, 0, sizeof(double) * 8, q));
-  k_af_loss<<<grid(n), kT, 0, q>>>(n, a->k, a->dp.mass, a->dp.rho0, a->xs, a->lists(0), a->rho, a->sums);
-  UPF_CUDA(cudaGetLastError());
+  UPF_TRY(a->loss_pass(a->sums));
   UPF_CUDA(cudaEventRecord(e1, q));
   double sums[4];
   UPF_CUDA(cudaMemcpyAsync(sums, a->sums, sizeof(double) * 4, cudaMemcpyDeviceToHost, q));
@@ -940,7 +948,7 @@ upf_status upf_adjoint_forward(upf_adjoint* a, const float* vel4, float viscosit
   }
   L += a->opt.density_weight * sums[3] / n;
   a->loss = L;
-  a->have_forward = true;
+  a->have_forward = a->final_in_slot0 = true;
   if (loss) *loss = L;
   return UPF_OK;
 }
@@ -958,7 +966,16 @@ upf_status upf_adjoint_backward(upf_adjoint* a, float* grad_vel4, double* grad_v
   UPF_CUDA(cudaEventCreate(&e0));
   UPF_CUDA(cudaEventCreate(&e1));
   UPF_CUDA(cudaEventRecord(e0, q));
-  // seeds: the final state's lists and densities are in slot 0 (forward)
+  // seeds: the final state's lists and densities in slot 0, as forward leaves
+  // them; the replay below takes the slot, so a further backward builds them
+  // again (the same sort, lists and sums per particle)
+  if (!a->final_in_slot0) {
+    UPF_CUDA(cudaMemcpyAsync(a->x, a->xf, sizeof(float4) * n, cudaMemcpyDeviceToDevice, q));
+    UPF_CUDA(cudaMemcpyAsync(a->v, a->vf, sizeof(float4) * n, cudaMemcpyDeviceToDevice, q));
+    a->keys_ready = false;
+    UPF_TRY(a->loss_pass(a->sums + 8));
+  }
+  a->final_in_slot0 = false;
   double sums[4];
   UPF_CUDA(cudaMemcpyAsync(sums, a->sums, sizeof(double) * 4, cudaMemcpyDeviceToHost, q));
   UPF_CUDA(cudaStreamSynchronize(q));
