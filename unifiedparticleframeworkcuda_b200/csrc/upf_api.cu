@@ -1331,6 +1331,8 @@ upf_status upf_phase_predict_correct(upf_system* s) {
 upf_status upf_phase_integrate(upf_system* s) {
   UPF_TRY(phase_guard(s));
   s->stepped = true;
+  // (density and pressure may be the caller's: upf_get_device_state)
+  if (s->prm.method == UPF_METHOD_WCSPH) UPF_CUDA(launch_wcsph_exchange(*s, s->stream));
   UPF_CUDA(launch_integrate_phase(*s, s->stream));
   return UPF_OK;
 }

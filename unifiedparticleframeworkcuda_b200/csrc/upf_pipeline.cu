@@ -322,7 +322,24 @@ __global__ void __launch_bounds__(kBlock) k_wcsph_density(DevParams P, uint32_t 
   wcsph_store(P, m4, W, i, pos[i], den);
 }
 
-// ---------------------------------------------------------------- neighbour lists
+// What the force pass gathers, from density and pressure as they are now: a
+// caller that integrates phase by phase may have replaced them.
+__global__ void __launch_bounds__(kBlock) k_wcsph_exchange(float mass, uint32_t n, const float4* __restrict__ pos,
+                                                            const WcsphOut W) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  float4 x = pos[i], v = W.vel[i];
+  x.w = 0.0f;
+  v.w = -1.0f;
+  if (W.type[i] == UPF_LIQUID) {
+    const float den = W.rho[i];
+    x.w = W.press[i] / (den * den);
+    v.w = mass / den;
+  }
+  W.xq[i] = x;
+  W.vn[i] = v;
+}
+
 // ---------------------------------------------------------------- sorted sets
 // What starts a step, where the graph's first kernel does it: the statistics
 // (k_step_init) and the loop state (k_loop_init).
@@ -2808,6 +2825,11 @@ cudaError_t launch_force_phase(System& s, cudaStream_t st) {
     return run_external<false>(s.shape, st, s.dp, BatchView{}, n, s.B, s.wvol, s.rb.id_body, s.nbr, s.ncnt, s.luts,
                                s.force, s.pforce, s.xs, s.press, s.pq, s.st);
   }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_wcsph_exchange(System& s, cudaStream_t st) {
+  if (s.n_dyn) k_wcsph_exchange<<<grid_of(s.n_dyn), kBlock, 0, st>>>(s.dp.mass, s.n_dyn, s.B.pos, wcsph_out(s));
   return cudaGetLastError();
 }
 

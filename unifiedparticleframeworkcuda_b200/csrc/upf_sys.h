@@ -413,6 +413,8 @@ cudaError_t launch_sort_phase(System& s, cudaStream_t st, bool starts_step = fal
 // in_step: the sort phase has started the step; WCSPH densities in the same launch
 cudaError_t launch_neighbor_phase(System& s, cudaStream_t st, bool in_step = false);
 cudaError_t launch_force_phase(System& s, cudaStream_t st);
+// WCSPH: what the integration gathers, from the present density and pressure
+cudaError_t launch_wcsph_exchange(System& s, cudaStream_t st);
 cudaError_t launch_loop_init(System& s, cudaStream_t st);
 cudaError_t launch_loop_body(System& s, cudaStream_t st, cudaGraphConditionalHandle h, bool use_handle);
 cudaError_t launch_loop_density(System& s, cudaStream_t st);
