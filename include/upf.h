@@ -289,10 +289,11 @@ upf_status upf_phase_loop_control(upf_system* s, int32_t* cont);
  * ids, predicted positions, correction pressure, pq4 (position, pressure /
  * rest_density^2: what the pressure-force pass gathers), predicted density.
  * Between the phases of a step the caller may replace what the next phase
- * reads: a WCSPH system's density and pressure before upf_phase_integrate.
- * predicted_pos4 and pq4 are PCISPH's;
- * in a WCSPH system they are the step's scratch, whose contents mean nothing
- * to a caller.
+ * reads: sorted positions before upf_phase_neighbors (moved by less than half
+ * a grid unit: the cells are the sort's), a WCSPH system's density and
+ * pressure before upf_phase_integrate. predicted_pos4 and pq4 are PCISPH's; in
+ * a WCSPH system they are the step's scratch, whose contents mean nothing to a
+ * caller.
  * loop_max_density_bits: the loop test's running maximum (float bits).
  * stream: the system's stream; work on these arrays belongs on it. */
 typedef struct upf_device_state {

@@ -6,7 +6,8 @@ import numpy as np
 import pytest
 import torch
 
-from unifiedparticleframeworkcuda_b200 import FLAG_SURFACE_TENSION, FLAG_WALL_WEIGHT, RIGID, UpfDeviceState, scenes
+from unifiedparticleframeworkcuda_b200 import (FLAG_SURFACE_TENSION, FLAG_WALL_WEIGHT, FROZEN, RIGID, UpfDeviceState,
+                                                scenes)
 
 pytestmark = pytest.mark.gpu
 
@@ -59,3 +60,35 @@ def test_wcsph_density_and_pressure_between_forces_and_integration(upf_lib, side
     assert not np.array_equal(plain["vel"], want["vel"])
     for k in want:
         assert np.array_equal(got[k], want[k]), k
+
+
+@pytest.mark.parametrize("scene", ["small_pcisph", "small_wcsph"])
+def test_positions_between_sort_and_lists(upf_lib, scene):
+    """Sorted positions moved by the caller: the lists are those of the moved
+    positions, with boundary particles in the scene."""
+    sc = getattr(scenes, scene)()
+    p = upf_lib.derive_params(sc.params)
+    h = np.float32(p.support_radius)
+    wall = np.flatnonzero(sc.type == FROZEN)
+    with upf_lib.ParticleSystem(p, capacity=sc.n, derive=False) as s:
+        s.set_particles(sc.pos, sc.vel, sc.type)
+        s.phase("sort")
+        s.synchronize()
+        ids = s.sorted_keys()[1]
+        a = arrays(upf_lib, s)["sorted_pos4"]
+        # under half a grid unit to either side: within the margin of the cells
+        shift = np.float32(0.05 * p.particle_spacing) * np.where(np.arange(len(ids)) % 2, 1, -1).astype(np.float32)
+        a[:, 0] += torch.as_tensor(shift, device="cuda")
+        torch.cuda.synchronize()
+        x = sc.pos[:, :3].astype(np.float32).copy()
+        x[ids] = a.cpu().numpy()[:, :3]
+        s.phase("neighbors")
+        s.synchronize()
+        counts, lists = s.neighbors()
+    every = np.concatenate([ids.astype(np.int64), wall])
+    for k in range(0, len(ids), 7):
+        i = int(ids[k])
+        d = x[i] - x[every]
+        r = np.sqrt((d[:, 0] * d[:, 0] + d[:, 1] * d[:, 1]) + d[:, 2] * d[:, 2])
+        want = np.sort(every[(r < h) & (every != i)])
+        assert np.array_equal(np.sort(lists[k, :counts[k]]).astype(np.int64), want), i

@@ -1299,6 +1299,8 @@ upf_status upf_phase_sort(upf_system* s) {
 upf_status upf_phase_neighbors(upf_system* s) {
   UPF_TRY(phase_guard(s));
   s->stepped = true;
+  // (the sorted positions may be the caller's: upf_get_device_state)
+  UPF_CUDA(launch_merged_positions(*s, s->stream));
   UPF_CUDA(launch_neighbor_phase(*s, s->stream));
   return UPF_OK;
 }

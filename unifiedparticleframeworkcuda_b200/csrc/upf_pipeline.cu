@@ -436,6 +436,19 @@ __global__ void __launch_bounds__(kBlock) k_reorder(
   if (last && (lo == no || (other[lo] >> shift) != c)) mend[c] = m + 1;
 }
 
+// The dynamic particles of the merged sequence at their present positions: a
+// caller that runs phase by phase may have moved them since the sort.
+__global__ void __launch_bounds__(kBlock) k_merged_positions(uint32_t n, uint32_t total, const float4* __restrict__ pos,
+                                                              float4* __restrict__ mpos) {
+  const uint32_t m = blockIdx.x * blockDim.x + threadIdx.x;
+  if (m >= total) return;
+  const float code = mpos[m].w;
+  const uint32_t i = __float_as_uint(code);
+  if (i >= n) return;
+  const float4 x = pos[i];
+  mpos[m] = make_float4(x.x, x.y, x.z, code);
+}
+
 // GetNeighbors (UnifiedPhysics.cpp:2242-2280) with ZIndex::BoxQuery
 // (zIndex.cpp:43-73). Candidates are the search cells (aligned Morton blocks
 // of 2^cell_shift grid units, at most the reference's block size) covering
@@ -2789,6 +2802,12 @@ static bool stages_lists(const System& s) {
   const LaunchShape sh = loop_shape(s);
   return s.ucodes && !s.loop_in_graph && (s.stage_always || loop_mode_staged(sh.density_mode) ||
                                           loop_mode_staged(sh.pforce_mode));
+}
+
+cudaError_t launch_merged_positions(System& s, cudaStream_t st) {
+  const uint32_t total = s.n_dyn + s.n_static;
+  if (s.n_dyn && s.n_static) k_merged_positions<<<grid_of(total), kBlock, 0, st>>>(s.n_dyn, total, s.B.pos, s.mpos);
+  return cudaGetLastError();
 }
 
 static WcsphOut wcsph_out(System& s) { return WcsphOut{s.B.vel, s.B.type, s.rho, s.press, s.pq, s.xs}; }

@@ -412,6 +412,8 @@ int rigid_launches_per_step(const System& s);
 cudaError_t launch_sort_phase(System& s, cudaStream_t st, bool starts_step = false);
 // in_step: the sort phase has started the step; WCSPH densities in the same launch
 cudaError_t launch_neighbor_phase(System& s, cudaStream_t st, bool in_step = false);
+// the list build's copy of the sorted positions, from the positions as they are
+cudaError_t launch_merged_positions(System& s, cudaStream_t st);
 cudaError_t launch_force_phase(System& s, cudaStream_t st);
 // WCSPH: what the integration gathers, from the present density and pressure
 cudaError_t launch_wcsph_exchange(System& s, cudaStream_t st);
