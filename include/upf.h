@@ -531,7 +531,20 @@ upf_status upf_profile_step(upf_system* s, upf_phase_times* out);
  * walks lists rewritten as 16-bit positions in that set (the rewrite runs
  * once per step, after the list build). Batches allow up to 256 threads and
  * modes 0 and 1. Shapes change timing only: every shape gives the same
- * results. */
+ * results.
+ * Until shapes are set the library chooses how a step runs its predict-correct
+ * loop: all iterations in one cooperative launch where the system has at most
+ * 1,024 dynamic particles (a batch: slots, each scene's count rounded up to
+ * 256) an SM, 151,552 on a B200; above that, a single system's passes from
+ * staged neighbourhoods (mode 2, 256 threads, 4 rows), a batch's at the shapes
+ * that upf_batch_get_launch_config reports. Any successful
+ * upf_set_launch_config is a choice, also of the values that were reported:
+ * from then on the loop's passes run as launches of their own at those shapes.
+ * upf_autotune gives the choice back: up to 1,024 particles an SM the loop is
+ * one launch again, above it the passes run at the tuned shapes. A tuned
+ * config set in another handle is a choice there, and so ends the one-launch
+ * loop of a small one (1,728 particles: 0.33 ms a step of 50 iterations in one
+ * launch, 0.89 with passes); tune each handle, or leave it as it is. */
 typedef struct upf_launch_config {
   int32_t nlist_threads;      /* 64, 128, 256 */
   int32_t external_threads;   /* 128, 256 */
@@ -541,11 +554,14 @@ typedef struct upf_launch_config {
   int32_t pforce_rows;
   int32_t density_mode;       /* list entries by 0: the TMA ring; 1: direct loads; 2: staged neighbourhoods */
   int32_t pforce_mode;
-  int32_t nlist_mode;         /* particles whose lists one warp builds: 0 by the particle count, 1 half as many */
+  int32_t nlist_mode;         /* particles whose lists one warp builds: 0 by the particle count (4 below 16,384,
+                                 up to 32), 1 half as many, at least 4 */
   float measured_ms[4];       /* autotune: per-launch ms of the chosen shapes
                                  (neighbour lists, external forces, predicted
                                  density, pressure force); 0 otherwise */
 } upf_launch_config;
+/* The shapes of the passes as launches of their own: those set or tuned, or
+ * the library's choice for the particles in hand. */
 upf_status upf_get_launch_config(upf_system* s, upf_launch_config* out);
 upf_status upf_set_launch_config(upf_system* s, const upf_launch_config* cfg);
 /* Times every shape of each tunable pass on the system's current state
@@ -763,10 +779,15 @@ upf_status upf_adjoint_times(upf_adjoint* a, float* forward_ms, float* backward_
  * that fallback on small scenes.
  * upf_test_fill_list_values(s, byte): every byte of a PCISPH system's list
  * values, the rows past max_neighbors included, set to `byte` (0xff: NaN);
- * what a step leaves of them must not reach its results. */
+ * what a step leaves of them must not reach its results.
+ * upf_test_loop_route(s, &one_launch): whether the system's steps run their
+ * predict-correct loop in one launch (1) or its passes as launches of their
+ * own (0); upf_test_batch_loop_route likewise for a batch. */
 upf_status upf_test_fail_allocation(int32_t nth);
 upf_status upf_test_stage_union_cap(upf_system* s, uint32_t cap);
 upf_status upf_test_fill_list_values(upf_system* s, uint32_t byte);
+upf_status upf_test_loop_route(upf_system* s, int32_t* one_launch);
+upf_status upf_test_batch_loop_route(upf_batch* b, int32_t* one_launch);
 upf_status upf_selftest_bounded_wait(int device, uint32_t limit_us);
 upf_status upf_selftest_support_bins(int device, const upf_params* p, const float* r2, uint32_t n, int32_t* bins);
 

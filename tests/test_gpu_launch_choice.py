@@ -1,0 +1,95 @@
+"""Which launches a step's predict-correct loop takes: the library's choice
+while nothing is set, the caller's shapes from the first that is set, whatever
+they are and whatever was set before, and the library's again after tuning."""
+import ctypes as C
+
+import pytest
+
+from unifiedparticleframeworkcuda_b200 import UpfLaunchConfig, scenes
+
+pytestmark = pytest.mark.gpu
+
+PASSES, ONE_LAUNCH = 0, 1
+
+
+def route(upf, handle):
+    r = C.c_int32(-1)
+    batch = isinstance(handle, upf.ParticleBatch)
+    f = upf.lib().upf_test_batch_loop_route if batch else upf.lib().upf_test_loop_route
+    upf.check(f(handle.handle, C.byref(r)), "loop_route")
+    return r.value
+
+
+def loop_of(cfg):
+    return (cfg.density_mode, cfg.density_threads, cfg.density_rows, cfg.pforce_mode, cfg.pforce_threads,
+            cfg.pforce_rows)
+
+
+def with_loop(cfg, loop):
+    c = UpfLaunchConfig.from_buffer_copy(cfg)
+    (c.density_mode, c.density_threads, c.density_rows, c.pforce_mode, c.pforce_threads, c.pforce_rows) = loop
+    return c
+
+
+def system(upf, sc):
+    s = upf.ParticleSystem(upf.derive_params(sc.params), capacity=sc.n, derive=False)
+    s.set_particles(sc.pos, sc.vel, sc.type)
+    return s
+
+
+OTHER = (0, 128, 4, 0, 128, 4)
+
+
+@pytest.mark.parametrize("first", [None, OTHER])
+def test_small_system(upf_lib, first):
+    with system(upf_lib, scenes.small_pcisph()) as s:
+        assert route(upf_lib, s) == ONE_LAUNCH
+        stored = s.launch_config()
+        if first:
+            s.set_launch_config(with_loop(stored, first))
+            assert route(upf_lib, s) == PASSES and loop_of(s.launch_config()) == first
+        # the shapes that were stored from the beginning are a choice as well
+        s.set_launch_config(stored)
+        assert route(upf_lib, s) == PASSES and loop_of(s.launch_config()) == loop_of(stored)
+        s.step(1)
+        s.autotune(1)
+        assert route(upf_lib, s) == ONE_LAUNCH
+        s.step(1)
+        s.synchronize()
+
+
+def test_large_system_reports_and_honours_its_shapes(upf_lib):
+    s = 0.01
+    nx, ny, nz = 60, 54, 48
+    sc = scenes.pcisph_dam(nx, ny, nz, seed=3, box=(s * (nx + 8), s * (ny + 4), s * (nz + 6)), spacing=s)
+    with system(upf_lib, scenes.small_pcisph()) as small:
+        stored = loop_of(small.launch_config())
+    staged = (2, 256, 4, 2, 256, 4)
+    with system(upf_lib, sc) as big:
+        assert loop_of(big.launch_config()) == staged  # what its untuned steps run
+        for loop in (stored, OTHER, stored, staged):
+            big.set_launch_config(with_loop(big.launch_config(), loop))
+            assert loop_of(big.launch_config()) == loop
+            assert route(upf_lib, big) == PASSES
+            big.step(1)
+            big.synchronize()
+        tuned = big.autotune(1)
+        assert loop_of(big.launch_config()) == loop_of(tuned)
+
+
+def test_batch(upf_lib):
+    scs = scenes.batch_scenes(num=3, seed=13, counts=(2048, 4096))
+    with upf_lib.ParticleBatch.from_scenes(scs) as b:
+        assert route(upf_lib, b) == ONE_LAUNCH
+        stored = b.launch_config()
+        b.set_launch_config(stored)
+        assert route(upf_lib, b) == PASSES
+        b.step(1)
+        b.autotune(1)
+        assert route(upf_lib, b) == ONE_LAUNCH
+        b.set_launch_config(with_loop(stored, OTHER))
+        assert route(upf_lib, b) == PASSES
+        b.autotune(1)
+        assert route(upf_lib, b) == ONE_LAUNCH
+        b.step(1)
+        b.synchronize()

@@ -248,12 +248,6 @@ LaunchShape config_to_shape(const upf_launch_config& c) {
   return s;
 }
 
-bool same_loop_shapes(const LaunchShape& a, const LaunchShape& b) {
-  return a.density_mode == b.density_mode && a.density_threads == b.density_threads &&
-         a.density_rows == b.density_rows && a.pforce_mode == b.pforce_mode &&
-         a.pforce_threads == b.pforce_threads && a.pforce_rows == b.pforce_rows;
-}
-
 upf_status autotune_shapes(const TuneOps& ops, int repeats, upf_launch_config* out) {
   if (repeats < 1) repeats = 1;
   cudaStream_t st = ops.stream;
@@ -701,6 +695,15 @@ upf_status upf_test_fill_list_values(upf_system* s, uint32_t byte) {
   UPF_CUDA(cudaMemsetAsync(s->lval, (int)byte, sizeof(uint32_t) * s->nstride * list_value_rows(s->prm.max_neighbors),
                            s->stream));
   UPF_CUDA(cudaStreamSynchronize(s->stream));
+  return UPF_OK;
+}
+
+upf_status upf_test_loop_route(upf_system* s, int32_t* one_launch) {
+  if (!s || !one_launch) {
+    set_error("upf_test_loop_route: null");
+    return UPF_ERR_INVALID_ARG;
+  }
+  *one_launch = loop_fused(*s);
   return UPF_OK;
 }
 
@@ -1596,7 +1599,7 @@ upf_status upf_get_launch_config(upf_system* s, upf_launch_config* out) {
     set_error("upf_get_launch_config: null");
     return UPF_ERR_INVALID_ARG;
   }
-  shape_to_config(s->shape, out);
+  shape_to_config(loop_shape(*s), out);
   return UPF_OK;
 }
 
@@ -1612,8 +1615,7 @@ upf_status upf_set_launch_config(upf_system* s, const upf_launch_config* cfg) {
     return UPF_ERR_INVALID_ARG;
   }
   UPF_CUDA(cudaStreamSynchronize(s->stream));
-  // (the shapes in use, given back unchanged, are no choice)
-  s->shape_set = s->shape_set || !same_loop_shapes(s->shape, sh);
+  s->shape_set = true;
   s->shape = sh;
   return s->have_particles ? build_step_graph(*s) : UPF_OK;
 }

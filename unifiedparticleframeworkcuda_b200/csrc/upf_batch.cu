@@ -646,6 +646,15 @@ upf_status upf_batch_wait_frames(upf_batch* b) {
   return UPF_OK;
 }
 
+upf_status upf_test_batch_loop_route(upf_batch* b, int32_t* one_launch) {
+  if (!b || !one_launch) {
+    set_error("upf_test_batch_loop_route: null");
+    return UPF_ERR_INVALID_ARG;
+  }
+  *one_launch = batch_loop_fused(*b);
+  return UPF_OK;
+}
+
 upf_status upf_batch_get_launch_config(upf_batch* b, upf_launch_config* out) {
   if (!b || !out) {
     set_error("upf_batch_get_launch_config: null");
@@ -667,7 +676,7 @@ upf_status upf_batch_set_launch_config(upf_batch* b, const upf_launch_config* cf
     return UPF_ERR_INVALID_ARG;
   }
   UPF_CUDA(cudaStreamSynchronize(b->stream));
-  b->shape_set = b->shape_set || !same_loop_shapes(b->shape, sh);
+  b->shape_set = true;
   b->shape = sh;
   return b->have_particles ? build_batch_graph(b) : UPF_OK;
 }
@@ -721,6 +730,7 @@ upf_status upf_batch_autotune(upf_batch* b, int32_t repeats, upf_launch_config* 
   ops.density = [](void* c, cudaStream_t st) { return batch_launch_loop_density(*static_cast<BatchTune*>(c)->b, st); };
   ops.pforce = [](void* c, cudaStream_t st) { return batch_launch_loop_pforce(*static_cast<BatchTune*>(c)->b, st); };
   UPF_TRY(autotune_shapes(ops, repeats, chosen));
+  b->shape_set = false;
   UPF_TRY(batch_check_errors(b));
   return build_batch_graph(b);
 }

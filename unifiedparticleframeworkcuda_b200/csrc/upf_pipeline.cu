@@ -2786,7 +2786,7 @@ cudaError_t launch_list_staging(System& s, cudaStream_t st) {
 // particles takes 53 us staged against 66 at LaunchShape's own values (165
 // against 198 at 1,048,576), and staging, 44 us (145), is paid from the fourth
 // iteration on (a step takes at least three, and 14 in a settled scene).
-static LaunchShape loop_shape(const System& s) {
+LaunchShape loop_shape(const System& s) {
   LaunchShape sh = s.shape;
   if (s.ucodes && !s.shape_set && !s.shape_tuned && !s.stage_always && s.n_dyn > s.loop_sms * kLoopResident) {
     sh.density_mode = sh.pforce_mode = 2;

@@ -231,8 +231,8 @@ struct System {
   unsigned long long* loop_sync = nullptr;  // [2] its barrier
   uint32_t* loop_max = nullptr;   // [2] the maximum predicted density of odd and even iterations
   uint32_t loop_sms = 0;          // the device's SMs (0: no cooperative launches)
-  bool shape_set = false;         // the caller chose the loop passes' shapes: they run as launches of their own
-  bool shape_tuned = false;       // the autotuner chose them (loop_shape)
+  bool shape_set = false;         // the caller set the passes' shapes: the loop's run as launches of their own
+  bool shape_tuned = false;       // the autotuner chose them once (loop_shape)
   bool loop_in_graph = false;     // the step graph being captured has the fused loop: no staging
 
   RigidArrays rb;
@@ -299,7 +299,7 @@ struct BatchSystem {
   unsigned long long* loop_sync = nullptr;  // as System's: the fused loop's barrier, and its running scenes
   uint32_t* loop_max = nullptr;             // [scenes][2]
   uint32_t loop_sms = 0;
-  bool shape_set = false;
+  bool shape_set = false;                   // as System's
   BatchView view;
 
   cudaGraphExec_t step_exec = nullptr;
@@ -395,7 +395,6 @@ struct TuneOps {
 upf_status autotune_shapes(const TuneOps& ops, int repeats, upf_launch_config* out);
 void shape_to_config(const LaunchShape& s, upf_launch_config* c);
 LaunchShape config_to_shape(const upf_launch_config& c);
-bool same_loop_shapes(const LaunchShape& a, const LaunchShape& b);
 
 // upf_rigid.cu: list entry -> sorted index after a sort; body force/torque,
 // body integration and rigid particle sync after integration
@@ -422,6 +421,8 @@ cudaError_t launch_loop_body(System& s, cudaStream_t st, cudaGraphConditionalHan
 cudaError_t launch_loop_density(System& s, cudaStream_t st);
 cudaError_t launch_loop_pforce(System& s, cudaStream_t st);
 cudaError_t launch_loop_ctl(System& s, cudaStream_t st, cudaGraphConditionalHandle h, bool use_handle);
+// the shapes the loop passes run at, where they are launches of their own
+LaunchShape loop_shape(const System& s);
 // the whole loop in one cooperative launch: whether a step graph of this
 // system (batch) takes it, the launch, and the SM count it is sized by
 bool loop_fused(const System& s);
