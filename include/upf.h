@@ -535,16 +535,20 @@ upf_status upf_profile_step(upf_system* s, upf_phase_times* out);
  * Until shapes are set the library chooses how a step runs its predict-correct
  * loop: all iterations in one cooperative launch where the system has at most
  * 1,024 dynamic particles (a batch: slots, each scene's count rounded up to
- * 256) an SM, 151,552 on a B200; above that, a single system's passes from
- * staged neighbourhoods (mode 2, 256 threads, 4 rows), a batch's at the shapes
- * that upf_batch_get_launch_config reports. Any successful
- * upf_set_launch_config is a choice, also of the values that were reported:
- * from then on the loop's passes run as launches of their own at those shapes.
- * upf_autotune gives the choice back: up to 1,024 particles an SM the loop is
- * one launch again, above it the passes run at the tuned shapes. A tuned
- * config set in another handle is a choice there, and so ends the one-launch
- * loop of a small one (1,728 particles: 0.33 ms a step of 50 iterations in one
- * launch, 0.89 with passes); tune each handle, or leave it as it is. */
+ * 256) an SM, 151,552 on a B200, or the passes' launches while at least two
+ * other such loops are in flight on the device (on streams of their own: the
+ * passes of several fill one another's gaps, launches of the whole loop queue;
+ * up to 12 an SM they fit beside one another and stay). Above that, a single
+ * system's passes run from staged neighbourhoods (mode 2, 256 threads, 4
+ * rows), a batch's at the shapes that upf_batch_get_launch_config reports. Any
+ * successful upf_set_launch_config is a choice, also of the values that were
+ * reported: from then on the loop's passes run as launches of their own at
+ * those shapes. upf_autotune gives the choice back: up to 1,024 particles an
+ * SM the loop is one launch again, above it the passes run at the tuned
+ * shapes. A tuned config set in another handle is a choice there, and so ends
+ * the one-launch loop of a small one (1,728 particles: 0.33 ms a step of 50
+ * iterations in one launch, 0.89 with passes); tune each handle, or leave it
+ * as it is. */
 typedef struct upf_launch_config {
   int32_t nlist_threads;      /* 64, 128, 256 */
   int32_t external_threads;   /* 128, 256 */
@@ -781,13 +785,21 @@ upf_status upf_adjoint_times(upf_adjoint* a, float* forward_ms, float* backward_
  * values, the rows past max_neighbors included, set to `byte` (0xff: NaN);
  * what a step leaves of them must not reach its results.
  * upf_test_loop_route(s, &one_launch): whether the system's steps run their
- * predict-correct loop in one launch (1) or its passes as launches of their
- * own (0); upf_test_batch_loop_route likewise for a batch. */
+ * predict-correct loop in one launch (1), its passes as launches of their
+ * own (0), or one of the two as each step finds the device (2);
+ * upf_test_batch_loop_route likewise for a batch.
+ * upf_test_meet_others(s): as if the last step had met two other loops: the
+ * next one takes the passes where it would have been one launch;
+ * upf_test_batch_meet_others likewise.
+ * upf_test_tuned_loop(s, cfg): cfg's shapes as if upf_autotune had picked them. */
 upf_status upf_test_fail_allocation(int32_t nth);
 upf_status upf_test_stage_union_cap(upf_system* s, uint32_t cap);
 upf_status upf_test_fill_list_values(upf_system* s, uint32_t byte);
 upf_status upf_test_loop_route(upf_system* s, int32_t* one_launch);
 upf_status upf_test_batch_loop_route(upf_batch* b, int32_t* one_launch);
+upf_status upf_test_meet_others(upf_system* s);
+upf_status upf_test_tuned_loop(upf_system* s, const upf_launch_config* cfg);
+upf_status upf_test_batch_meet_others(upf_batch* b);
 upf_status upf_selftest_bounded_wait(int device, uint32_t limit_us);
 upf_status upf_selftest_support_bins(int device, const upf_params* p, const float* r2, uint32_t n, int32_t* bins);
 

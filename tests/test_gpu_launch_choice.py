@@ -3,13 +3,14 @@ while nothing is set, the caller's shapes from the first that is set, whatever
 they are and whatever was set before, and the library's again after tuning."""
 import ctypes as C
 
+import numpy as np
 import pytest
 
 from unifiedparticleframeworkcuda_b200 import UpfLaunchConfig, scenes
 
 pytestmark = pytest.mark.gpu
 
-PASSES, ONE_LAUNCH = 0, 1
+PASSES, ONE_LAUNCH, EITHER = 0, 1, 2
 
 
 def route(upf, handle):
@@ -93,3 +94,78 @@ def test_batch(upf_lib):
         assert route(upf_lib, b) == ONE_LAUNCH
         b.step(1)
         b.synchronize()
+
+
+def end_state(handle, scenes_):
+    got = [handle.particles(k) for k in range(scenes_)] if scenes_ else [handle.particles()]
+    st = handle.stats()
+    return got, [(s.iterations, s.total_iterations, s.max_predicted_density) for s in (st if scenes_ else [st])]
+
+
+def same(a, b):
+    assert a[1] == b[1]
+    for u, v in zip(a[0], b[0]):
+        for k in u:
+            assert np.array_equal(u[k], v[k]), k
+
+
+# what a step does beside other loops: its passes, for as long as they are
+# there, and one launch again after them; at default and at tuned shapes
+@pytest.mark.parametrize("loop", [None, (2, 256, 4, 2, 256, 8), (1, 256, 4, 0, 128, 4)])
+def test_a_system_beside_others(upf_lib, loop):
+    sc = scenes.pcisph_dam(20, 18, 16, seed=6, box=(0.3, 0.25, 0.25))
+    with system(upf_lib, sc) as s, system(upf_lib, sc) as t:
+        for _ in range(5):
+            s.step(1)
+        if loop:
+            upf_lib.check(upf_lib.lib().upf_test_tuned_loop(t.handle, C.byref(with_loop(t.launch_config(), loop))),
+                          "upf_test_tuned_loop")
+        for meet in (False, True, True, False, False):
+            if meet:
+                upf_lib.check(upf_lib.lib().upf_test_meet_others(t.handle), "upf_test_meet_others")
+            t.step(1)
+        assert route(upf_lib, t) == EITHER and route(upf_lib, s) == ONE_LAUNCH
+        same(end_state(t, 0), end_state(s, 0))
+
+
+def test_a_batch_beside_others(upf_lib):
+    scs = scenes.batch_scenes(num=4, seed=13, counts=(2048, 8192))
+    with upf_lib.ParticleBatch.from_scenes(scs) as a, upf_lib.ParticleBatch.from_scenes(scs) as b:
+        a.step(4)
+        for meet in (True, True, False, False):
+            if meet:
+                upf_lib.check(upf_lib.lib().upf_test_batch_meet_others(b.handle), "upf_test_batch_meet_others")
+            b.step(1)
+        assert route(upf_lib, b) == EITHER and route(upf_lib, a) == ONE_LAUNCH
+        same(end_state(b, 4), end_state(a, 4))
+
+
+def test_the_smallest_system_does_not_yield(upf_lib):
+    with system(upf_lib, scenes.small_pcisph()) as s:
+        upf_lib.check(upf_lib.lib().upf_test_meet_others(s.handle), "upf_test_meet_others")
+        s.step(2)
+        s.synchronize()
+        assert route(upf_lib, s) == ONE_LAUNCH
+
+
+def test_many_systems_at_once(upf_lib):
+    """Six systems on streams of their own, stepped without waiting: each as
+    if alone."""
+    scs = [scenes.pcisph_dam(20 + k, 18, 17, seed=k, box=(0.35, 0.25, 0.25)) for k in range(6)]
+    want = []
+    for sc in scs:
+        with system(upf_lib, sc) as s:
+            s.step(8)
+            want.append(end_state(s, 0))
+    sys_ = [system(upf_lib, sc) for sc in scs]
+    for _ in range(4):
+        for s in sys_:
+            s.step(1)
+    for s in sys_:
+        s.synchronize()
+    for _ in range(4):
+        for s in sys_:
+            s.step(1)
+    for s, w in zip(sys_, want):
+        same(end_state(s, 0), w)
+        s.close()

@@ -111,6 +111,9 @@ def lib():
             "upf_test_fill_list_values": [vp, C.c_uint32],
             "upf_test_loop_route": [vp, i32p],
             "upf_test_batch_loop_route": [vp, i32p],
+            "upf_test_meet_others": [vp],
+            "upf_test_tuned_loop": [vp, C.POINTER(UpfLaunchConfig)],
+            "upf_test_batch_meet_others": [vp],
             "upf_selftest_bounded_wait": [C.c_int, C.c_uint32],
             "upf_selftest_support_bins": [C.c_int, P, fp, C.c_uint32, i32p],
             "upf_morton_keys": [vp, C.c_uint32, fp, fp, vp, vp],

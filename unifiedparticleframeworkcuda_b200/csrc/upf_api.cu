@@ -394,75 +394,118 @@ upf_status autotune_shapes(const TuneOps& ops, int repeats, upf_launch_config* o
   return UPF_OK;
 }
 
-// One step as a graph: pre -> [while: loop] -> post. The loop body is
-// captured into the body graph of a conditional while-node; the body's last
-// kernel sets the node's condition.
+// A conditional node at the capture point of `at`; the capture goes on after it.
+static cudaError_t add_conditional(cudaStream_t at, cudaGraphConditionalHandle h, cudaGraphConditionalNodeType type,
+                                   unsigned int bodies, cudaGraph_t** body) {
+  cudaStreamCaptureStatus cst;
+  cudaGraph_t g = nullptr;
+  const cudaGraphNode_t* deps = nullptr;
+  size_t ndeps = 0;
+  cudaError_t e = cudaStreamGetCaptureInfo(at, &cst, nullptr, &g, &deps, &ndeps);
+  if (e != cudaSuccess) return e;
+  cudaGraphNodeParams np = {};
+  np.type = cudaGraphNodeTypeConditional;
+  np.conditional.handle = h;
+  np.conditional.type = type;
+  np.conditional.size = bodies;
+  cudaGraphNode_t node;
+  if ((e = cudaGraphAddNode(&node, g, deps, ndeps, &np)) != cudaSuccess) return e;
+  *body = np.conditional.phGraph_out;
+  return cudaStreamUpdateCaptureDependencies(at, &node, 1, cudaStreamSetCaptureDependencies);
+}
+
+static cudaError_t new_handle(cudaStream_t at, cudaGraphConditionalHandle* h) {
+  cudaStreamCaptureStatus cst;
+  cudaGraph_t g = nullptr;
+  const cudaError_t e = cudaStreamGetCaptureInfo(at, &cst, nullptr, &g, nullptr, nullptr);
+  return e == cudaSuccess ? cudaGraphConditionalHandleCreate(h, g, 1, cudaGraphCondAssignDefault) : e;
+}
+
+template <class Fn>
+static cudaError_t capture_body(cudaGraph_t body, Fn&& fn) {
+  cudaStream_t bs = nullptr;
+  cudaError_t e = cudaStreamCreateWithFlags(&bs, cudaStreamNonBlocking);
+  if (e != cudaSuccess) return e;
+  e = cudaStreamBeginCaptureToGraph(bs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+  if (e == cudaSuccess) {
+    const cudaError_t eb = fn(bs);
+    cudaGraph_t out = nullptr;
+    const cudaError_t ee = cudaStreamEndCapture(bs, &out);
+    e = eb != cudaSuccess ? eb : ee;
+  }
+  cudaStreamDestroy(bs);
+  return e;
+}
+
+// Whether the steps of a handle have met others since its graph was built for
+// itself alone. (Not while its stream is being captured: the graph in use is
+// then the caller's.)
+bool met_others(const uint32_t* crowd_host, bool crowded, cudaStream_t st) {
+  if (crowded || !*reinterpret_cast<const volatile uint32_t*>(crowd_host)) return false;
+  cudaStreamCaptureStatus capturing;
+  if (cudaStreamIsCapturing(st, &capturing) == cudaSuccess) return capturing == cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return false;
+}
+
+// One step as a graph: pre -> [while: loop] -> post, or with one_launch
+// pre -> [if: one_launch, else: while: loop] -> post, where a kernel of `pre`
+// sets the choice. The loop body is captured into the body graph of a
+// conditional while-node; the body's last kernel sets the node's condition.
 upf_status capture_step_graph(const GraphParts& parts, cudaGraph_t* graph_out, cudaGraphExec_t* exec_out) {
   *graph_out = nullptr;
   *exec_out = nullptr;
-  cudaStream_t cs = nullptr, body_stream = nullptr;
+  cudaStream_t cs = nullptr;
   UPF_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-  UPF_CUDA(cudaStreamCreateWithFlags(&body_stream, cudaStreamNonBlocking));
-  auto cleanup = [&]() {
-    cudaStreamDestroy(cs);
-    cudaStreamDestroy(body_stream);
-  };
   cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) {
-    cleanup();
+    cudaStreamDestroy(cs);
     set_error("cudaStreamBeginCapture: %s", cudaGetErrorString(e));
     return UPF_ERR_CUDA;
   }
-  auto fail = [&](const char* what, cudaError_t err) {
-    cudaGraph_t g = nullptr;
-    cudaStreamEndCapture(cs, &g);
-    if (g) cudaGraphDestroy(g);
-    cleanup();
-    set_error("step graph: %s: %s", what, cudaGetErrorString(err));
-    return UPF_ERR_CUDA;
+  const char* what = "capture";
+  auto iterate = [&](cudaStream_t at) {
+    cudaGraphConditionalHandle h;
+    cudaGraph_t* body = nullptr;
+    cudaError_t r = parts.before_loop ? parts.before_loop(parts.ctx, at) : cudaSuccess;
+    if (r == cudaSuccess) r = new_handle(at, &h);
+    if (r == cudaSuccess) r = add_conditional(at, h, cudaGraphCondTypeWhile, 1, &body);
+    return r == cudaSuccess ? capture_body(body[0], [&](cudaStream_t bs) { return parts.loop(parts.ctx, bs, h); }) : r;
   };
-  if (parts.pre && (e = parts.pre(parts.ctx, cs)) != cudaSuccess) return fail("pre", e);
-  if (parts.loop) {
-    cudaStreamCaptureStatus cst;
-    cudaGraph_t g = nullptr;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t ndeps = 0;
-    if ((e = cudaStreamGetCaptureInfo(cs, &cst, nullptr, &g, &deps, &ndeps)) != cudaSuccess)
-      return fail("capture info", e);
-    cudaGraphConditionalHandle handle;
-    if ((e = cudaGraphConditionalHandleCreate(&handle, g, 1, cudaGraphCondAssignDefault)) != cudaSuccess)
-      return fail("conditional handle", e);
-    cudaGraphNodeParams np = {};
-    np.type = cudaGraphNodeTypeConditional;
-    np.conditional.handle = handle;
-    np.conditional.type = cudaGraphCondTypeWhile;
-    np.conditional.size = 1;
-    cudaGraphNode_t cnode;
-    if ((e = cudaGraphAddNode(&cnode, g, deps, ndeps, &np)) != cudaSuccess) return fail("while node", e);
-    cudaGraph_t body = np.conditional.phGraph_out[0];
-    if ((e = cudaStreamUpdateCaptureDependencies(cs, &cnode, 1, cudaStreamSetCaptureDependencies)) != cudaSuccess)
-      return fail("capture dependencies", e);
-    if ((e = cudaStreamBeginCaptureToGraph(body_stream, body, nullptr, nullptr, 0,
-                                           cudaStreamCaptureModeThreadLocal)) != cudaSuccess)
-      return fail("body capture", e);
-    cudaError_t eb = parts.loop(parts.ctx, body_stream, handle);
-    cudaGraph_t body_out = nullptr;
-    cudaError_t ee = cudaStreamEndCapture(body_stream, &body_out);
-    if (eb != cudaSuccess) return fail("loop body", eb);
-    if (ee != cudaSuccess) return fail("body end capture", ee);
-  }
-  if (parts.post && (e = parts.post(parts.ctx, cs)) != cudaSuccess) return fail("post", e);
+  [&]() {
+    cudaGraphConditionalHandle route = 0;
+    what = "route";
+    if (parts.one_launch && (e = new_handle(cs, &route)) != cudaSuccess) return;
+    what = "pre";
+    if (parts.pre && (e = parts.pre(parts.ctx, cs, route)) != cudaSuccess) return;
+    what = "loop";
+    if (parts.one_launch) {
+      cudaGraph_t* body = nullptr;
+      if ((e = add_conditional(cs, route, cudaGraphCondTypeIf, 2, &body)) != cudaSuccess) return;
+      if ((e = capture_body(body[0], [&](cudaStream_t bs) { return parts.one_launch(parts.ctx, bs); })) != cudaSuccess)
+        return;
+      if ((e = capture_body(body[1], iterate)) != cudaSuccess) return;
+    } else if (parts.loop && (e = iterate(cs)) != cudaSuccess) {
+      return;
+    }
+    what = "post";
+    if (parts.post) e = parts.post(parts.ctx, cs);
+  }();
   cudaGraph_t graph = nullptr;
-  e = cudaStreamEndCapture(cs, &graph);
-  cleanup();
-  if (e != cudaSuccess) {
-    set_error("step graph end capture: %s", cudaGetErrorString(e));
-    return UPF_ERR_CUDA;
+  const cudaError_t ee = cudaStreamEndCapture(cs, &graph);
+  cudaStreamDestroy(cs);
+  if (e == cudaSuccess && ee != cudaSuccess) {
+    what = "end capture";
+    e = ee;
   }
-  e = cudaGraphInstantiate(exec_out, graph, 0);
+  if (e == cudaSuccess) {
+    what = "instantiate";
+    e = cudaGraphInstantiate(exec_out, graph, 0);
+  }
   if (e != cudaSuccess) {
-    cudaGraphDestroy(graph);
-    set_error("step graph instantiate: %s", cudaGetErrorString(e));
+    if (graph) cudaGraphDestroy(graph);
+    *exec_out = nullptr;
+    set_error("step graph: %s: %s", what, cudaGetErrorString(e));
     return UPF_ERR_CUDA;
   }
   *graph_out = graph;
@@ -478,37 +521,55 @@ void destroy_graph(System& s) {
   s.step_graph = nullptr;
 }
 
-// One step of a system: sort -> neighbours -> forces -> [while: loop body] -> integrate.
+LoopTurn turn_of(const System& s) { return s.loop_yields ? LoopTurn{s.loop_sync + 2, s.crowd_host} : LoopTurn{}; }
+
+// One step of a system: sort -> neighbours -> forces -> loop -> integrate. The
+// loop is a while-node over its passes, one launch, or the device's choice of
+// the two (enter_loop).
 upf_status build_step_graph(System& s) {
   destroy_graph(s);
   GraphParts parts;
   parts.ctx = &s;
-  parts.pre = [](void* c, cudaStream_t st) {
+  parts.pre = [](void* c, cudaStream_t st, cudaGraphConditionalHandle route) {
     System& S = *static_cast<System*>(c);
     const bool pcisph = S.prm.method == UPF_METHOD_PCISPH;
-    cudaError_t e = launch_sort_phase(S, st, true);
+    cudaError_t e = launch_sort_phase(S, st, true, turn_of(S), route);
     if (e == cudaSuccess) e = launch_neighbor_phase(S, st, true);
     if (e == cudaSuccess && pcisph) e = launch_force_phase(S, st);
     return e;
   };
   s.loop_in_graph = loop_fused(s);
-  if (s.prm.method == UPF_METHOD_PCISPH && !s.loop_in_graph)
+  s.loop_yields = s.loop_in_graph && loop_yields(s.n_dyn, s.loop_sms);
+  s.loop_both = s.loop_yields && s.crowded;
+  if (s.loop_both) {
+    parts.one_launch = [](void* c, cudaStream_t st) { return launch_fused_loop(*static_cast<System*>(c), st); };
+    parts.before_loop = [](void* c, cudaStream_t st) { return launch_loop_staging(*static_cast<System*>(c), st); };
+  }
+  if (s.prm.method == UPF_METHOD_PCISPH && (!s.loop_in_graph || s.loop_both))
     parts.loop = [](void* c, cudaStream_t st, cudaGraphConditionalHandle h) {
       return launch_loop_body(*static_cast<System*>(c), st, h, true);
     };
   parts.post = [](void* c, cudaStream_t st) {
     System& S = *static_cast<System*>(c);
-    cudaError_t e = S.loop_in_graph ? launch_fused_loop(S, st) : cudaSuccess;
-    return e == cudaSuccess ? launch_integrate_phase(S, st) : e;
+    cudaError_t e = S.loop_in_graph && !S.loop_both ? launch_fused_loop(S, st) : cudaSuccess;
+    return e == cudaSuccess ? launch_integrate_phase(S, st, turn_of(S)) : e;
   };
   // capturing runs the launchers' host code without running the kernels:
   // the host-side record of whether the current lists are staged is kept,
   // and whether a step of this graph stages them is noted for upf_step
   const bool staged_now = s.lists_staged;
   const upf_status rc = capture_step_graph(parts, &s.step_graph, &s.step_exec);
-  s.graph_stages = s.lists_staged;
-  s.loop_in_graph = false;
+  s.graph_stages = s.lists_staged && !s.loop_in_graph;
+  const bool fused = s.loop_in_graph;
+  s.loop_in_graph = s.loop_yields = s.loop_both = false;
   s.lists_staged = staged_now;
+  if (rc != UPF_OK && fused) {
+    // a share of the device (MPS) that does not hold the cooperative grid, or
+    // not in a conditional body: the passes
+    cudaGetLastError();
+    s.loop_sms = 0;
+    return build_step_graph(s);
+  }
   return rc;
 }
 
@@ -703,7 +764,26 @@ upf_status upf_test_loop_route(upf_system* s, int32_t* one_launch) {
     set_error("upf_test_loop_route: null");
     return UPF_ERR_INVALID_ARG;
   }
-  *one_launch = loop_fused(*s);
+  *one_launch = loop_fused(*s) ? 1 + (s->crowded && loop_yields(s->n_dyn, s->loop_sms)) : 0;
+  return UPF_OK;
+}
+
+upf_status upf_test_tuned_loop(upf_system* s, const upf_launch_config* cfg) {
+  UPF_TRY(upf_set_launch_config(s, cfg));
+  s->shape_set = false;
+  s->shape_tuned = true;
+  return s->have_particles ? build_step_graph(*s) : UPF_OK;
+}
+
+upf_status upf_test_meet_others(upf_system* s) {
+  if (!s) {
+    set_error("upf_test_meet_others: null");
+    return UPF_ERR_INVALID_ARG;
+  }
+  const unsigned long long seen = 2;
+  UPF_CUDA(cudaStreamSynchronize(s->stream));
+  UPF_CUDA(cudaMemcpy(s->loop_sync + 2, &seen, sizeof(seen), cudaMemcpyHostToDevice));
+  *s->crowd_host = 1;
   return UPF_OK;
 }
 
@@ -896,7 +976,7 @@ upf_status upf_create(const upf_params* p, int device, uint32_t capacity, upf_sy
   ALLOC(s->mpos, c);
   ALLOC(s->spos, c); ALLOC(s->skeys, c); ALLOC(s->sid, c);
   ALLOC(s->luts, 5 * UPF_LUT_ENTRIES + kThresholds);
-  ALLOC(s->st, 1); ALLOC(s->loop_sync, 2); ALLOC(s->loop_max, 2);
+  ALLOC(s->st, 1); ALLOC(s->loop_sync, 3); ALLOC(s->loop_max, 2);
   s->loop_sms = loop_cooperative_sms();
   if (p->method == UPF_METHOD_PCISPH) {
     // staged neighbourhoods of the loop passes (loop-pass mode 2)
@@ -908,12 +988,14 @@ upf_status upf_create(const upf_params* p, int device, uint32_t capacity, upf_sy
 #undef ALLOC
   if ((st = encode_list_maps(s->nbr_maps, s->lval_maps, s->nbr, s->lval, s->nstride, p->max_neighbors)) != UPF_OK)
     return bail(st);
-  e = cudaMallocHost((void**)&s->st_host, sizeof(DevState));
+  e = cudaMallocHost((void**)&s->st_host, sizeof(DevState) + sizeof(uint32_t));
   if (e != cudaSuccess) {
     s->st_host = nullptr;
     set_error("cudaMallocHost: %s", cudaGetErrorString(e));
     return bail(UPF_ERR_ALLOC);
   }
+  s->crowd_host = (uint32_t*)(s->st_host + 1);
+  *s->crowd_host = 0;
   std::vector<float> lut(5 * UPF_LUT_ENTRIES + kThresholds);
   build_luts(*p, lut.data());
   build_bin_thresholds(*p, lut.data() + 5 * UPF_LUT_ENTRIES);
@@ -927,6 +1009,7 @@ upf_status upf_create(const upf_params* p, int device, uint32_t capacity, upf_sy
   if (e == cudaSuccess && s->ucount)
     e = cudaMemset(s->ucount, 0xff, sizeof(uint32_t) * (((size_t)c + kStageChunk - 1) / kStageChunk));
   if (e == cudaSuccess) e = cudaMemset(s->st, 0, sizeof(DevState));
+  if (e == cudaSuccess) e = cudaMemset(s->loop_sync, 0, sizeof(unsigned long long) * 3);
   if (e != cudaSuccess) {
     set_error("upload: %s", cudaGetErrorString(e));
     return bail(UPF_ERR_CUDA);
@@ -1211,6 +1294,7 @@ upf_status upf_step(upf_system* s, int32_t nsteps) {
     set_error("upf_step: call upf_set_particles first");
     return UPF_ERR_STATE;
   }
+  if (met_others(s->crowd_host, s->crowded, s->stream)) s->crowded = s->graph_stale = true;
   if (s->graph_stale) {
     UPF_TRY(build_step_graph(*s));
     s->graph_stale = false;

@@ -103,28 +103,46 @@ void destroy_batch_graph(upf_batch* b) {
   b->step_graph = nullptr;
 }
 
+LoopTurn turn_of(const BatchSystem& b) {
+  return b.loop_yields ? LoopTurn{b.loop_sync + 2, b.crowd_host} : LoopTurn{};
+}
+
 upf_status build_batch_graph(upf_batch* b) {
   destroy_batch_graph(b);
   GraphParts parts;
   parts.ctx = static_cast<BatchSystem*>(b);
-  parts.pre = [](void* c, cudaStream_t st) {
+  // the loop as in a system's graph (build_step_graph)
+  const bool fused = batch_loop_fused(*b);
+  b->loop_yields = fused && loop_yields(b->n_slots, b->loop_sms);
+  b->loop_both = b->loop_yields && b->crowded;
+  parts.pre = [](void* c, cudaStream_t st, cudaGraphConditionalHandle route) {
     BatchSystem& B = *static_cast<BatchSystem*>(c);
     cudaError_t e = batch_launch_sort(B, st);
     if (e == cudaSuccess) e = batch_launch_neighbors(B, st);
     if (e == cudaSuccess) e = batch_launch_forces(B, st);
-    if (e == cudaSuccess) e = batch_launch_loop_init(B, st);
+    if (e == cudaSuccess) e = batch_launch_loop_init(B, st, turn_of(B), route);
     return e;
   };
-  if (!batch_loop_fused(*b))
+  if (b->loop_both)
+    parts.one_launch = [](void* c, cudaStream_t st) {
+      return batch_launch_fused_loop(*static_cast<BatchSystem*>(c), st);
+    };
+  if (!fused || b->loop_both)
     parts.loop = [](void* c, cudaStream_t st, cudaGraphConditionalHandle h) {
       return batch_capture_loop_body(*static_cast<BatchSystem*>(c), st, h);
     };
   parts.post = [](void* c, cudaStream_t st) {
     BatchSystem& B = *static_cast<BatchSystem*>(c);
-    cudaError_t e = batch_loop_fused(B) ? batch_launch_fused_loop(B, st) : cudaSuccess;
-    return e == cudaSuccess ? batch_launch_integrate(B, st) : e;
+    cudaError_t e = batch_loop_fused(B) && !B.loop_both ? batch_launch_fused_loop(B, st) : cudaSuccess;
+    return e == cudaSuccess ? batch_launch_integrate(B, st, turn_of(B)) : e;
   };
-  return capture_step_graph(parts, &b->step_graph, &b->step_exec);
+  const upf_status rc = capture_step_graph(parts, &b->step_graph, &b->step_exec);
+  if (rc != UPF_OK && fused) {  // as build_step_graph
+    cudaGetLastError();
+    b->loop_sms = 0;
+    return build_batch_graph(b);
+  }
+  return rc;
 }
 
 upf_status batch_guard(upf_batch* b, const char* where) {
@@ -276,19 +294,21 @@ upf_status upf_batch_create(const upf_params* params, const uint32_t* counts, ui
   ALLOC(b->st_d, num_scenes);
   ALLOC(b->group_scene_d, group_scene.size()); ALLOC(b->seg_begin_d, num_scenes); ALLOC(b->seg_end_d, num_scenes);
   ALLOC(b->cell_base_d, num_scenes); ALLOC(b->any_active_d, 1);
-  ALLOC(b->loop_sync, 2); ALLOC(b->loop_max, (size_t)2 * num_scenes);
+  ALLOC(b->loop_sync, 3); ALLOC(b->loop_max, (size_t)2 * num_scenes);
   b->loop_sms = loop_cooperative_sms();
   ALLOC(b->active_groups_d, n / kSegAlign + 1); ALLOC(b->n_active_groups_d, 1);
   ALLOC(b->x.comp_begin_d, num_scenes); ALLOC(b->x.stage_a, std::max<size_t>(total, 1));
   ALLOC(b->x.stage_b, std::max<size_t>(total, 1));
 #undef ALLOC
   if ((st = encode_list_maps(b->nbr_maps, b->lval_maps, b->nbr, b->lval, n, rows)) != UPF_OK) return bail(st);
-  e = cudaMallocHost((void**)&b->st_h, sizeof(DevState) * num_scenes);
+  e = cudaMallocHost((void**)&b->st_h, sizeof(DevState) * num_scenes + sizeof(uint32_t));
   if (e != cudaSuccess) {
     b->st_h = nullptr;
     set_error("cudaMallocHost: %s", cudaGetErrorString(e));
     return bail(UPF_ERR_ALLOC);
   }
+  b->crowd_host = (uint32_t*)(b->st_h + num_scenes);
+  *b->crowd_host = 0;
   // per-scene parameters and tables
   std::vector<DevParams> dps(num_scenes);
   std::vector<float> luts((size_t)num_scenes * kLutFloats);
@@ -313,6 +333,7 @@ upf_status upf_batch_create(const upf_params* params, const uint32_t* counts, ui
   if (e == cudaSuccess)
     e = cudaMemcpy(b->x.comp_begin_d, comp_begin.data(), sizeof(uint32_t) * num_scenes, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemset(b->st_d, 0, sizeof(DevState) * num_scenes);
+  if (e == cudaSuccess) e = cudaMemset(b->loop_sync, 0, sizeof(unsigned long long) * 3);
   if (e == cudaSuccess) e = cudaMemset(b->A.type, 0xff, sizeof(int32_t) * n);  // padding: no type
   if (e == cudaSuccess) e = cudaMemset(b->A.pos, 0, sizeof(float4) * n);
   if (e == cudaSuccess) e = cudaMemset(b->A.vel, 0, sizeof(float4) * n);
@@ -406,6 +427,10 @@ upf_status upf_batch_step(upf_batch* b, int32_t nsteps) {
   if (nsteps < 0) {
     set_error("upf_batch_step: negative step count");
     return UPF_ERR_INVALID_ARG;
+  }
+  if (met_others(b->crowd_host, b->crowded, b->stream)) {
+    b->crowded = true;
+    UPF_TRY(build_batch_graph(b));
   }
   for (int32_t k = 0; k < nsteps; ++k) UPF_CUDA(cudaGraphLaunch(b->step_exec, b->stream));
   return UPF_OK;
@@ -651,7 +676,19 @@ upf_status upf_test_batch_loop_route(upf_batch* b, int32_t* one_launch) {
     set_error("upf_test_batch_loop_route: null");
     return UPF_ERR_INVALID_ARG;
   }
-  *one_launch = batch_loop_fused(*b);
+  *one_launch = batch_loop_fused(*b) ? 1 + (b->crowded && loop_yields(b->n_slots, b->loop_sms)) : 0;
+  return UPF_OK;
+}
+
+upf_status upf_test_batch_meet_others(upf_batch* b) {
+  if (!b) {
+    set_error("upf_test_batch_meet_others: null");
+    return UPF_ERR_INVALID_ARG;
+  }
+  const unsigned long long seen = 2;
+  UPF_CUDA(cudaStreamSynchronize(b->stream));
+  UPF_CUDA(cudaMemcpy(b->loop_sync + 2, &seen, sizeof(seen), cudaMemcpyHostToDevice));
+  *b->crowd_host = 1;
   return UPF_OK;
 }
 

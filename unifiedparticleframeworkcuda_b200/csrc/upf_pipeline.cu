@@ -348,7 +348,37 @@ struct StepStart {
   unsigned long long* sync = nullptr;
   uint32_t* loop_max = nullptr;
   int count_step = 0;
+  LoopTurn turn;
+  cudaGraphConditionalHandle route = 0;
 };
+
+// The loops in flight on the device that could be one launch and would hold
+// more than half of its SMs (loop_yields). Such launches run one after another,
+// slower than the same loops' passes side by side, which fill one another's
+// gaps: eight systems of 8,000 particles, 50 iterations each, 3.5 ms a round in
+// one launch each, 2.1 as passes (2.8 before the one-launch loop); of 21,000
+// 4.5, 2.6 and 3.3; of 53,157 6.5, 4.5 and 5.1. Alone and in pairs the one
+// launch is the faster (8,000: 0.45 and 0.85 ms against 0.95 and 1.07). So a
+// step takes the passes where at least two other loops are in flight when it
+// begins, or were when its last one ended (steps that begin together see one
+// another only then). Either form gives the same results.
+// A step's choice costs a conditional node, 15 us; a graph without one tells
+// the host when it has met two others (LoopTurn), and the handle then takes a
+// graph with both forms. A program with one or two systems pays nothing.
+__device__ uint32_t g_loops_in_flight = 0;
+constexpr uint32_t kLoopsBeside = 2;
+__device__ __forceinline__ void enter_loop(const LoopTurn& turn, cudaGraphConditionalHandle route) {
+  const uint32_t beside = max(atomicAdd(&g_loops_in_flight, 1u), (uint32_t)*turn.seen);
+  if (route)
+    cudaGraphSetConditional(route, beside < kLoopsBeside ? 1u : 0u);
+  else if (beside >= kLoopsBeside)
+    *reinterpret_cast<volatile uint32_t*>(turn.crowd) = 1;
+}
+__device__ __forceinline__ void leave_loop(const LoopTurn& turn) {
+  const uint32_t beside = atomicSub(&g_loops_in_flight, 1u) - 1u;
+  *turn.seen = beside;
+  if (beside >= kLoopsBeside) *reinterpret_cast<volatile uint32_t*>(turn.crowd) = 1;
+}
 
 __device__ __forceinline__ void step_init(DevState* st, int count_step) {
   st->ke = 0;
@@ -389,6 +419,7 @@ __global__ void __launch_bounds__(kBlock) k_reorder(
   if (t == 0 && start.st) {
     step_init(start.st, start.count_step);
     if (start.sync) loop_init(start.st, start.sync, start.loop_max);
+    if (start.turn.seen) enter_loop(start.turn, start.route);
   }
   if (t >= n + ns) return;
   const bool dyn = t < n;
@@ -2367,8 +2398,10 @@ __global__ void k_step_init_batch(DevState* st, uint32_t nscenes) {
 }
 
 __global__ void k_loop_init_batch(DevState* st, uint32_t nscenes, int32_t* any_active,
-                                  unsigned long long* sync, uint32_t* loop_max) {
+                                  unsigned long long* sync, uint32_t* loop_max, const LoopTurn turn,
+                                  cudaGraphConditionalHandle route) {
   if (threadIdx.x == 0) {
+    if (turn.seen) enter_loop(turn, route);
     sync[0] = 0;        // arrivals at the fused loop's barrier
     sync[1] = nscenes;  // scenes whose loop still runs
   }
@@ -2453,8 +2486,10 @@ template <bool kBatch>
 __global__ void __launch_bounds__(kBlock) k_pcisph_integrate(
     const __grid_constant__ DevParams Pk, const BatchView bv, uint32_t n, DynArrays B, DynArrays A,
     uint32_t* __restrict__ keysA, const float4* __restrict__ force, const float4* __restrict__ pforce,
-    const float* __restrict__ rho, const float* __restrict__ press, DevState* __restrict__ st_plain) {
+    const float* __restrict__ rho, const float* __restrict__ press, DevState* __restrict__ st_plain,
+    const LoopTurn turn) {
   __shared__ DevParams sP;
+  if (turn.seen && blockIdx.x == 0 && threadIdx.x == 0) leave_loop(turn);
   const Scope sc = enter_scope<kBatch>(Pk, nullptr, st_plain, n, bv, &sP, false);
   if (kBatch) __syncthreads();
   const DevParams& P = *sc.P;
@@ -2743,7 +2778,8 @@ cudaError_t copy_arrays(const CopyList& list, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_sort_phase(System& s, cudaStream_t st, bool starts_step) {
+cudaError_t launch_sort_phase(System& s, cudaStream_t st, bool starts_step, const LoopTurn& turn,
+                              cudaGraphConditionalHandle route) {
   const uint32_t n = s.n_dyn;
   if (n == 0) {
     if (starts_step) {
@@ -2760,7 +2796,8 @@ cudaError_t launch_sort_phase(System& s, cudaStream_t st, bool starts_step) {
   if ((e = cudaMemsetAsync(s.cells, 0, sizeof(uint32_t) * s.ncells * (s.n_static ? 4 : 2), st)) != cudaSuccess) return e;
   StepStart start;
   const bool pcisph = s.prm.method == UPF_METHOD_PCISPH;
-  if (starts_step) start = StepStart{s.st, pcisph ? s.loop_sync : nullptr, s.loop_max, pcisph ? 0 : 1};
+  if (starts_step)
+    start = StepStart{s.st, pcisph ? s.loop_sync : nullptr, s.loop_max, pcisph ? 0 : 1, turn, route};
   k_reorder<<<grid_of(n + s.n_static), kBlock, 0, st>>>(
       n, s.perm, s.keysA, s.A, s.B, pcisph, 3 * (int)s.dp.cell_shift, s.ncells, s.cstart(), s.cend(), s.n_static,
       s.skeys, s.spos, s.dp.static_base, s.mpos, s.mstart(), s.mend(), start);
@@ -2794,6 +2831,13 @@ LaunchShape loop_shape(const System& s) {
     sh.density_rows = sh.pforce_rows = 4;
   }
   return sh;
+}
+
+// (the form of a step graph whose loop may be one launch: before its passes only)
+cudaError_t launch_loop_staging(System& s, cudaStream_t st) {
+  const LaunchShape sh = loop_shape(s);
+  const bool staged = s.ucodes && (loop_mode_staged(sh.density_mode) || loop_mode_staged(sh.pforce_mode));
+  return staged ? launch_stage_lists(s, st) : cudaSuccess;
 }
 
 // the lists are staged when a loop pass reads staged neighbourhoods (or
@@ -2871,6 +2915,13 @@ cudaError_t launch_loop_init(System& s, cudaStream_t st) {
 template <bool kBatch, int kThreads, int kResident, int kLanes, int kHeld, int kRows>
 static cudaError_t run_loop_shape(cudaStream_t st, uint32_t n, void** args) {
   constexpr uint32_t chunk = kThreads / kLanes;
+  // every CTA must be resident at once (where not, the caller takes the passes)
+  int per_sm = 0;
+  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+      &per_sm, k_pcisph_loop<kBatch, kThreads, kResident, kLanes, kHeld, kRows>, kThreads,
+      loop_smem<kThreads, kLanes, kHeld, kRows>());
+  if (e != cudaSuccess) return e;
+  if (per_sm < kResident / kThreads) return cudaErrorCooperativeLaunchTooLarge;
   return cudaLaunchCooperativeKernel((const void*)k_pcisph_loop<kBatch, kThreads, kResident, kLanes, kHeld, kRows>,
                                      dim3((n + chunk - 1) / chunk), dim3(kThreads), args,
                                      loop_smem<kThreads, kLanes, kHeld, kRows>(), st);
@@ -2909,6 +2960,11 @@ uint32_t loop_cooperative_sms() {
   }
   return (uint32_t)sms;
 }
+
+// The smallest scenes' grids (32 lanes, 8 particles a CTA) find room on the
+// SMs two at a time, and as launches one after another are the faster form
+// however many there are (eight of 1,728: 1.1 ms a round, 2.0 as passes): no choice.
+bool loop_yields(uint32_t n, uint32_t sms) { return n > sms * 12; }
 
 bool loop_fused(const System& s) {
   return s.prm.method == UPF_METHOD_PCISPH && !s.shape_set && s.n_dyn && s.n_dyn <= s.loop_sms * kLoopResident;
@@ -2998,7 +3054,7 @@ cudaError_t launch_upload_keys(System& s, cudaStream_t st) {
   return morton_keys(s.A.pos, s.n_dyn, s.dp.origin, s.dp.scales, s.keysA, st);
 }
 
-cudaError_t launch_integrate_phase(System& s, cudaStream_t st) {
+cudaError_t launch_integrate_phase(System& s, cudaStream_t st, const LoopTurn& turn) {
   const uint32_t n = s.n_dyn;
   if (n == 0) return cudaSuccess;
   if (s.prm.method == UPF_METHOD_WCSPH) {
@@ -3016,8 +3072,8 @@ cudaError_t launch_integrate_phase(System& s, cudaStream_t st) {
     }
 #undef UPF_WF
   } else {
-    k_pcisph_integrate<false><<<grid_of(n), kBlock, 0, st>>>(s.dp, BatchView{}, n, s.B, s.A, s.keysA, s.force, s.pforce, s.rho, s.press,
-                                                      s.st);
+    k_pcisph_integrate<false><<<grid_of(n), kBlock, 0, st>>>(s.dp, BatchView{}, n, s.B, s.A, s.keysA, s.force, s.pforce,
+                                                             s.rho, s.press, s.st, turn);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     return launch_rigid_phase(s, st);
@@ -3107,8 +3163,9 @@ cudaError_t batch_launch_forces(BatchSystem& b, cudaStream_t st) {
                             b.force, b.pforce, b.xs, b.press, b.pq, nullptr);
 }
 
-cudaError_t batch_launch_loop_init(BatchSystem& b, cudaStream_t st) {
-  k_loop_init_batch<<<1, 256, 0, st>>>(b.st_d, b.n_scenes, b.any_active_d, b.loop_sync, b.loop_max);
+cudaError_t batch_launch_loop_init(BatchSystem& b, cudaStream_t st, const LoopTurn& turn,
+                                   cudaGraphConditionalHandle route) {
+  k_loop_init_batch<<<1, 256, 0, st>>>(b.st_d, b.n_scenes, b.any_active_d, b.loop_sync, b.loop_max, turn, route);
   return cudaGetLastError();
 }
 
@@ -3231,11 +3288,11 @@ cudaError_t batch_launch_loop_body(BatchSystem& b, cudaStream_t st, cudaGraphCon
   return e;
 }
 
-cudaError_t batch_launch_integrate(BatchSystem& b, cudaStream_t st) {
+cudaError_t batch_launch_integrate(BatchSystem& b, cudaStream_t st, const LoopTurn& turn) {
   const uint32_t n = b.n_slots;
   if (!n) return cudaSuccess;
   k_pcisph_integrate<true><<<grid_of(n), kBlock, 0, st>>>(DevParams{}, b.view, n, b.B, b.A, b.keysA, b.force,
-                                                          b.pforce, b.rho, b.press, nullptr);
+                                                          b.pforce, b.rho, b.press, nullptr, turn);
   return cudaGetLastError();
 }
 

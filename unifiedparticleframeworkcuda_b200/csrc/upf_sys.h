@@ -147,6 +147,13 @@ struct FrameIO {
 cudaError_t frame_streams_create(FrameIO& io, cudaStream_t compute);
 void frame_streams_destroy(FrameIO& io);  // waits for the copies; buffers stay with their owner
 
+// A step's turn among the device's one-launch loops (enter_loop): the loops
+// seen beside the last one, and the host's word for having met two others.
+struct LoopTurn {
+  unsigned long long* seen = nullptr;  // null: not counted
+  uint32_t* crowd = nullptr;
+};
+
 struct System {
   upf_params prm{};
   DevParams dp{};
@@ -228,12 +235,16 @@ struct System {
   cudaGraph_t step_graph = nullptr;
   int key_bits = 30;
   // the predict-correct loop as one cooperative launch (k_pcisph_loop)
-  unsigned long long* loop_sync = nullptr;  // [2] its barrier
+  unsigned long long* loop_sync = nullptr;  // [2] its barrier, the loops seen beside the last one (leave_loop)
   uint32_t* loop_max = nullptr;   // [2] the maximum predicted density of odd and even iterations
   uint32_t loop_sms = 0;          // the device's SMs (0: no cooperative launches)
   bool shape_set = false;         // the caller set the passes' shapes: the loop's run as launches of their own
   bool shape_tuned = false;       // the autotuner chose them once (loop_shape)
   bool loop_in_graph = false;     // the step graph being captured has the fused loop: no staging
+  bool loop_yields = false;       // and counts among the device's loops (loop_yields())
+  bool loop_both = false;         // and has the passes beside it
+  bool crowded = false;           // the step graph is the one with both forms, for good
+  uint32_t* crowd_host = nullptr;  // pinned: set by a step that met others (behind st_host)
 
   RigidArrays rb;
   std::vector<void*> rigid_allocations;   // freed when bodies are set again
@@ -296,10 +307,14 @@ struct BatchSystem {
   uint32_t* active_groups_d = nullptr;  // [n_slots / kSegAlign] groups of the scenes still iterating
   uint32_t* n_active_groups_d = nullptr;
   uint32_t active_grid = 0;             // resident CTAs of the active-group passes
-  unsigned long long* loop_sync = nullptr;  // as System's: the fused loop's barrier, and its running scenes
+  unsigned long long* loop_sync = nullptr;  // as System's: the fused loop's barrier, its running scenes, loops seen
   uint32_t* loop_max = nullptr;             // [scenes][2]
   uint32_t loop_sms = 0;
   bool shape_set = false;                   // as System's
+  bool loop_yields = false;                 // as System's
+  bool loop_both = false;
+  bool crowded = false;
+  uint32_t* crowd_host = nullptr;           // behind st_h
   BatchView view;
 
   cudaGraphExec_t step_exec = nullptr;
@@ -339,7 +354,8 @@ cudaError_t batch_launch_keys(BatchSystem& b, cudaStream_t st);   // keys only
 cudaError_t batch_launch_sort(BatchSystem& b, cudaStream_t st);
 cudaError_t batch_launch_neighbors(BatchSystem& b, cudaStream_t st);
 cudaError_t batch_launch_forces(BatchSystem& b, cudaStream_t st);
-cudaError_t batch_launch_loop_init(BatchSystem& b, cudaStream_t st);
+cudaError_t batch_launch_loop_init(BatchSystem& b, cudaStream_t st, const LoopTurn& turn = {},
+                                   cudaGraphConditionalHandle route = 0);
 cudaError_t batch_launch_loop_body(BatchSystem& b, cudaStream_t st, cudaGraphConditionalHandle h, bool use_handle);
 cudaError_t batch_launch_loop_density(BatchSystem& b, cudaStream_t st);
 cudaError_t batch_launch_loop_pforce(BatchSystem& b, cudaStream_t st);
@@ -352,16 +368,20 @@ cudaError_t batch_launch_loop_pforce_active(BatchSystem& b, cudaStream_t st);
 cudaError_t batch_capture_loop_body(BatchSystem& b, cudaStream_t st, cudaGraphConditionalHandle h);
 cudaError_t batch_launch_loop_ctl(BatchSystem& b, cudaStream_t st, cudaGraphConditionalHandle h = 0,
                                   bool use_handle = false);
-cudaError_t batch_launch_integrate(BatchSystem& b, cudaStream_t st);
+cudaError_t batch_launch_integrate(BatchSystem& b, cudaStream_t st, const LoopTurn& turn = {});
 
 // upf_api.cu: one step as a CUDA graph, `loop` (if given) under a
-// conditional while-node between `pre` and `post`
+// conditional while-node between `pre` and `post`; with `one_launch`, that
+// where `pre` has set its handle to 1, and else before_loop and the while-node
 struct GraphParts {
-  cudaError_t (*pre)(void* ctx, cudaStream_t st) = nullptr;
+  cudaError_t (*pre)(void* ctx, cudaStream_t st, cudaGraphConditionalHandle route) = nullptr;
+  cudaError_t (*one_launch)(void* ctx, cudaStream_t st) = nullptr;
+  cudaError_t (*before_loop)(void* ctx, cudaStream_t st) = nullptr;
   cudaError_t (*loop)(void* ctx, cudaStream_t st, cudaGraphConditionalHandle h) = nullptr;
   cudaError_t (*post)(void* ctx, cudaStream_t st) = nullptr;
   void* ctx = nullptr;
 };
+bool met_others(const uint32_t* crowd_host, bool crowded, cudaStream_t st);
 upf_status capture_step_graph(const GraphParts& parts, cudaGraph_t* graph_out, cudaGraphExec_t* exec_out);
 DevParams make_dev_params(const upf_params& p, uint32_t nstride);
 upf_status encode_list_map(CUtensorMap* map, void* base, CUtensorMapDataType dt, uint32_t elem_bytes,
@@ -408,7 +428,9 @@ int rigid_launches_per_step(const System& s);
 
 // upf_pipeline.cu: phase launchers (all asynchronous on s.stream)
 // starts_step: with the step's (and loop's) initial state
-cudaError_t launch_sort_phase(System& s, cudaStream_t st, bool starts_step = false);
+// (turn: and enters the loop; route: the handle of its form, where the graph has both)
+cudaError_t launch_sort_phase(System& s, cudaStream_t st, bool starts_step = false, const LoopTurn& turn = {},
+                              cudaGraphConditionalHandle route = 0);
 // in_step: the sort phase has started the step; WCSPH densities in the same launch
 cudaError_t launch_neighbor_phase(System& s, cudaStream_t st, bool in_step = false);
 // the list build's copy of the sorted positions, from the positions as they are
@@ -430,9 +452,12 @@ cudaError_t launch_fused_loop(System& s, cudaStream_t st);
 bool batch_loop_fused(const BatchSystem& b);
 cudaError_t batch_launch_fused_loop(BatchSystem& b, cudaStream_t st);
 uint32_t loop_cooperative_sms();
+// whether the fused loop of n particles (slots) gives way to its passes beside others
+bool loop_yields(uint32_t n, uint32_t sms);
+cudaError_t launch_loop_staging(System& s, cudaStream_t st);  // staging where the loop's passes need it
 cudaError_t launch_list_staging(System& s, cudaStream_t st);  // k_stage_lists over the current lists
 cudaError_t launch_upload_keys(System& s, cudaStream_t st);
-cudaError_t launch_integrate_phase(System& s, cudaStream_t st);
+cudaError_t launch_integrate_phase(System& s, cudaStream_t st, const LoopTurn& turn = {});
 cudaError_t launch_static_setup(System& s, cudaStream_t st);
 int pipeline_launches_per_step(const System& s, int iterations);
 
