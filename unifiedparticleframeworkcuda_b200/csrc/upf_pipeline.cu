@@ -2736,20 +2736,6 @@ static cudaError_t nlist_opt_in() {
                               (int)nlist_smem<256, 32>());
 }
 
-// Likewise the fused loop's.
-template <bool kBatch, int kThreads, int kResident, int kLanes, int kHeld, int kRows>
-static cudaError_t loop_opt_in_shape() {
-  return cudaFuncSetAttribute(k_pcisph_loop<kBatch, kThreads, kResident, kLanes, kHeld, kRows>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)loop_smem<kThreads, kLanes, kHeld, kRows>());
-}
-template <bool kBatch>
-static cudaError_t loop_opt_in() {
-  cudaError_t e = loop_opt_in_shape<kBatch, 256, 768, 32, 48, 1>();
-  if (e == cudaSuccess) e = loop_opt_in_shape<kBatch, 256, 768, 16, 48, 2>();
-  return e;
-}
-
 cudaError_t pipeline_init() {
   static std::mutex mu;
   static bool done[64] = {};
@@ -2763,8 +2749,6 @@ cudaError_t pipeline_init() {
   if ((e = nlist_opt_in<true, false, false>()) != cudaSuccess) return e;
   if ((e = nlist_opt_in<false, false, true>()) != cudaSuccess) return e;
   if ((e = nlist_opt_in<false, true, true>()) != cudaSuccess) return e;
-  if ((e = loop_opt_in<false>()) != cudaSuccess) return e;
-  if ((e = loop_opt_in<true>()) != cudaSuccess) return e;
   if (dev >= 0 && dev < 64) done[dev] = true;
   return cudaSuccess;
 }
@@ -2915,6 +2899,7 @@ cudaError_t launch_loop_init(System& s, cudaStream_t st) {
 template <bool kBatch, int kThreads, int kResident, int kLanes, int kHeld, int kRows>
 static cudaError_t run_loop_shape(cudaStream_t st, uint32_t n, void** args) {
   constexpr uint32_t chunk = kThreads / kLanes;
+  static_assert(loop_smem<kThreads, kLanes, kHeld, kRows>() + 3072 <= 48 * 1024, "fits without opting in (with the table)");
   // every CTA must be resident at once (where not, the caller takes the passes)
   int per_sm = 0;
   const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
