@@ -126,6 +126,34 @@ def test_full_size_staged_modes_equal_the_default_shape(upf_lib):
             assert np.array_equal(got[f], ref[f]), f
 
 
+def test_full_size_untuned_and_staged_passes_equal_plain_ones(upf_lib):
+    """pcisph_dam_break_1M, two steps from rest: an untuned system, whose
+    passes are staged by default, and both staged shapes, against passes that
+    walk the plain lists (the TMA ring and direct loads)."""
+    sc = scenes.pcisph_dam()
+    p = upf_lib.derive_params(sc.params)
+    out = []
+    for shape in ((0, 128, 4), (1, 256, 4), None, (2, 256, 4), (2, 256, 8)):
+        with upf_lib.ParticleSystem(p, capacity=sc.n, derive=False) as s:
+            s.set_particles(sc.pos, sc.vel, sc.type)
+            c = s.launch_config()
+            if shape:
+                c.density_mode, c.density_threads, c.density_rows = shape
+                c.pforce_mode, c.pforce_threads, c.pforce_rows = shape
+                s.set_launch_config(c)
+            else:
+                assert c.density_mode == 2 and c.pforce_mode == 2
+            s.step(2)
+            g = s.particles()
+            o = np.argsort(g["id"], kind="stable")
+            out.append(({k: g[k][o] for k in ("pos", "vel", "density", "pressure")}, s.stats().iterations))
+    ref, it = out[0]
+    for got, it2 in out[1:]:
+        assert it2 == it
+        for f in ref:
+            assert np.array_equal(got[f], ref[f]), f
+
+
 def test_full_size_coupling_step(upf_lib, oracle_lib):
     sc = scenes.coupling_scene()
     assert sc.num_bodies == 16
