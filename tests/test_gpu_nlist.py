@@ -94,6 +94,12 @@ def test_particles_a_warp_do_not_change_the_lists(upf_lib, n):
         assert np.array_equal(u, v)
 
 
+@pytest.mark.parametrize("n", [29999, 30000, 360000])
+def test_counts_at_which_a_warp_takes_more(upf_lib, n):
+    """Likewise at the counts where the number doubles, and below one."""
+    test_particles_a_warp_do_not_change_the_lists(upf_lib, n)
+
+
 def test_more_neighbours_than_the_list_holds_is_an_error(upf_lib):
     p, pos, typ = cloud(700, 0, seed=9, clump=300)
     p.max_neighbors = 128

@@ -36,3 +36,9 @@ def test_step_equals_phases_and_oracle(upf_lib, oracle_lib, side, flags, rigid):
     s.close()
     for k in a:
         assert np.array_equal(a[k], b[k]), k
+
+
+# the sizes nearest the line between four lanes and one
+@pytest.mark.parametrize("side", [31, 32])
+def test_step_equals_phases_and_oracle_at_the_line(upf_lib, oracle_lib, side):
+    test_step_equals_phases_and_oracle(upf_lib, oracle_lib, side, FLAG_SURFACE_TENSION, 7)

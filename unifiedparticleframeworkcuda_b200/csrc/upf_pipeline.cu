@@ -916,7 +916,9 @@ __device__ __forceinline__ void integrate_store(const DevParams& P, uint32_t i, 
 // thousands of particles a thread each leaves an SM a few warps, whose 30
 // entries of dependent gathers are the pass. The lanes' terms (pressure,
 // viscosity, with kSurface surface tension, per component) wait in shared
-// memory and are taken off in list order by a lane per component.
+// memory and are taken off in list order by a lane per component. With more
+// particles the warps hide the gathers, and the terms' way through shared
+// memory only adds to them (launch_integrate_phase).
 constexpr int kForceRows = 4;  // list entries a lane takes at a time
 template <int kLanes, bool kSurface>
 __global__ void __launch_bounds__(kBlock) k_wcsph_force_integrate(
@@ -2617,12 +2619,14 @@ inline uint32_t grid_of(uint32_t n) { return (n + kBlock - 1) / kBlock; }
 
 // ---- launches of the tunable passes at a LaunchShape
 // Particles a warp of the list build takes. More share the cell look-up and
-// write longer rows (at 1,048,576 particles 0.79 ms with 32, 0.87 with 16);
-// fewer leave more warps (at 32,768 0.062 ms with 8, 0.075 with 4 and 0.063
-// with 16; at 262,144 16 and 32 are level, and 16 has the shorter last wave).
-// nlist_mode 1 halves the number.
+// write longer rows; fewer leave more warps. The lines lie where two
+// neighbouring choices are level: 4 and 8 a warp at 8,000 particles 33.7 and
+// 35.8 us, at 16,250 42.0 and 39.9; 8 and 16 at 27,000 48.1 and 50.0, at 32,768
+// 56.3 and 52.2 (WCSPH steps: 88.2 and 90.6, 95.4 and 90.6); 16 and 32 at
+// 327,680 279.6 and 281.5, at 384,000 326.6 and 322.6 (at 1,048,576 839 and
+// 777). nlist_mode 1 halves the number.
 inline int nlist_warp_particles(const LaunchShape& sh, uint32_t n) {
-  const int w = n >= 524288 ? 32 : (n >= 65536 ? 16 : (n >= 16384 ? 8 : 4));
+  const int w = n >= 360000 ? 32 : (n >= 30000 ? 16 : (n >= 16384 ? 8 : 4));
   return sh.nlist_mode == 1 && w > 4 ? w / 2 : w;
 }
 
@@ -3043,12 +3047,14 @@ cudaError_t launch_integrate_phase(System& s, cudaStream_t st, const LoopTurn& t
   const uint32_t n = s.n_dyn;
   if (n == 0) return cudaSuccess;
   if (s.prm.method == UPF_METHOD_WCSPH) {
-    // four lanes a particle while they all find room on the SMs at once
+    // four lanes a particle where one would leave an SM too few warps to hide
+    // the gathers: steps of 17,576 particles 72 us with four and 78 with one, of
+    // 27,000 84 and 88; of 32,768 98 and 96, of 64,000 142 and 131
 #define UPF_WF(L, S)                                                                                             \
   k_wcsph_force_integrate<L, S><<<(uint32_t)(((uint64_t)n * L + kBlock - 1) / kBlock), kBlock, 0, st>>>(           \
       s.dp, n, s.B, s.A, s.keysA, s.nbr, s.lval, s.ncnt, s.luts, s.rho, s.press, s.pq, s.xs, s.force, s.st)
     const bool surface = s.prm.flags & UPF_FLAG_SURFACE_TENSION;
-    if (n <= 65536) {
+    if (n < 30000) {
       if (surface) UPF_WF(4, true);
       else UPF_WF(4, false);
     } else {
