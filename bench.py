@@ -1127,17 +1127,18 @@ def run_ours(args, rank, world, local_rank):
     achieved = kbytes / (kms / 1e3) / 1e9
     step_bytes = algorithmic_bytes(nf, nb, args.steps, total_iters, method)
     # DRAM bytes per fluid particle per launch, measured by ncu captures of
-    # the same kernels on the 262k-fluid dam (read + write, one launch) and
-    # scaled here by the fluid count (the list length per particle does not
+    # the same kernels (read + write, one launch; the plain passes on the
+    # 262k-fluid dam, the staged ones on a dam of 524,288) and scaled here by
+    # the fluid count (the list length per particle does not
     # depend on the scene size); not measured in this run. Keyed by the list
     # mode the tuned shape reads: staged neighbourhoods (mode 2) stream
     # 16-bit union positions in place of 32-bit list entries
     staged = (tuned.get("density_mode" if kname == "k_pcisph_density" else "pforce_mode") == 2)
-    traffic_per_particle = {("k_pcisph_density", False): 157.9, ("k_pcisph_density", True): 110.7,
-                            ("k_pcisph_pressure_force", False): 361.2, ("k_pcisph_pressure_force", True): 280.8}
+    traffic_per_particle = {("k_pcisph_density", False): 158.5, ("k_pcisph_density", True): 109.1,
+                            ("k_pcisph_pressure_force", False): 341.8, ("k_pcisph_pressure_force", True): 299.8}
     traffic = traffic_per_particle[(kname, staged)] * nf if (kname, staged) in traffic_per_particle else None
-    traffic_source = ("ncu dram__bytes_read+write per fluid particle on the 262k-fluid dam, scaled to %d fluid "
-                      "particles" % nf) if traffic is not None else None
+    traffic_source = ("ncu dram__bytes_read+write per fluid particle on a dam of %s, scaled to %d fluid "
+                      "particles" % ("524,288" if staged else "262,144", nf)) if traffic is not None else None
 
     # end to end through the C ABI with host buffers, over the same steps as
     # the timed region (restored from the checkpoint): every step uploads its

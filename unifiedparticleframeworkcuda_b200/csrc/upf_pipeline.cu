@@ -506,15 +506,16 @@ __global__ void __launch_bounds__(kBlock) k_merged_positions(uint32_t n, uint32_
 // memory. At the end lane p turns particle p's words into its list: all lanes
 // write entry after entry, so the column-major rows leave as runs of kW
 // words.
-// Bound: instruction issue (630 warp instructions a particle). On a dam one
+// Bound: instruction issue (71% of it at 262,144; 650 warp instructions a
+// particle at 1,048,576, 740 at 262,144). On a dam one
 // particle's cells are 14 chunks, the cells of four 26, of eight 34: with 9
 // instructions a test and about 10 a chunk, four together come cheapest. Held
 // to 64 registers (eight 128-thread CTAs an SM; at 80 0.98 against 0.93 ms a
 // build of the dam from rest, at 48 it spills).
 // A thread per particle, as before, had its lanes in different cells (10.7 of
 // 32 active, 950 warp instructions a particle). Builds from rest, before and
-// now: 1,048,576 + 279,308 boundary particles 1.01 and 0.79 ms, 262,144 0.376
-// and 0.245, 32,768 (WCSPH) 0.134 and 0.062, 256 scenes 4.72 and 3.43.
+// now: 1,048,576 + 279,308 boundary particles 1.01 and 0.79 ms, 262,144 0.37
+// and 0.24, 32,768 (WCSPH) 0.132 and 0.050, 256 scenes 4.72 and 3.47.
 constexpr int kNlistTogether = 4;
 constexpr uint32_t kNlistWords = 16;  // words of accepted bits held per particle
 template <int kW>
@@ -2030,10 +2031,13 @@ __global__ void k_loop_ctl(DevParams P, DevState* st, cudaGraphConditionalHandle
 // graph nodes is mostly the nodes: their launches, drains and cold starts,
 // and gathers with few warps to hide them. A step of 50 iterations, before
 // and now (sort, lists and forces included, about 0.1 ms): 1,728 particles
-// 1.15 and 0.34 ms, 8,000 1.31 and 0.48, 33,792 1.31 and 0.77, 53,157 1.44
-// and 0.89, 109,200 1.74 and 1.15, 136,192 2.0 and 1.40. Above that several chunks a CTA came to
-// 2.87 ms at 196,608 against 2.73 with the passes as launches of their own
-// (3.45 and 3.23 at 262,144), so those keep the launches.
+// 1.28 and 0.33 ms, 8,000 1.32 and 0.45, 33,792 1.37 and 0.76, 53,157 1.52
+// and 0.88, 109,200 1.85 and 1.14, 136,192 2.19 and 1.39. What bounds it: at
+// 1,728 the barriers (13% of issue, most stalls there), at 53,157 the gathers
+// and the barriers alike (56% of the load pipe's wavefronts, 38% of issue).
+// Above that several chunks a CTA came to 2.87 ms at 196,608 against 2.73 with
+// the passes as launches of their own (3.45 and 3.23 at 262,144), so those keep
+// the launches.
 // kLanes: lanes a particle. With few particles one thread each leaves an SM a
 // warp or two, and an iteration is their 3,000 instructions one after the
 // other; instead kLanes lanes compute the terms of every kLanes-th list entry
@@ -2891,15 +2895,15 @@ cudaError_t launch_loop_init(System& s, cudaStream_t st) {
 
 // The fused loop's shape for n particles (or slots): as many lanes a particle
 // as the SMs hold at once, at 768 threads of 80 registers each in CTAs of 256
-// (steps of 50 iterations of 4,096, 8,000, 21,952 particles 0.400, 0.494 and
-// 0.642 ms, at 1,024 threads of 64 in CTAs of 512 0.417, 0.512 and 0.732, in
-// CTAs of 128 longer by half: the barrier's cost is its arrivals); where 1,024
-// hold twice the lanes, those (33,792: 0.773 with four lanes, 0.881 with two).
-// One lane at 768 threads an SM instead of CTAs of 128 with eight rows: 62,400
-// 0.942 and 1.140, 109,200 1.160 and 1.354. Lists are held in shared memory by
-// the smallest scenes alone, where it hides latency (1,728: 0.340, 0.363
-// without); with more lists an SM the shared memory is worth more as L1 for
-// the gathers (8,000: 0.495 held and 0.476, 53,157: 0.951 and 0.891).
+// (steps of 50 iterations of 4,096, 8,000, 21,952 particles take 4, 4 and 14%
+// longer at 1,024 threads of 64 in CTAs of 512, half as long again in CTAs of
+// 128: the barrier's cost is its arrivals); where 1,024 hold twice the lanes,
+// those (33,792: 14% longer with two lanes than with four). One lane at 768
+// threads an SM instead of CTAs of 128 with eight rows, which take 21% longer
+// at 62,400 and 17% at 109,200. Lists are held in shared memory by the
+// smallest scenes alone, where it hides latency (1,728: 7% longer without);
+// with more lists an SM the shared memory is worth more as L1 for the gathers
+// (held, 8,000 take 4% longer, 53,157 7%).
 template <bool kBatch, int kThreads, int kResident, int kLanes, int kHeld, int kRows>
 static cudaError_t run_loop_shape(cudaStream_t st, uint32_t n, void** args) {
   constexpr uint32_t chunk = kThreads / kLanes;
