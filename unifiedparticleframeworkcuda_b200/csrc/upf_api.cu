@@ -780,9 +780,9 @@ upf_status upf_test_meet_others(upf_system* s) {
     set_error("upf_test_meet_others: null");
     return UPF_ERR_INVALID_ARG;
   }
-  const unsigned long long seen = 2;
+  const unsigned long long met = 1;
   UPF_CUDA(cudaStreamSynchronize(s->stream));
-  UPF_CUDA(cudaMemcpy(s->loop_sync + 2, &seen, sizeof(seen), cudaMemcpyHostToDevice));
+  UPF_CUDA(cudaMemcpy(s->loop_sync + 2, &met, sizeof(met), cudaMemcpyHostToDevice));
   *s->crowd_host = 1;
   return UPF_OK;
 }
@@ -976,7 +976,7 @@ upf_status upf_create(const upf_params* p, int device, uint32_t capacity, upf_sy
   ALLOC(s->mpos, c);
   ALLOC(s->spos, c); ALLOC(s->skeys, c); ALLOC(s->sid, c);
   ALLOC(s->luts, 5 * UPF_LUT_ENTRIES + kThresholds);
-  ALLOC(s->st, 1); ALLOC(s->loop_sync, 3); ALLOC(s->loop_max, 2);
+  ALLOC(s->st, 1); ALLOC(s->loop_sync, 4); ALLOC(s->loop_max, 2);
   s->loop_sms = loop_cooperative_sms();
   if (p->method == UPF_METHOD_PCISPH) {
     // staged neighbourhoods of the loop passes (loop-pass mode 2)
@@ -1009,7 +1009,7 @@ upf_status upf_create(const upf_params* p, int device, uint32_t capacity, upf_sy
   if (e == cudaSuccess && s->ucount)
     e = cudaMemset(s->ucount, 0xff, sizeof(uint32_t) * (((size_t)c + kStageChunk - 1) / kStageChunk));
   if (e == cudaSuccess) e = cudaMemset(s->st, 0, sizeof(DevState));
-  if (e == cudaSuccess) e = cudaMemset(s->loop_sync, 0, sizeof(unsigned long long) * 3);
+  if (e == cudaSuccess) e = cudaMemset(s->loop_sync, 0, sizeof(unsigned long long) * 4);
   if (e != cudaSuccess) {
     set_error("upload: %s", cudaGetErrorString(e));
     return bail(UPF_ERR_CUDA);

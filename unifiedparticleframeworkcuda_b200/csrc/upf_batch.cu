@@ -294,7 +294,7 @@ upf_status upf_batch_create(const upf_params* params, const uint32_t* counts, ui
   ALLOC(b->st_d, num_scenes);
   ALLOC(b->group_scene_d, group_scene.size()); ALLOC(b->seg_begin_d, num_scenes); ALLOC(b->seg_end_d, num_scenes);
   ALLOC(b->cell_base_d, num_scenes); ALLOC(b->any_active_d, 1);
-  ALLOC(b->loop_sync, 3); ALLOC(b->loop_max, (size_t)2 * num_scenes);
+  ALLOC(b->loop_sync, 4); ALLOC(b->loop_max, (size_t)2 * num_scenes);
   b->loop_sms = loop_cooperative_sms();
   ALLOC(b->active_groups_d, n / kSegAlign + 1); ALLOC(b->n_active_groups_d, 1);
   ALLOC(b->x.comp_begin_d, num_scenes); ALLOC(b->x.stage_a, std::max<size_t>(total, 1));
@@ -333,7 +333,7 @@ upf_status upf_batch_create(const upf_params* params, const uint32_t* counts, ui
   if (e == cudaSuccess)
     e = cudaMemcpy(b->x.comp_begin_d, comp_begin.data(), sizeof(uint32_t) * num_scenes, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemset(b->st_d, 0, sizeof(DevState) * num_scenes);
-  if (e == cudaSuccess) e = cudaMemset(b->loop_sync, 0, sizeof(unsigned long long) * 3);
+  if (e == cudaSuccess) e = cudaMemset(b->loop_sync, 0, sizeof(unsigned long long) * 4);
   if (e == cudaSuccess) e = cudaMemset(b->A.type, 0xff, sizeof(int32_t) * n);  // padding: no type
   if (e == cudaSuccess) e = cudaMemset(b->A.pos, 0, sizeof(float4) * n);
   if (e == cudaSuccess) e = cudaMemset(b->A.vel, 0, sizeof(float4) * n);
@@ -685,9 +685,9 @@ upf_status upf_test_batch_meet_others(upf_batch* b) {
     set_error("upf_test_batch_meet_others: null");
     return UPF_ERR_INVALID_ARG;
   }
-  const unsigned long long seen = 2;
+  const unsigned long long met = 1;
   UPF_CUDA(cudaStreamSynchronize(b->stream));
-  UPF_CUDA(cudaMemcpy(b->loop_sync + 2, &seen, sizeof(seen), cudaMemcpyHostToDevice));
+  UPF_CUDA(cudaMemcpy(b->loop_sync + 2, &met, sizeof(met), cudaMemcpyHostToDevice));
   *b->crowd_host = 1;
   return UPF_OK;
 }

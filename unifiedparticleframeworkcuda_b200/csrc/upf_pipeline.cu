@@ -360,24 +360,31 @@ struct StepStart {
 // 4.5, 2.6 and 3.3; of 53,157 6.5, 4.5 and 5.1. Alone and in pairs the one
 // launch is the faster (8,000: 0.45 and 0.85 ms against 0.95 and 1.07). So a
 // step takes the passes where at least two other loops are in flight when it
-// begins, or were when its last one ended (steps that begin together see one
-// another only then). Either form gives the same results.
+// begins, or three were at some time during its last one (of three steps that
+// begin together only the third sees two others at its beginning). Either form
+// gives the same results.
 // A step's choice costs a conditional node, 15 us; a graph without one tells
 // the host when it has met two others (LoopTurn), and the handle then takes a
 // graph with both forms. A program with one or two systems pays nothing.
-__device__ uint32_t g_loops_in_flight = 0;
 constexpr uint32_t kLoopsBeside = 2;
+__device__ uint32_t g_loops_in_flight = 0;
+__device__ unsigned long long g_loops_entered = 0;  // since the library was loaded
+__device__ unsigned long long g_last_crowd = 0;     // the latest to enter beside two others, by that count
 __device__ __forceinline__ void enter_loop(const LoopTurn& turn, cudaGraphConditionalHandle route) {
-  const uint32_t beside = max(atomicAdd(&g_loops_in_flight, 1u), (uint32_t)*turn.seen);
+  const bool crowd = atomicAdd(&g_loops_in_flight, 1u) >= kLoopsBeside;
+  const unsigned long long entry = atomicAdd(&g_loops_entered, 1ull) + 1;
+  if (crowd) atomicMax(&g_last_crowd, entry);
+  turn.words[1] = entry;
   if (route)
-    cudaGraphSetConditional(route, beside < kLoopsBeside ? 1u : 0u);
-  else if (beside >= kLoopsBeside)
+    cudaGraphSetConditional(route, crowd || turn.words[0] ? 0u : 1u);
+  else if (crowd)
     *reinterpret_cast<volatile uint32_t*>(turn.crowd) = 1;
 }
 __device__ __forceinline__ void leave_loop(const LoopTurn& turn) {
-  const uint32_t beside = atomicSub(&g_loops_in_flight, 1u) - 1u;
-  *turn.seen = beside;
-  if (beside >= kLoopsBeside) *reinterpret_cast<volatile uint32_t*>(turn.crowd) = 1;
+  const bool crowd = atomicMax(&g_last_crowd, 0ull) >= turn.words[1];
+  atomicSub(&g_loops_in_flight, 1u);
+  turn.words[0] = crowd;
+  if (crowd) *reinterpret_cast<volatile uint32_t*>(turn.crowd) = 1;
 }
 
 __device__ __forceinline__ void step_init(DevState* st, int count_step) {
@@ -419,7 +426,7 @@ __global__ void __launch_bounds__(kBlock) k_reorder(
   if (t == 0 && start.st) {
     step_init(start.st, start.count_step);
     if (start.sync) loop_init(start.st, start.sync, start.loop_max);
-    if (start.turn.seen) enter_loop(start.turn, start.route);
+    if (start.turn.words) enter_loop(start.turn, start.route);
   }
   if (t >= n + ns) return;
   const bool dyn = t < n;
@@ -2407,7 +2414,7 @@ __global__ void k_loop_init_batch(DevState* st, uint32_t nscenes, int32_t* any_a
                                   unsigned long long* sync, uint32_t* loop_max, const LoopTurn turn,
                                   cudaGraphConditionalHandle route) {
   if (threadIdx.x == 0) {
-    if (turn.seen) enter_loop(turn, route);
+    if (turn.words) enter_loop(turn, route);
     sync[0] = 0;        // arrivals at the fused loop's barrier
     sync[1] = nscenes;  // scenes whose loop still runs
   }
@@ -2495,7 +2502,7 @@ __global__ void __launch_bounds__(kBlock) k_pcisph_integrate(
     const float* __restrict__ rho, const float* __restrict__ press, DevState* __restrict__ st_plain,
     const LoopTurn turn) {
   __shared__ DevParams sP;
-  if (turn.seen && blockIdx.x == 0 && threadIdx.x == 0) leave_loop(turn);
+  if (turn.words && blockIdx.x == 0 && threadIdx.x == 0) leave_loop(turn);
   const Scope sc = enter_scope<kBatch>(Pk, nullptr, st_plain, n, bv, &sP, false);
   if (kBatch) __syncthreads();
   const DevParams& P = *sc.P;

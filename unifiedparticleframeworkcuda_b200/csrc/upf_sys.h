@@ -147,10 +147,10 @@ struct FrameIO {
 cudaError_t frame_streams_create(FrameIO& io, cudaStream_t compute);
 void frame_streams_destroy(FrameIO& io);  // waits for the copies; buffers stay with their owner
 
-// A step's turn among the device's one-launch loops (enter_loop): the loops
-// seen beside the last one, and the host's word for having met two others.
+// A step's turn among the device's one-launch loops (enter_loop): whether the
+// last step met two others, this one's number, and the host's word for it.
 struct LoopTurn {
-  unsigned long long* seen = nullptr;  // null: not counted
+  unsigned long long* words = nullptr;  // [2]; null: not counted
   uint32_t* crowd = nullptr;
 };
 
@@ -235,7 +235,7 @@ struct System {
   cudaGraph_t step_graph = nullptr;
   int key_bits = 30;
   // the predict-correct loop as one cooperative launch (k_pcisph_loop)
-  unsigned long long* loop_sync = nullptr;  // [2] its barrier, the loops seen beside the last one (leave_loop)
+  unsigned long long* loop_sync = nullptr;  // [2] its barrier, [2] LoopTurn
   uint32_t* loop_max = nullptr;   // [2] the maximum predicted density of odd and even iterations
   uint32_t loop_sms = 0;          // the device's SMs (0: no cooperative launches)
   bool shape_set = false;         // the caller set the passes' shapes: the loop's run as launches of their own
@@ -307,7 +307,7 @@ struct BatchSystem {
   uint32_t* active_groups_d = nullptr;  // [n_slots / kSegAlign] groups of the scenes still iterating
   uint32_t* n_active_groups_d = nullptr;
   uint32_t active_grid = 0;             // resident CTAs of the active-group passes
-  unsigned long long* loop_sync = nullptr;  // as System's: the fused loop's barrier, its running scenes, loops seen
+  unsigned long long* loop_sync = nullptr;  // as System's: the fused loop's barrier, its running scenes, LoopTurn
   uint32_t* loop_max = nullptr;             // [scenes][2]
   uint32_t loop_sms = 0;
   bool shape_set = false;                   // as System's
