@@ -538,17 +538,18 @@ upf_status upf_profile_step(upf_system* s, upf_phase_times* out);
  * 256) an SM, 151,552 on a B200, or the passes' launches while at least two
  * other such loops are in flight on the device (on streams of their own: the
  * passes of several fill one another's gaps, launches of the whole loop queue;
- * up to 12 an SM they fit beside one another and stay). Above that, a single
- * system's passes run from staged neighbourhoods (mode 2, 256 threads, 4
- * rows), a batch's at the shapes that upf_batch_get_launch_config reports. Any
- * successful upf_set_launch_config is a choice, also of the values that were
- * reported: from then on the loop's passes run as launches of their own at
- * those shapes. upf_autotune gives the choice back: up to 1,024 particles an
- * SM the loop is one launch again, above it the passes run at the tuned
- * shapes. A tuned config set in another handle is a choice there, and so ends
- * the one-launch loop of a small one (1,728 particles: 0.33 ms a step of 50
- * iterations in one launch, 0.89 with passes); tune each handle, or leave it
- * as it is. */
+ * up to 12 an SM they fit beside one another and stay). In calls of fewer than
+ * 16 steps a handle makes that choice once it has met others, from its next
+ * call on. Above 1,024 an SM, a single system's passes run from staged
+ * neighbourhoods (mode 2, 256 threads, 4 rows), a batch's at the shapes that
+ * upf_batch_get_launch_config reports. Any successful upf_set_launch_config is
+ * a choice, also of the values that were reported: from then on the loop's
+ * passes run as launches of their own at those shapes. upf_autotune gives the
+ * choice back: up to 1,024 particles an SM the loop is one launch again, above
+ * it the passes run at the tuned shapes. A tuned config set in another handle
+ * is a choice there, and so ends the one-launch loop of a small one (1,728
+ * particles: 0.33 ms a step of 50 iterations in one launch, 0.89 with passes);
+ * tune each handle, or leave it as it is. */
 typedef struct upf_launch_config {
   int32_t nlist_threads;      /* 64, 128, 256 */
   int32_t external_threads;   /* 128, 256 */

@@ -140,6 +140,26 @@ def test_a_batch_beside_others(upf_lib):
         same(end_state(b, 4), end_state(a, 4))
 
 
+def test_a_call_of_many_steps(upf_lib):
+    """As many calls of one step, for a system and a batch; then short calls."""
+    sc = scenes.pcisph_dam(20, 18, 16, seed=6, box=(0.3, 0.25, 0.25))
+    with system(upf_lib, sc) as s, system(upf_lib, sc) as t:
+        for _ in range(19):
+            s.step(1)
+        t.step(17)
+        assert route(upf_lib, t) == EITHER and route(upf_lib, s) == ONE_LAUNCH
+        t.step(2)
+        same(end_state(t, 0), end_state(s, 0))
+    scs = scenes.batch_scenes(num=3, seed=13, counts=(2048, 4096))
+    with upf_lib.ParticleBatch.from_scenes(scs) as a, upf_lib.ParticleBatch.from_scenes(scs) as b:
+        for _ in range(17):
+            a.step(1)
+        b.step(16)
+        b.step(1)
+        assert route(upf_lib, b) == EITHER
+        same(end_state(b, 3), end_state(a, 3))
+
+
 def test_the_smallest_system_does_not_yield(upf_lib):
     with system(upf_lib, scenes.small_pcisph()) as s:
         upf_lib.check(upf_lib.lib().upf_test_meet_others(s.handle), "upf_test_meet_others")

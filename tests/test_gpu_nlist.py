@@ -94,9 +94,9 @@ def test_particles_a_warp_do_not_change_the_lists(upf_lib, n):
         assert np.array_equal(u, v)
 
 
-@pytest.mark.parametrize("n", [29999, 30000, 360000])
+@pytest.mark.parametrize("n", [29999, 30000])
 def test_counts_at_which_a_warp_takes_more(upf_lib, n):
-    """Likewise at the counts where the number doubles, and below one."""
+    """Likewise on both sides of the count where it takes 16."""
     test_particles_a_warp_do_not_change_the_lists(upf_lib, n)
 
 

@@ -437,11 +437,14 @@ static cudaError_t capture_body(cudaGraph_t body, Fn&& fn) {
   return e;
 }
 
-// Whether the steps of a handle have met others since its graph was built for
-// itself alone. (Not while its stream is being captured: the graph in use is
-// then the caller's.)
-bool met_others(const uint32_t* crowd_host, bool crowded, cudaStream_t st) {
-  if (crowded || !*reinterpret_cast<const volatile uint32_t*>(crowd_host)) return false;
+// Whether a call of nsteps takes the graph with both forms of the loop (built
+// at its first use): once a step of the handle has met others, and in calls of
+// many steps, whose launches are all made before the first of them can tell.
+// Not built while the stream is being captured.
+bool takes_both(const uint32_t* crowd_host, int32_t nsteps, bool built, cudaStream_t st) {
+  constexpr int32_t kManySteps = 16;
+  if (nsteps < kManySteps && !*reinterpret_cast<const volatile uint32_t*>(crowd_host)) return false;
+  if (built) return true;
   cudaStreamCaptureStatus capturing;
   if (cudaStreamIsCapturing(st, &capturing) == cudaSuccess) return capturing == cudaStreamCaptureStatusNone;
   cudaGetLastError();
@@ -515,19 +518,23 @@ upf_status capture_step_graph(const GraphParts& parts, cudaGraph_t* graph_out, c
 namespace {
 
 void destroy_graph(System& s) {
-  if (s.step_exec) cudaGraphExecDestroy(s.step_exec);
-  if (s.step_graph) cudaGraphDestroy(s.step_graph);
-  s.step_exec = nullptr;
-  s.step_graph = nullptr;
+  for (cudaGraphExec_t* e : {&s.step_exec, &s.both_exec}) {
+    if (*e) cudaGraphExecDestroy(*e);
+    *e = nullptr;
+  }
+  for (cudaGraph_t* g : {&s.step_graph, &s.both_graph}) {
+    if (*g) cudaGraphDestroy(*g);
+    *g = nullptr;
+  }
 }
 
 LoopTurn turn_of(const System& s) { return s.loop_yields ? LoopTurn{s.loop_sync + 2, s.crowd_host} : LoopTurn{}; }
 
 // One step of a system: sort -> neighbours -> forces -> loop -> integrate. The
 // loop is a while-node over its passes, one launch, or the device's choice of
-// the two (enter_loop).
-upf_status build_step_graph(System& s) {
-  destroy_graph(s);
+// the two (enter_loop; `both`: that graph, beside the other).
+upf_status build_step_graph(System& s, bool both = false) {
+  if (!both) destroy_graph(s);
   GraphParts parts;
   parts.ctx = &s;
   parts.pre = [](void* c, cudaStream_t st, cudaGraphConditionalHandle route) {
@@ -540,7 +547,7 @@ upf_status build_step_graph(System& s) {
   };
   s.loop_in_graph = loop_fused(s);
   s.loop_yields = s.loop_in_graph && loop_yields(s.n_dyn, s.loop_sms);
-  s.loop_both = s.loop_yields && s.crowded;
+  s.loop_both = s.loop_yields && both;
   if (s.loop_both) {
     parts.one_launch = [](void* c, cudaStream_t st) { return launch_fused_loop(*static_cast<System*>(c), st); };
     parts.before_loop = [](void* c, cudaStream_t st) { return launch_loop_staging(*static_cast<System*>(c), st); };
@@ -558,14 +565,15 @@ upf_status build_step_graph(System& s) {
   // the host-side record of whether the current lists are staged is kept,
   // and whether a step of this graph stages them is noted for upf_step
   const bool staged_now = s.lists_staged;
-  const upf_status rc = capture_step_graph(parts, &s.step_graph, &s.step_exec);
+  const upf_status rc = capture_step_graph(parts, both ? &s.both_graph : &s.step_graph,
+                                           both ? &s.both_exec : &s.step_exec);
   s.graph_stages = s.lists_staged && !s.loop_in_graph;
+  s.graph_yields = s.loop_yields;
   const bool fused = s.loop_in_graph;
   s.loop_in_graph = s.loop_yields = s.loop_both = false;
   s.lists_staged = staged_now;
-  if (rc != UPF_OK && fused) {
-    // a share of the device (MPS) that does not hold the cooperative grid, or
-    // not in a conditional body: the passes
+  if (rc != UPF_OK && fused && !both) {
+    // a share of the device (MPS) that does not hold the cooperative grid: the passes
     cudaGetLastError();
     s.loop_sms = 0;
     return build_step_graph(s);
@@ -764,7 +772,7 @@ upf_status upf_test_loop_route(upf_system* s, int32_t* one_launch) {
     set_error("upf_test_loop_route: null");
     return UPF_ERR_INVALID_ARG;
   }
-  *one_launch = loop_fused(*s) ? 1 + (s->crowded && loop_yields(s->n_dyn, s->loop_sms)) : 0;
+  *one_launch = loop_fused(*s) ? 1 + (s->both_exec != nullptr) : 0;
   return UPF_OK;
 }
 
@@ -1294,13 +1302,20 @@ upf_status upf_step(upf_system* s, int32_t nsteps) {
     set_error("upf_step: call upf_set_particles first");
     return UPF_ERR_STATE;
   }
-  if (met_others(s->crowd_host, s->crowded, s->stream)) s->crowded = s->graph_stale = true;
   if (s->graph_stale) {
     UPF_TRY(build_step_graph(*s));
     s->graph_stale = false;
   }
   s->stepped = true;
-  for (int32_t k = 0; k < nsteps; ++k) UPF_CUDA(cudaGraphLaunch(s->step_exec, s->stream));
+  cudaGraphExec_t exec = s->step_exec;
+  if (s->graph_yields && takes_both(s->crowd_host, nsteps, s->both_exec != nullptr, s->stream)) {
+    if (!s->both_exec && build_step_graph(*s, true) != UPF_OK) {
+      cudaGetLastError();  // (as one launch, then)
+      s->graph_yields = false;
+    }
+    if (s->both_exec) exec = s->both_exec;
+  }
+  for (int32_t k = 0; k < nsteps; ++k) UPF_CUDA(cudaGraphLaunch(exec, s->stream));
   if (nsteps > 0) s->lists_staged = s->graph_stages;
   return UPF_OK;
 }

@@ -97,30 +97,34 @@ struct upf_batch : BatchSystem {
 namespace {
 
 void destroy_batch_graph(upf_batch* b) {
-  if (b->step_exec) cudaGraphExecDestroy(b->step_exec);
-  if (b->step_graph) cudaGraphDestroy(b->step_graph);
-  b->step_exec = nullptr;
-  b->step_graph = nullptr;
+  for (cudaGraphExec_t* e : {&b->step_exec, &b->both_exec}) {
+    if (*e) cudaGraphExecDestroy(*e);
+    *e = nullptr;
+  }
+  for (cudaGraph_t* g : {&b->step_graph, &b->both_graph}) {
+    if (*g) cudaGraphDestroy(*g);
+    *g = nullptr;
+  }
 }
 
 LoopTurn turn_of(const BatchSystem& b) {
   return b.loop_yields ? LoopTurn{b.loop_sync + 2, b.crowd_host} : LoopTurn{};
 }
 
-upf_status build_batch_graph(upf_batch* b) {
-  destroy_batch_graph(b);
+upf_status build_batch_graph(upf_batch* b, bool both = false) {
+  if (!both) destroy_batch_graph(b);
   GraphParts parts;
   parts.ctx = static_cast<BatchSystem*>(b);
   // the loop as in a system's graph (build_step_graph)
   const bool fused = batch_loop_fused(*b);
   b->loop_yields = fused && loop_yields(b->n_slots, b->loop_sms);
-  b->loop_both = b->loop_yields && b->crowded;
+  b->loop_both = b->loop_yields && both;
   parts.pre = [](void* c, cudaStream_t st, cudaGraphConditionalHandle route) {
     BatchSystem& B = *static_cast<BatchSystem*>(c);
-    cudaError_t e = batch_launch_sort(B, st);
+    cudaError_t e = batch_launch_sort(B, st, turn_of(B), route);
     if (e == cudaSuccess) e = batch_launch_neighbors(B, st);
     if (e == cudaSuccess) e = batch_launch_forces(B, st);
-    if (e == cudaSuccess) e = batch_launch_loop_init(B, st, turn_of(B), route);
+    if (e == cudaSuccess) e = batch_launch_loop_init(B, st);
     return e;
   };
   if (b->loop_both)
@@ -136,8 +140,9 @@ upf_status build_batch_graph(upf_batch* b) {
     cudaError_t e = batch_loop_fused(B) && !B.loop_both ? batch_launch_fused_loop(B, st) : cudaSuccess;
     return e == cudaSuccess ? batch_launch_integrate(B, st, turn_of(B)) : e;
   };
-  const upf_status rc = capture_step_graph(parts, &b->step_graph, &b->step_exec);
-  if (rc != UPF_OK && fused) {  // as build_step_graph
+  const upf_status rc = capture_step_graph(parts, both ? &b->both_graph : &b->step_graph,
+                                           both ? &b->both_exec : &b->step_exec);
+  if (rc != UPF_OK && fused && !both) {  // as build_step_graph
     cudaGetLastError();
     b->loop_sms = 0;
     return build_batch_graph(b);
@@ -428,11 +433,15 @@ upf_status upf_batch_step(upf_batch* b, int32_t nsteps) {
     set_error("upf_batch_step: negative step count");
     return UPF_ERR_INVALID_ARG;
   }
-  if (met_others(b->crowd_host, b->crowded, b->stream)) {
-    b->crowded = true;
-    UPF_TRY(build_batch_graph(b));
+  cudaGraphExec_t exec = b->step_exec;
+  if (b->loop_yields && takes_both(b->crowd_host, nsteps, b->both_exec != nullptr, b->stream)) {
+    if (!b->both_exec && build_batch_graph(b, true) != UPF_OK) {
+      cudaGetLastError();  // (as one launch, then)
+      b->loop_yields = false;
+    }
+    if (b->both_exec) exec = b->both_exec;
   }
-  for (int32_t k = 0; k < nsteps; ++k) UPF_CUDA(cudaGraphLaunch(b->step_exec, b->stream));
+  for (int32_t k = 0; k < nsteps; ++k) UPF_CUDA(cudaGraphLaunch(exec, b->stream));
   return UPF_OK;
 }
 
@@ -676,7 +685,7 @@ upf_status upf_test_batch_loop_route(upf_batch* b, int32_t* one_launch) {
     set_error("upf_test_batch_loop_route: null");
     return UPF_ERR_INVALID_ARG;
   }
-  *one_launch = batch_loop_fused(*b) ? 1 + (b->crowded && loop_yields(b->n_slots, b->loop_sms)) : 0;
+  *one_launch = batch_loop_fused(*b) ? 1 + (b->both_exec != nullptr) : 0;
   return UPF_OK;
 }
 

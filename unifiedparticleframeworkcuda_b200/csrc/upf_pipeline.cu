@@ -363,29 +363,43 @@ struct StepStart {
 // begins, or three were at some time during its last one (of three steps that
 // begin together only the third sees two others at its beginning). Either form
 // gives the same results.
-// A step's choice costs a conditional node, 15 us; a graph without one tells
-// the host when it has met two others (LoopTurn), and the handle then takes a
-// graph with both forms. A program with one or two systems pays nothing.
+// A step's choice costs a conditional node, 10 to 15 us, so there are two
+// graphs (takes_both): one without, whose steps tell the host when they have
+// met two others (LoopTurn), and one with both forms for the calls after that
+// and for calls of many steps. (The whole loop's launch, which returns at once
+// where it is not wanted, before a while-node that is mostly skipped: 8 to 10 us.)
 constexpr uint32_t kLoopsBeside = 2;
 __device__ uint32_t g_loops_in_flight = 0;
 __device__ unsigned long long g_loops_entered = 0;  // since the library was loaded
 __device__ unsigned long long g_last_crowd = 0;     // the latest to enter beside two others, by that count
+// (by a warp that has nothing else to do: two round trips to the L2)
 __device__ __forceinline__ void enter_loop(const LoopTurn& turn, cudaGraphConditionalHandle route) {
-  const bool crowd = atomicAdd(&g_loops_in_flight, 1u) >= kLoopsBeside;
+  const unsigned long long met = turn.words[0];
+  const uint32_t beside = atomicAdd(&g_loops_in_flight, 1u);
   const unsigned long long entry = atomicAdd(&g_loops_entered, 1ull) + 1;
-  if (crowd) atomicMax(&g_last_crowd, entry);
+  const bool crowd = beside >= kLoopsBeside;
   turn.words[1] = entry;
+  if (crowd) atomicMax(&g_last_crowd, entry);
   if (route)
-    cudaGraphSetConditional(route, crowd || turn.words[0] ? 0u : 1u);
+    cudaGraphSetConditional(route, crowd || met ? 0u : 1u);
   else if (crowd)
     *reinterpret_cast<volatile uint32_t*>(turn.crowd) = 1;
 }
-__device__ __forceinline__ void leave_loop(const LoopTurn& turn) {
-  const bool crowd = atomicMax(&g_last_crowd, 0ull) >= turn.words[1];
-  atomicSub(&g_loops_in_flight, 1u);
-  turn.words[0] = crowd;
-  if (crowd) *reinterpret_cast<volatile uint32_t*>(turn.crowd) = 1;
-}
+// The loop is done: the loads that tell whether it met others are under way
+// while the caller works, and met() takes them.
+struct LeftLoop {
+  unsigned long long last = 0, entry = 1;
+  __device__ __forceinline__ void leave(const LoopTurn& turn) {
+    last = *reinterpret_cast<volatile unsigned long long*>(&g_last_crowd);
+    entry = turn.words[1];
+    atomicSub(&g_loops_in_flight, 1u);
+  }
+  __device__ __forceinline__ void met(const LoopTurn& turn) const {
+    const bool crowd = last >= entry;
+    turn.words[0] = crowd;
+    if (crowd) *reinterpret_cast<volatile uint32_t*>(turn.crowd) = 1;
+  }
+};
 
 __device__ __forceinline__ void step_init(DevState* st, int count_step) {
   st->ke = 0;
@@ -426,9 +440,11 @@ __global__ void __launch_bounds__(kBlock) k_reorder(
   if (t == 0 && start.st) {
     step_init(start.st, start.count_step);
     if (start.sync) loop_init(start.st, start.sync, start.loop_max);
-    if (start.turn.words) enter_loop(start.turn, start.route);
   }
-  if (t >= n + ns) return;
+  if (t >= n + ns) {
+    if (start.turn.words && t == ((n + ns + 31) & ~31u)) enter_loop(start.turn, start.route);
+    return;
+  }
   const bool dyn = t < n;
   const uint32_t j = dyn ? t : t - n;  // place in the own set
   const uint32_t* __restrict__ own = dyn ? keys : skeys;
@@ -2369,9 +2385,13 @@ __global__ void __launch_bounds__(kBlock) k_scene_digits(uint32_t nslots, const 
 // (the scene's Morton key of the gathered position; kPadKey for padding).
 __global__ void __launch_bounds__(kBlock) k_reorder_batch(const BatchView bv, uint32_t nslots,
                                                            const uint32_t* __restrict__ perm, DynArrays A,
-                                                           DynArrays B, uint32_t* __restrict__ keys) {
+                                                           DynArrays B, uint32_t* __restrict__ keys,
+                                                           const LoopTurn turn, cudaGraphConditionalHandle route) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nslots) return;
+  if (i >= nslots) {  // (a CTA of its own: the slots are whole CTAs)
+    if (turn.words && i == nslots) enter_loop(turn, route);
+    return;
+  }
   const uint32_t j = perm[i];
   const float4 x = A.pos[j];
   B.pos[i] = x;
@@ -2411,10 +2431,8 @@ __global__ void k_step_init_batch(DevState* st, uint32_t nscenes) {
 }
 
 __global__ void k_loop_init_batch(DevState* st, uint32_t nscenes, int32_t* any_active,
-                                  unsigned long long* sync, uint32_t* loop_max, const LoopTurn turn,
-                                  cudaGraphConditionalHandle route) {
+                                  unsigned long long* sync, uint32_t* loop_max) {
   if (threadIdx.x == 0) {
-    if (turn.words) enter_loop(turn, route);
     sync[0] = 0;        // arrivals at the fused loop's barrier
     sync[1] = nscenes;  // scenes whose loop still runs
   }
@@ -2502,7 +2520,9 @@ __global__ void __launch_bounds__(kBlock) k_pcisph_integrate(
     const float* __restrict__ rho, const float* __restrict__ press, DevState* __restrict__ st_plain,
     const LoopTurn turn) {
   __shared__ DevParams sP;
-  if (turn.words && blockIdx.x == 0 && threadIdx.x == 0) leave_loop(turn);
+  const bool leaves = turn.words && blockIdx.x == 0 && threadIdx.x == 0;
+  LeftLoop left;
+  if (leaves) left.leave(turn);
   const Scope sc = enter_scope<kBatch>(Pk, nullptr, st_plain, n, bv, &sP, false);
   if (kBatch) __syncthreads();
   const DevParams& P = *sc.P;
@@ -2538,6 +2558,7 @@ __global__ void __launch_bounds__(kBlock) k_pcisph_integrate(
   } else if (kBatch && i < n) {
     keysA[i] = kPadKeyBatch;  // padding slots sort after the scene's particles
   }
+  if (leaves) left.met(turn);
   if (!(ke == ke)) {
     atomicOr(&st->error_flags, (uint32_t)ERR_NAN);
     ke = 0;
@@ -2633,11 +2654,14 @@ inline uint32_t grid_of(uint32_t n) { return (n + kBlock - 1) / kBlock; }
 // write longer rows; fewer leave more warps. The lines lie where two
 // neighbouring choices are level: 4 and 8 a warp at 8,000 particles 33.7 and
 // 35.8 us, at 16,250 42.0 and 39.9; 8 and 16 at 27,000 48.1 and 50.0, at 32,768
-// 56.3 and 52.2 (WCSPH steps: 88.2 and 90.6, 95.4 and 90.6); 16 and 32 at
-// 327,680 279.6 and 281.5, at 384,000 326.6 and 322.6 (at 1,048,576 839 and
-// 777). nlist_mode 1 halves the number.
-inline int nlist_warp_particles(const LaunchShape& sh, uint32_t n) {
-  const int w = n >= 360000 ? 32 : (n >= 30000 ? 16 : (n >= 16384 ? 8 : 4));
+// 56.3 and 52.2 (WCSPH steps: 88.2 and 90.6, 95.4 and 90.6). A batch's scenes
+// bend the order of a warp's particles and differ in their cells: 8 and 16 at
+// 37,120 slots 66.5 and 74.8, at 45,312 46.1 and 52.2 or 66.5 and 62.3, at
+// 67,328 80.9 and 72.6. 16 and 32 are level from 262,144 (230 and 235) on in a
+// dam, at 670,208 slots in a batch (521 and 527; 374,272: 269 and 298), and at
+// 1,048,576 particles 839 and 777. nlist_mode 1 halves the number.
+inline int nlist_warp_particles(const LaunchShape& sh, uint32_t n, bool batch) {
+  const int w = n >= 524288 ? 32 : (n >= (batch ? 65536u : 30000u) ? 16 : (n >= 16384 ? 8 : 4));
   return sh.nlist_mode == 1 && w > 4 ? w / 2 : w;
 }
 
@@ -2650,7 +2674,7 @@ cudaError_t run_nlist(const LaunchShape& sh, cudaStream_t st, const DevParams& P
   k_build_nlist<kBatch, kMerged, kWcsph, T, W><<<(n + T / 32 * W - 1) / (T / 32 * W), T, nlist_smem<T, W>(), st>>>(P, bv, n, pos, mpos,  \
                                                                                         cstart, cend, nbr, lval, \
                                                                                         ncnt, luts, stp, wc)
-  switch (sh.nlist_threads * 100 + nlist_warp_particles(sh, n)) {
+  switch (sh.nlist_threads * 100 + nlist_warp_particles(sh, n, kBatch)) {
     case 6404: UPF_NL(64, 4); break;
     case 6408: UPF_NL(64, 8); break;
     case 6416: UPF_NL(64, 16); break;
@@ -2797,7 +2821,9 @@ cudaError_t launch_sort_phase(System& s, cudaStream_t st, bool starts_step, cons
   const bool pcisph = s.prm.method == UPF_METHOD_PCISPH;
   if (starts_step)
     start = StepStart{s.st, pcisph ? s.loop_sync : nullptr, s.loop_max, pcisph ? 0 : 1, turn, route};
-  k_reorder<<<grid_of(n + s.n_static), kBlock, 0, st>>>(
+  // (with a warp behind the particles that enters the loop)
+  const uint32_t threads = ((n + s.n_static + 31) & ~31u) + (start.turn.words ? 1 : 0);
+  k_reorder<<<grid_of(threads), kBlock, 0, st>>>(
       n, s.perm, s.keysA, s.A, s.B, pcisph, 3 * (int)s.dp.cell_shift, s.ncells, s.cstart(), s.cend(), s.n_static,
       s.skeys, s.spos, s.dp.static_base, s.mpos, s.mstart(), s.mend(), start);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -3125,7 +3151,7 @@ cudaError_t batch_launch_keys(BatchSystem& b, cudaStream_t st) {
 // Two stable LSD stages: the Morton keys (padding above them), then the
 // scene index; each scene's particles end up in its own segment in Morton
 // order, exactly the order a sort of that scene alone gives.
-cudaError_t batch_launch_sort(BatchSystem& b, cudaStream_t st) {
+cudaError_t batch_launch_sort(BatchSystem& b, cudaStream_t st, const LoopTurn& turn, cudaGraphConditionalHandle route) {
   const uint32_t n = b.n_slots;
   if (!n) return cudaSuccess;
   cudaError_t e;
@@ -3142,7 +3168,7 @@ cudaError_t batch_launch_sort(BatchSystem& b, cudaStream_t st) {
     e = radix_sort_pairs(b.digits, b.perm, kalt, valt, counts, n, b.scene_bits, false, st);
     if (e != cudaSuccess) return e;
   }
-  k_reorder_batch<<<grid_of(n), kBlock, 0, st>>>(b.view, n, b.perm, b.A, b.B, b.keysA);
+  k_reorder_batch<<<grid_of(n) + (turn.words ? 1 : 0), kBlock, 0, st>>>(b.view, n, b.perm, b.A, b.B, b.keysA, turn, route);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if ((e = cudaMemsetAsync(b.cstart, 0, sizeof(uint32_t) * b.n_cells, st)) != cudaSuccess) return e;
   if ((e = cudaMemsetAsync(b.cend, 0, sizeof(uint32_t) * b.n_cells, st)) != cudaSuccess) return e;
@@ -3165,9 +3191,8 @@ cudaError_t batch_launch_forces(BatchSystem& b, cudaStream_t st) {
                             b.force, b.pforce, b.xs, b.press, b.pq, nullptr);
 }
 
-cudaError_t batch_launch_loop_init(BatchSystem& b, cudaStream_t st, const LoopTurn& turn,
-                                   cudaGraphConditionalHandle route) {
-  k_loop_init_batch<<<1, 256, 0, st>>>(b.st_d, b.n_scenes, b.any_active_d, b.loop_sync, b.loop_max, turn, route);
+cudaError_t batch_launch_loop_init(BatchSystem& b, cudaStream_t st) {
+  k_loop_init_batch<<<1, 256, 0, st>>>(b.st_d, b.n_scenes, b.any_active_d, b.loop_sync, b.loop_max);
   return cudaGetLastError();
 }
 

@@ -243,7 +243,9 @@ struct System {
   bool loop_in_graph = false;     // the step graph being captured has the fused loop: no staging
   bool loop_yields = false;       // and counts among the device's loops (loop_yields())
   bool loop_both = false;         // and has the passes beside it
-  bool crowded = false;           // the step graph is the one with both forms, for good
+  bool graph_yields = false;      // a step of the step graph counts among the device's loops
+  cudaGraph_t both_graph = nullptr;  // the graph with both forms, once a call has taken it
+  cudaGraphExec_t both_exec = nullptr;
   uint32_t* crowd_host = nullptr;  // pinned: set by a step that met others (behind st_host)
 
   RigidArrays rb;
@@ -313,7 +315,8 @@ struct BatchSystem {
   bool shape_set = false;                   // as System's
   bool loop_yields = false;                 // as System's
   bool loop_both = false;
-  bool crowded = false;
+  cudaGraph_t both_graph = nullptr;
+  cudaGraphExec_t both_exec = nullptr;
   uint32_t* crowd_host = nullptr;           // behind st_h
   BatchView view;
 
@@ -351,11 +354,11 @@ cudaError_t launch_nlist_plain(const DevParams& P, uint32_t n, const float4* pos
 // upf_pipeline.cu: batched phase launchers (asynchronous on `st`)
 cudaError_t batch_launch_init(BatchSystem& b, cudaStream_t st);   // keys and lagged state after upload
 cudaError_t batch_launch_keys(BatchSystem& b, cudaStream_t st);   // keys only
-cudaError_t batch_launch_sort(BatchSystem& b, cudaStream_t st);
+cudaError_t batch_launch_sort(BatchSystem& b, cudaStream_t st, const LoopTurn& turn = {},  // (as launch_sort_phase)
+                              cudaGraphConditionalHandle route = 0);
 cudaError_t batch_launch_neighbors(BatchSystem& b, cudaStream_t st);
 cudaError_t batch_launch_forces(BatchSystem& b, cudaStream_t st);
-cudaError_t batch_launch_loop_init(BatchSystem& b, cudaStream_t st, const LoopTurn& turn = {},
-                                   cudaGraphConditionalHandle route = 0);
+cudaError_t batch_launch_loop_init(BatchSystem& b, cudaStream_t st);
 cudaError_t batch_launch_loop_body(BatchSystem& b, cudaStream_t st, cudaGraphConditionalHandle h, bool use_handle);
 cudaError_t batch_launch_loop_density(BatchSystem& b, cudaStream_t st);
 cudaError_t batch_launch_loop_pforce(BatchSystem& b, cudaStream_t st);
@@ -381,7 +384,7 @@ struct GraphParts {
   cudaError_t (*post)(void* ctx, cudaStream_t st) = nullptr;
   void* ctx = nullptr;
 };
-bool met_others(const uint32_t* crowd_host, bool crowded, cudaStream_t st);
+bool takes_both(const uint32_t* crowd_host, int32_t nsteps, bool built, cudaStream_t st);
 upf_status capture_step_graph(const GraphParts& parts, cudaGraph_t* graph_out, cudaGraphExec_t* exec_out);
 DevParams make_dev_params(const upf_params& p, uint32_t nstride);
 upf_status encode_list_map(CUtensorMap* map, void* base, CUtensorMapDataType dt, uint32_t elem_bytes,
